@@ -64,6 +64,32 @@ def test_reference_mesher_cases(ctx, oracle):
     assert ctx.world_mesh(mm, greedy=True) == (24, 12)
 
 
+@pytest.mark.parametrize("shape", [(16, 2, 16), (16, 15, 32), (32, 31, 16), (16, 32, 16), (16, 33, 16), (32, 65, 48),
+                                   (16, 1024, 16)])
+def test_world_mesh_slices_of_every_width(ctx, oracle, shape):
+    """Rows of one lane, of a ragged and a full warp and of several warp widths, odd layer counts, runs that cross the
+    32-cell chunks: long equal runs with seeded holes, and uniform noise."""
+    rng = np.random.default_rng(shape[1])
+    layers = np.repeat(rng.integers(0, 12, (shape[0] // 4, (shape[1] + 39) // 40, shape[2] // 8)), 4, 0)
+    layers = np.repeat(np.repeat(layers, 40, 1)[:, :shape[1]], 8, 2).astype(np.uint8)
+    layers[rng.random(shape) < 0.01] = 0
+    mm = np.arange(256, dtype=np.uint32) % 64
+    for vox in (layers, rng.integers(0, 3, shape).astype(np.uint8), np.full(shape, 7, np.uint8)):
+        ctx.world_upload(vox, chunk_x0=-2, chunk_z0=1)
+        for greedy in (True, False):
+            ctx.world_mesh(mm, voxel_size=0.3, greedy=greedy)
+            v, t = ctx.world_read_mesh()
+            ov, ot = oracle.world_mesh(vox, mm, greedy=greedy, chunk_x0=-2, chunk_z0=1, voxel_size=0.3)
+            assert np.array_equal(v.view(np.uint8), ov.view(np.uint8))
+            assert np.array_equal(t.view(np.uint8), ot.view(np.uint8))
+
+
+@pytest.mark.parametrize("shape", [(16, 2, 16), (48, 9, 16), (16, 257, 32)])
+def test_world_generate_ragged_columns(ctx, oracle, shape):
+    p = dict(scenes.world_params(3, *shape), cave_min_y=0)
+    assert np.array_equal(ctx.world_generate(p, read_back=True), oracle.world_generate(p))
+
+
 def _world_scene(ctx, seed=3, n=48):
     w = scenes.voxel_world(seed=seed, nx=n, ny=n, nz=n)
     ctx.world_generate(w["params"])
