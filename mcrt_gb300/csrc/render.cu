@@ -497,12 +497,15 @@ __global__ void k_raygen(DeviceScene S, RenderParams P, PathBuffers B, int keep_
 //  * A warp fetches rays for its idle lanes in batches (one atomicAdd on the
 //    work counter counters[4] per batch) whenever at least kRefill lanes are
 //    idle, so lanes do not sit out the longest ray of a fixed assignment.
-//  * Traversal phase: a lane walks internal nodes; a leaf it reaches is
-//    postponed and the lane keeps traversing until every active lane of the
-//    warp holds a postponed leaf (warp vote); then the lanes test their leaves
-//    together.  The vote only shapes scheduling: every order enters every box
-//    that can hold a hit at or before the closest t (the cull's slack,
-//    kCullSlack), so the hit is the reference order's.
+//  * Traversal phase: a lane walks internal nodes and postpones the first leaf
+//    it reaches, going on until it reaches a second; once fewer than
+//    kKeepWalking lanes still walk while others hold a leaf, the warp tests
+//    its leaves together.  (Going on until the last lane reached a leaf cost
+//    22.2 ms of closest-hit time per 1.3M-triangle frame, leaving at 8, 12, 16
+//    and 20 lanes 18.9, 18.55, 18.65 and 19.1.)  The vote only shapes
+//    scheduling: every order enters every box that can hold a hit at or before
+//    the closest t (the cull's slack, kCullSlack), so the hit is the reference
+//    order's.
 // Sphere BVHs (the reference's binding 5) are traversed at ray fetch with the
 // reference-order walk (spheres_hit); their count is small.
 
@@ -517,6 +520,15 @@ __global__ void k_raygen(DeviceScene S, RenderParams P, PathBuffers B, int keep_
 // (top = kTopNodes records, 8 KB per block, loaded once per block; the nodes
 // below are read through L1 as in the other variants).
 struct ExtendVariant { int width, block, min_blocks, stack, refill, top; };
+// Lanes that must still be walking nodes for a warp to go on with them while
+// others hold a postponed leaf.
+constexpr int kKeepWalking = 12;
+// Node visits between two rounds of sharing, once a warp has idle lanes and no ray is left.
+constexpr uint32_t kShareSteps = 4;
+constexpr uint32_t kNoRay = 0xffffffffu;
+// a ray whose stack would overflow keeps its queue index with bit 31 set
+// (indices are below 2^31 - 1) until it joins the overflow list
+constexpr uint32_t kOvfBit = 0x80000000u;
 constexpr int kExtendVariants = 8;
 constexpr ExtendVariant kVariantTable[kExtendVariants] = {
     {2, 128, 8, 64, 8, 0},  {2, 64, 20, 32, 8, 0},  {2, 64, 20, 32, 4, 0},   {2, 128, 10, 32, 8, (int)kTopNodes},
@@ -529,17 +541,16 @@ template <int STACK, int TOP>
 __device__ __forceinline__ void visit_compact2(const DeviceScene &S, const float4 *s_top, const RayInv &r,
                                                float tmax, uint32_t *cur, float *cur_t, uint2 *stack, uint32_t *sp,
                                                bool *overflow) {
-    float4 a, b, c;
-    uint4 e;
+    float4 a, b, c, e4;
     if (TOP > 0 && (*cur & kTopBit)) {
         const float4 *np = s_top + 4u * (*cur & ~kTopBit);
-        a = np[0]; b = np[1]; c = np[2];
-        e = *reinterpret_cast<const uint4 *>(np + 3);
+        a = np[0]; b = np[1]; c = np[2]; e4 = np[3];
     } else {
         const float4 *np = S.cnodes + 4ull * *cur;
-        a = __ldg(np); b = __ldg(np + 1); c = __ldg(np + 2);
-        e = __ldg(reinterpret_cast<const uint4 *>(np + 3));
+        ld_pair(np, &a, &b);
+        ld_pair(np + 2, &c, &e4);
     }
+    const uint2 e = make_uint2(__float_as_uint(e4.x), __float_as_uint(e4.y));
     float tl, tr;
     bool hl = e.x != kNoChild && slab(r, a.x, a.z, c.x, a.y, a.w, c.y, kTMin, tmax, &tl);
     bool hr = e.y != kNoChild && slab(r, b.x, b.z, c.z, b.y, b.w, c.w, kTMin, tmax, &tr);
@@ -632,6 +643,25 @@ __device__ __forceinline__ void visit_wide4(const DeviceScene &S, const RayInv &
     }
 }
 
+// Whether result a of one lane's share of a ray comes before result b of
+// another's: the tie rule (smallest t; a sphere before a triangle, then the
+// smaller original id).
+__device__ __forceinline__ bool closer(const Closest &a, const Closest &b) {
+    if (a.t < b.t) return true;
+    if (a.t != b.t || a.prim == MCRT_HIT_MISS || b.prim == MCRT_HIT_MISS) return false;
+    const bool as = (a.prim & MCRT_HIT_SPHERE) != 0u, bs = (b.prim & MCRT_HIT_SPHERE) != 0u;
+    return as != bs ? as : a.prim < b.prim;
+}
+
+// Position of the k-th set bit (from 0) of a mask that has more than k.
+__device__ __forceinline__ uint32_t nth_bit(unsigned mask, uint32_t k) {
+    uint32_t pos = 0;
+#pragma unroll
+    for (uint32_t w = 16; w; w >>= 1)
+        if ((uint32_t)__popc(mask & ((1u << (pos + w)) - 1u)) <= k) pos += w;
+    return pos;
+}
+
 // The end of a traced queue entry.  Closest hit: the hit record, in queue
 // order.  Any hit (a shadow ray of path `slot`): an unoccluded ray adds its
 // contribution to the path's radiance; ADJ: the adjoint replay's shadow ray,
@@ -682,6 +712,236 @@ __device__ __forceinline__ void finish_ray(const DeviceScene &S, const PathBuffe
 // the next closest-hit launch (neither runs while the list is in use).
 constexpr uint32_t kOvfClosest = 3u, kOvfAny = 7u;
 
+// The walk of one queue by a persistent warp.  SHARE: idle lanes help the
+// others once no ray is left, and a queue that does not fill the grid's lanes
+// is spread over all its warps.
+// Rays of a queue take very different numbers of steps (18 nodes on average,
+// 140 to 350 for the longest of a frame), and a lone ray's step costs a round
+// trip to the L2, so a launch with few rays lasts as long as its longest ray.
+// Taking over the oldest stack entry of a busy lane (its largest pending
+// subtree) cuts that tail: bounces of 20 to 200 thousand rays into an 80,000
+// triangle mesh took 112 to 131 us without sharing, 75 to 105 us with it.
+// The subtrees taken over are the far ones, which a nearer hit often culls,
+// and the code costs registers: with 5 million rays (voxel world) a launch took
+// 1.57 ms with sharing, 1.49 ms without.
+constexpr uint32_t kShareLoad = 8;      // SHARE below this many rays per lane of the grid
+template <int WIDTH, int BLOCK, int STACK, int REFILL, int TOP, bool ANY, bool ADJ, bool COUNT, bool SHARE>
+__device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuffers &B, const AdjointParams &A,
+                                            float *gacc, const float4 *s_top, uint32_t n, const float4 *qo,
+                                            const float4 *qd) {
+    uint32_t *work = B.counters + (ANY ? 5 : 4);    // the queue's next unclaimed entry
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned below = (1u << lane) - 1u;
+    const bool has_mesh = S.n_mesh_nodes > 0;
+    const uint32_t n_warps = gridDim.x * (BLOCK / 32);
+    // fewer rays than the grid has lanes: every warp takes its share at once
+    const bool spread = SHARE && n < n_warps * 32u;
+    const uint32_t share = (n + n_warps - 1u) / n_warps;
+    uint32_t ray = kNoRay;            // queue index of the lane's ray, or none
+    bool exhausted = false;           // the queue has been handed out (warp-uniform)
+    RayInv r;
+    Closest best;
+    uint2 stack[STACK];
+    uint32_t sp = 0, sb = 0;          // entries [sb, sp)
+    uint32_t cur = kNoChild;          // next node code to visit
+    float cur_t = 0.0f;               // its entry distance
+    uint32_t leaf = kNoChild;         // postponed leaf code
+    uint32_t traced = 0;
+    uint32_t nn = 0;
+    uint32_t ntri = 0;                // COUNT: triangles tested
+    uint32_t slot = 0;                // ANY: the shadow ray's path
+    bool occl = false;                // ANY: an accepted hit was found
+    // drops everything the lane has left to do for its ray
+    auto drop = [&]() {
+        cur = kNoChild;
+        leaf = kNoChild;
+        sp = sb = 0;
+    };
+    // the lane's next step: cur an internal node to visit, or a leaf behind the postponed one, or none left
+    auto settle = [&]() {
+        for (;;) {
+            if (cur != kNoChild && cur_t > cull_t(best.t)) cur = kNoChild;   // culled since it was queued
+            if (cur == kNoChild) {                                        // pop the next live entry
+                while (sp > sb) {
+                    uint2 s = stack[--sp];
+                    if (__uint_as_float(s.y) <= cull_t(best.t)) { cur = s.x; cur_t = __uint_as_float(s.y); break; }
+                }
+                if (cur == kNoChild) { sp = sb = 0; return; }
+            }
+            if (!(cur & kLeafBit) || leaf != kNoChild) return;
+            leaf = cur;
+            cur = kNoChild;
+        }
+    };
+    for (;;) {
+        // ---- refill idle lanes
+        const unsigned idle_mask = __ballot_sync(0xffffffffu, ray == kNoRay);
+        if (exhausted && idle_mask == 0xffffffffu) break;
+        if (!exhausted && (__popc(idle_mask) >= REFILL || idle_mask == 0xffffffffu)) {
+            const int leader = __ffs(idle_mask) - 1;
+            uint32_t base = 0, end = n;
+            if (spread) {
+                base = ((blockIdx.x * BLOCK + threadIdx.x) >> 5) * share;
+                end = min(n, base + share);
+                exhausted = true;
+            } else {
+                if ((int)lane == leader) base = atomicAdd(work, (uint32_t)__popc(idle_mask));
+                base = __shfl_sync(0xffffffffu, base, leader);
+                if (base + (uint32_t)__popc(idle_mask) >= n) exhausted = true;
+            }
+            const uint32_t mine = base + __popc(idle_mask & below);
+            if (ray == kNoRay && mine < end) {
+                ray = mine;
+                float4 o4 = __ldcs(qo + mine), d4 = __ldcs(qd + mine);   // streamed: evict first
+                r = make_ray(xyz(o4), xyz(d4));
+                const float tmax = ANY ? d4.w : kTMax;
+                best = Closest{tmax, MCRT_HIT_MISS, 0u, 0.0f, 0.0f};
+                spheres_hit(S, r, kTMin, tmax, best, &nn);       // path_trace.wgsl:472-474
+                drop();
+                if (ANY) {
+                    slot = __float_as_uint(o4.w);
+                    occl = best.prim != MCRT_HIT_MISS;
+                    best.t = tmax;
+                }
+                if (has_mesh && !(ANY && occl)) {
+                    const float4 *np = reinterpret_cast<const float4 *>(S.mesh_nodes);
+                    float4 mn = __ldg(np), mx = __ldg(np + 1);
+                    float te;
+                    if (slab(r, mn.x, mn.y, mn.z, mx.x, mx.y, mx.z, kTMin, best.t, &te)) {
+                        if (S.n_cnodes == 0) {
+                            uint4 meta = __ldg(reinterpret_cast<const uint4 *>(np + 2));
+                            cur = leaf_code(meta.x, meta.y);
+                        } else {
+                            cur = TOP > 0 ? kTopBit : 0u;
+                        }
+                        cur_t = te;
+                    }
+                }
+            }
+        } else if (SHARE && exhausted && idle_mask) {
+            // ---- no ray is left: idle lanes take over the oldest stack entries (the largest subtrees) of busy ones
+            const unsigned offers = __ballot_sync(0xffffffffu, sp > sb);
+            const uint32_t pairs = min(__popc(idle_mask), __popc(offers));
+            if (pairs) {
+                const bool takes = ray == kNoRay && __popc(idle_mask & below) < pairs;
+                const bool gives = sp > sb && __popc(offers & below) < pairs;
+                uint2 e = make_uint2(kNoChild, 0u);
+                if (gives) e = stack[sb++];
+                const int from = takes ? (int)nth_bit(offers, __popc(idle_mask & below)) : (int)lane;
+                auto pass = [&](float &v) { v = __shfl_sync(0xffffffffu, v, from); };
+                pass(r.o.x); pass(r.o.y); pass(r.o.z);
+                pass(r.d.x); pass(r.d.y); pass(r.d.z);
+                pass(r.inv.x); pass(r.inv.y); pass(r.inv.z);
+                pass(best.t); pass(best.u); pass(best.v);
+                auto passu = [&](uint32_t &v) { v = __shfl_sync(0xffffffffu, v, from); };
+                passu(best.prim); passu(best.slot); passu(ray); passu(e.x); passu(e.y);
+                if (ANY) passu(slot);
+                if (takes) {
+                    drop();
+                    occl = false;
+                    cur = e.x;
+                    cur_t = __uint_as_float(e.y);
+                }
+            }
+        }
+        // ---- traversal phase
+        if (ray != kNoRay) settle();
+        for (uint32_t step = 0;; ++step) {
+            const bool go = cur < kLeafBit;                      // an internal node (leaves and kNoChild have bit 31)
+            const unsigned going = __ballot_sync(0xffffffffu, go);
+            if (going == 0) break;
+            if (__popc(going) < kKeepWalking && __any_sync(0xffffffffu, leaf != kNoChild)) break;
+            if (SHARE && exhausted && idle_mask && step >= kShareSteps) break;
+            if (go) {
+                ++nn;
+                bool full = false;
+                if (WIDTH == 4) visit_wide4<STACK>(S, r, best.t, &cur, &cur_t, stack, &sp, &full);
+                else visit_compact2<STACK, TOP>(S, s_top, r, best.t, &cur, &cur_t, stack, &sp, &full);
+                if (full) {                                      // to the overflow list
+                    ray |= kOvfBit;
+                    drop();
+                } else {
+                    settle();
+                }
+            }
+        }
+        // ---- leaf phase
+        while (leaf != kNoChild) {
+            if (ANY) {
+                if (leaf_any(S, r, (leaf & ~kLeafBit) >> 4, leaf_count(S, leaf), kTMin, best.t)) {
+                    occl = true;                                 // done: drop what is left
+                    drop();
+                    break;
+                }
+            } else {
+                const uint32_t cnt = leaf_count(S, leaf);
+                if (COUNT) ntri += cnt;
+                leaf_tris(S, r, (leaf & ~kLeafBit) >> 4, cnt, kTMin, best);
+            }
+            leaf = kNoChild;
+            if (cur != kNoChild && (cur & kLeafBit) && cur_t <= cull_t(best.t)) {
+                leaf = cur;
+                cur = kNoChild;
+            }
+        }
+        __syncwarp();
+        // ---- finished rays
+        bool done = ray != kNoRay && cur == kNoChild && sp == sb;
+        if (SHARE && exhausted) {
+            // a ray that several lanes share: the first to finish hands its result to another of them
+            for (unsigned fin = __ballot_sync(0xffffffffu, done); fin; fin &= fin - 1u) {
+                const int f = __ffs(fin) - 1;
+                const uint32_t id = __shfl_sync(0xffffffffu, ray, f) & ~kOvfBit;
+                const unsigned others =
+                    __ballot_sync(0xffffffffu, ray != kNoRay && (ray & ~kOvfBit) == id) & ~(1u << f);
+                if (!others) continue;
+                const bool into = (int)lane == __ffs(others) - 1;
+                const uint32_t fray = __shfl_sync(0xffffffffu, ray, f);
+                if (ANY) {
+                    const bool focc = __shfl_sync(0xffffffffu, (int)occl, f) != 0;
+                    if (into && (focc || (fray & kOvfBit))) {
+                        occl = occl || focc;
+                        ray |= fray & kOvfBit;
+                        drop();
+                    }
+                } else {
+                    Closest c;
+                    c.t = __shfl_sync(0xffffffffu, best.t, f);
+                    c.prim = __shfl_sync(0xffffffffu, best.prim, f);
+                    c.slot = __shfl_sync(0xffffffffu, best.slot, f);
+                    c.u = __shfl_sync(0xffffffffu, best.u, f);
+                    c.v = __shfl_sync(0xffffffffu, best.v, f);
+                    if (into) {
+                        if (closer(c, best)) best = c;
+                        if (fray & kOvfBit) {
+                            ray |= kOvfBit;
+                            drop();
+                        }
+                    }
+                }
+                if ((int)lane == f) {
+                    ray = kNoRay;
+                    done = false;
+                }
+            }
+        }
+        if (done) {
+            if (ray & kOvfBit) {
+                B.ovf[atomicAdd(B.counters + (ANY ? kOvfAny : kOvfClosest), 1u)] = ray & ~kOvfBit;
+            } else {
+                finish_ray<ANY, ADJ>(S, B, A, gacc, ray, slot, occl, best);
+                ++traced;
+            }
+            ray = kNoRay;
+        }
+    }
+    if (traced) atomicAdd(B.stats + (ANY ? 1 : 0), (unsigned long long)traced);
+    if (COUNT) {
+        atomicAdd(B.stats + 3, (unsigned long long)nn);
+        atomicAdd(B.stats + 4, (unsigned long long)ntri);
+    }
+}
+
 // ANY = true: the same persistent, refilled, speculative traversal for the
 // shadow-ray queue of next-event estimation, as an any-hit test: the cull
 // threshold stays the ray's t_max, so the set of boxes entered does not depend
@@ -715,137 +975,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_extend(DeviceScene S, PathBuffe
     }
     const float4 *qo = ANY ? B.sh_o : B.q_o[qi];
     const float4 *qd = ANY ? B.sh_d : B.q_d[qi];
-    uint32_t *work = B.counters + (ANY ? 5 : 4);    // the queue's next unclaimed entry
-    const uint32_t lane = threadIdx.x & 31u;
-    const bool has_mesh = S.n_mesh_nodes > 0;
-    uint32_t ray = 0xffffffffu;       // queue index of the lane's ray, or none
-    bool exhausted = false;           // the queue has been handed out (warp-uniform)
-    RayInv r;
-    Closest best;
-    uint2 stack[STACK];
-    uint32_t sp = 0;
-    uint32_t cur = kNoChild;          // next node code to visit
-    float cur_t = 0.0f;               // its entry distance
-    uint32_t leaf = kNoChild;         // postponed leaf code
-    uint32_t traced = 0;
-    uint32_t nn = 0;
-    uint32_t ntri = 0;                // COUNT: triangles tested
-    uint32_t slot = 0;                // ANY: the shadow ray's path
-    bool occl = false;                // ANY: an accepted hit was found
-    // a ray whose stack would overflow keeps its queue index with bit 31 set
-    // (indices are below 2^31) until it joins the overflow list
-    constexpr uint32_t kOvfBit = 0x80000000u;
-    for (;;) {
-        // ---- refill idle lanes
-        const bool idle = ray == 0xffffffffu;
-        const unsigned idle_mask = __ballot_sync(0xffffffffu, idle);
-        if (!exhausted && (__popc(idle_mask) >= REFILL || idle_mask == 0xffffffffu)) {
-            const int leader = __ffs(idle_mask) - 1;
-            uint32_t base = 0;
-            if ((int)lane == leader) base = atomicAdd(work, (uint32_t)__popc(idle_mask));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + (uint32_t)__popc(idle_mask) >= n) exhausted = true;
-            if (idle) {
-                const uint32_t mine = base + __popc(idle_mask & ((1u << lane) - 1u));
-                if (mine < n) {
-                    ray = mine;
-                    float4 o4 = __ldcs(qo + mine), d4 = __ldcs(qd + mine);   // streamed: evict first
-                    r = make_ray(xyz(o4), xyz(d4));
-                    const float tmax = ANY ? d4.w : kTMax;
-                    best = Closest{tmax, MCRT_HIT_MISS, 0u, 0.0f, 0.0f};
-                    spheres_hit(S, r, kTMin, tmax, best, &nn);       // path_trace.wgsl:472-474
-                    sp = 0;
-                    leaf = kNoChild;
-                    cur = kNoChild;
-                    if (ANY) {
-                        slot = __float_as_uint(o4.w);
-                        occl = best.prim != MCRT_HIT_MISS;
-                        best.t = tmax;
-                    }
-                    if (has_mesh && !(ANY && occl)) {
-                        const float4 *np = reinterpret_cast<const float4 *>(S.mesh_nodes);
-                        float4 mn = __ldg(np), mx = __ldg(np + 1);
-                        float te;
-                        if (slab(r, mn.x, mn.y, mn.z, mx.x, mx.y, mx.z, kTMin, best.t, &te)) {
-                            if (S.n_cnodes == 0) {
-                                uint4 meta = __ldg(reinterpret_cast<const uint4 *>(np + 2));
-                                cur = leaf_code(meta.x, meta.y);
-                            } else {
-                                cur = TOP > 0 ? kTopBit : 0u;
-                            }
-                            cur_t = te;
-                        }
-                    }
-                }
-            }
-        }
-        if (__ballot_sync(0xffffffffu, ray != 0xffffffffu) == 0) break;   // exhausted and all idle
-        if (ray != 0xffffffffu) {
-            // ---- traversal phase
-            for (;;) {
-                if (cur != kNoChild && cur_t > cull_t(best.t)) cur = kNoChild;   // culled since it was queued
-                if (cur == kNoChild) {                                        // pop the next live entry
-                    while (sp > 0) {
-                        uint2 s = stack[--sp];
-                        if (__uint_as_float(s.y) <= cull_t(best.t)) { cur = s.x; cur_t = __uint_as_float(s.y); break; }
-                    }
-                    if (cur == kNoChild) break;
-                }
-                if (cur & kLeafBit) {
-                    if (leaf != kNoChild) break;                              // one leaf already waits
-                    leaf = cur;
-                    cur = kNoChild;
-                    continue;
-                }
-                ++nn;
-                bool full = false;
-                if (WIDTH == 4) visit_wide4<STACK>(S, r, best.t, &cur, &cur_t, stack, &sp, &full);
-                else visit_compact2<STACK, TOP>(S, s_top, r, best.t, &cur, &cur_t, stack, &sp, &full);
-                if (full) {                                                   // to the overflow list
-                    ray |= kOvfBit;
-                    cur = kNoChild;
-                    sp = 0;
-                    leaf = kNoChild;
-                    break;
-                }
-                if (__all_sync(__activemask(), leaf != kNoChild)) break;
-            }
-            // ---- leaf phase
-            while (leaf != kNoChild) {
-                if (ANY) {
-                    if (leaf_any(S, r, (leaf & ~kLeafBit) >> 4, leaf_count(S, leaf), kTMin, best.t)) {
-                        occl = true;                                          // done: drop what is left
-                        cur = kNoChild;
-                        sp = 0;
-                    }
-                } else {
-                    const uint32_t cnt = leaf_count(S, leaf);
-                    if (COUNT) ntri += cnt;
-                    leaf_tris(S, r, (leaf & ~kLeafBit) >> 4, cnt, kTMin, best);
-                }
-                leaf = kNoChild;
-                if (cur != kNoChild && (cur & kLeafBit) && cur_t <= cull_t(best.t)) {
-                    leaf = cur;
-                    cur = kNoChild;
-                }
-            }
-            // ---- finished ray
-            if (cur == kNoChild && sp == 0) {
-                if (ray & kOvfBit) {
-                    B.ovf[atomicAdd(B.counters + (ANY ? kOvfAny : kOvfClosest), 1u)] = ray & ~kOvfBit;
-                } else {
-                    finish_ray<ANY, ADJ>(S, B, A, gacc, ray, slot, occl, best);
-                    ++traced;
-                }
-                ray = 0xffffffffu;
-            }
-        }
-    }
-    if (traced) atomicAdd(B.stats + (ANY ? 1 : 0), (unsigned long long)traced);
-    if (COUNT) {
-        atomicAdd(B.stats + 3, (unsigned long long)nn);
-        atomicAdd(B.stats + 4, (unsigned long long)ntri);
-    }
+    if (n < kShareLoad * (gridDim.x * BLOCK))
+        trace_queue<WIDTH, BLOCK, STACK, REFILL, TOP, ANY, ADJ, COUNT, true>(S, B, A, gacc, s_top, n, qo, qd);
+    else
+        trace_queue<WIDTH, BLOCK, STACK, REFILL, TOP, ANY, ADJ, COUNT, false>(S, B, A, gacc, s_top, n, qo, qd);
     if (ADJ) {
         __syncthreads();
         for (uint32_t k = threadIdx.x; k < 256u; k += BLOCK) {
@@ -1553,7 +1686,17 @@ void launch_extend(const DeviceScene &S, const RenderParams &P, PathBuffers &B, 
     prepare_extend_variants();
     const uint32_t nmax = P.npix * P.spp_pass;
     const bool count = (P.flags & MCRT_RENDER_COUNT) != 0;
-    if (primary) {                    // the camera rays: warp packets, every warp resident at once
+    // The camera rays as warp packets (every warp resident at once) or one per
+    // lane.  A packet walks the union of its 32 rays' nodes in one chain of
+    // dependent loads, so it pays while its rays see the same triangles: with
+    // many samples per pixel and pixels no smaller than the triangles.  Camera
+    // rays into a mesh, packets / lanes, in us: 1.3M triangles, 960x540, 1
+    // spp (0.4 paths per triangle) 1100 / 314; the same mesh, 1920x1080, 2 spp
+    // (3 paths) 824 / 643, 16 spp (25) 2013 / 2289; 80,000 triangles, 640x360,
+    // 2 spp (6) 245 / 199, 8 spp (23) 244 / 287; a voxel world of 4.9M faces, most
+    // of them out of sight, 1280x720, 8 spp (1.5) 893 / 1124.  The line, 4/3
+    // paths per triangle, leaves the last with packets.
+    if (primary && 3ull * nmax >= 4ull * S.n_triangles) {
         const int blocks = min(grid_blocks_for(nmax, kPacketBlock), sm_count() * g_packet_per_sm);
         if (count) k_extend_packet<true><<<blocks, kPacketBlock, 0, st>>>(S, B, qi);
         else k_extend_packet<false><<<blocks, kPacketBlock, 0, st>>>(S, B, qi);
@@ -1562,7 +1705,7 @@ void launch_extend(const DeviceScene &S, const RenderParams &P, PathBuffers &B, 
         // persistent: as many resident blocks as fit, never more warps than rays
         const int block = kVariantTable[v].block;
         const int per_sm = count ? g_count_per_sm[v] : g_extend_per_sm[v];
-        const int blocks = min(grid_blocks_for(nmax, block), sm_count() * per_sm);
+        const int blocks = min(grid_blocks_for(nmax, block / 32), sm_count() * per_sm);
         (count ? kCountKernels[v] : kExtendKernels[v])<<<blocks, block, 0, st>>>(S, B, qi, AdjointParams{});
         ::mcrt::note_launch();
     }
@@ -1587,7 +1730,7 @@ void launch_shadow(const DeviceScene &S, const RenderParams &P, PathBuffers &B, 
     prepare_extend_variants();
     const int block = kVariantTable[v].block;
     const int per_sm = adj ? g_shadow_adj_per_sm[v] : g_shadow_per_sm[v];
-    int blocks = min(grid_blocks_for(nmax, block), sm_count() * per_sm);
+    const int blocks = min(grid_blocks_for(nmax, block / 32), sm_count() * per_sm);
     if (adj) kShadowAdjKernels[v]<<<blocks, block, 0, st>>>(S, B, 0, *adj);
     else kShadowKernels[v]<<<blocks, block, 0, st>>>(S, B, 0, AdjointParams{});
     ::mcrt::note_launch();

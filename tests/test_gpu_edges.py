@@ -110,3 +110,22 @@ def test_grazing_camera_every_variant_renders_the_oracle_image(ctx, oracle):
     for v in range(8):
         got = ctx.render(cam, w, h, spp, max_depth=3, variant=v)
         assert np.array_equal(bits(got["rgba"]), bits(want["rgba"])), f"variant {v}"
+
+
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (7, 5, 1), (33, 31, 2), (96, 64, 16)])
+@pytest.mark.parametrize("variant", [0, 1, 5])
+def test_short_queues_are_shared_and_spread(ctx, oracle, w, h, spp, variant):
+    """Queues shorter than the grid: rays spread over the warps, idle lanes taking over stack entries (closest hit and
+    shadow rays), camera rays by lanes (fewer than 4/3 paths per triangle) and by packets."""
+    from mcrt_gb300 import scenes
+    sc = scenes.displaced_icosphere(5, level=5, width=w, height=h)
+    c = sc["camera"]
+    cam = M.compute_camera(w, h, c["look_from"], c["look_at"], c["vfov"], 0.0)
+    env = M.gradient_env_map()
+    sun = dict(sun_dir=[0.4, 0.8, 0.3], sun_irradiance=[2.0, 1.9, 1.7])
+    kw = dict(vertices=sc["vertices"], triangles=sc["triangles"], materials=sc["materials"], env=env, **sun)
+    ctx.upload_scene(**kw)
+    got = ctx.render(cam, w, h, spp, max_depth=12, nee=True, variant=variant)
+    want = oracle.OracleScene(**kw).render(cam, w, h, spp, max_depth=12, nee=True)
+    assert np.array_equal(bits(got["rgba"]), bits(want["rgba"]))
+    assert np.array_equal(bits(got["gbuf"]), bits(want["gbuf"]))

@@ -84,7 +84,7 @@ def test_world_mesh_slices_of_every_width(ctx, oracle, shape):
             assert np.array_equal(t.view(np.uint8), ot.view(np.uint8))
 
 
-@pytest.mark.parametrize("shape", [(16, 2, 16), (48, 9, 16), (16, 257, 32)])
+@pytest.mark.parametrize("shape", [(16, 3, 16), (48, 9, 16), (16, 257, 32)])
 def test_world_generate_ragged_columns(ctx, oracle, shape):
     p = dict(scenes.world_params(3, *shape), cave_min_y=0)
     assert np.array_equal(ctx.world_generate(p, read_back=True), oracle.world_generate(p))
