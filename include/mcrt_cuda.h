@@ -528,6 +528,8 @@ mcrt_status mcrt_read_image_rgba8(mcrt_ctx *ctx, uint32_t mode, uint8_t *out);
  * tree (included in [0] and [1]), [6] / [7] with MCRT_RENDER_COUNT: compact
  * BVH node records (64 B) and triangle records (48 B) the closest-hit kernels
  * fetched (the bounce-0 warp packets fetch one record per warp).
+ * Small scenes (at most 64 triangles and 16 spheres) are traced by one kernel
+ * per pass unless a variant is named: its time is [1], [2] and [3] are 0.
  * out_ms: 6 floats, out_counts: 8 uint64. */
 mcrt_status mcrt_last_timings(mcrt_ctx *ctx, float *out_ms, uint64_t *out_counts);
 

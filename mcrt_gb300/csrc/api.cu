@@ -57,6 +57,8 @@ struct mcrt_ctx {
     DBuf wnodes;
     uint32_t n_wnodes = 0;
     bool wide_valid = false;    // wnodes matches the current mesh BVH
+    DBuf small;                 // SmallScene of the current mesh, usable when small_ok
+    bool small_ok = false;
     DBuf spheres, sphere_ids, sphere_nodes, vertices, triangles, mesh_nodes, tri_order, trirecs, cnodes, materials,
         env, lights, light_cdf, tmp, staging, albedo, shade_recs, top;
     uint32_t albedo_layers = 0, albedo_size = 0;
@@ -241,6 +243,7 @@ cudaEvent_t ev(mcrt_ctx *ctx, size_t i) {
 mcrt_status finish_mesh(mcrt_ctx *ctx) {
     cudaStream_t st = ctx->stream;
     uint32_t nt = ctx->n_triangles, nn = ctx->n_mesh_nodes;
+    ctx->small_ok = false;
     CK(ctx->trirecs.ensure((size_t)std::max(nt, 1u) * sizeof(mcrt::TriRec)), "allocate triangle records");
     CK(ctx->shade_recs.ensure((size_t)std::max(nt, 1u) * 48), "allocate shading records");
     mcrt::launch_shade_recs(ctx->vertices.as<mcrt_gpu_vertex>(), ctx->triangles.as<mcrt_gpu_triangle>(), nt,
@@ -258,6 +261,15 @@ mcrt_status finish_mesh(mcrt_ctx *ctx) {
     if (ncn >= mcrt::kTopBit) return fail(ctx, MCRT_ERR_INVALID_ARG, "mesh too large for the compact BVH codes");
     CK(ctx->top.ensure((size_t)mcrt::kTopNodes * 64), "allocate top tree");
     CK(mcrt::gpu_make_top(cn, ncn, ctx->top.as<float4>(), st), "top tree");
+    if (nt <= mcrt::kSmallTris) {
+        CK(ctx->small.ensure(sizeof(mcrt::SmallScene)), "allocate small scene");
+        mcrt::launch_small_scene(device_scene(ctx), ctx->small.as<mcrt::SmallScene>(), st);
+        uint32_t ok = 0;
+        CK(cudaMemcpyAsync(&ok, &ctx->small.as<mcrt::SmallScene>()->ok, 4, cudaMemcpyDeviceToHost, st),
+           "read small scene");
+        CK(cudaStreamSynchronize(st), "small scene");
+        ctx->small_ok = ok != 0;
+    }
     ctx->wide_valid = false;                  // the 4-wide layout is built when a render first needs it
     ctx->n_wnodes = 0;
     return MCRT_OK;
@@ -293,6 +305,15 @@ mcrt_status render_variant(mcrt_ctx *ctx, const mcrt_render_opts &o, int *varian
     }
     *variant = v;
     return MCRT_OK;
+}
+
+// Whether a render with passes of n_slots paths takes the path kernel of small
+// scenes: few triangles and spheres for its passes (kSmallPass), and neither a
+// closest-hit variant nor the counting kernels asked for.
+bool small_scene(const mcrt_ctx *ctx, const mcrt_render_opts &o, uint32_t n_slots) {
+    if (!ctx->small_ok || o.variant != 0 || (o.flags & MCRT_RENDER_COUNT)) return false;
+    return n_slots <= mcrt::kSmallPass ? ctx->n_spheres <= mcrt::kSmallSpheres
+                                       : ctx->n_spheres == 0 && ctx->n_triangles <= mcrt::kFewTris;
 }
 
 // Light CDF over the light list (device), total weight read back.
@@ -406,7 +427,7 @@ void mcrt_destroy(mcrt_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     DBuf *bufs[] = {&ctx->spheres, &ctx->sphere_ids, &ctx->sphere_nodes, &ctx->vertices, &ctx->triangles,
                     &ctx->mesh_nodes, &ctx->tri_order, &ctx->trirecs, &ctx->cnodes, &ctx->top, &ctx->materials, &ctx->env,
-                    &ctx->lights, &ctx->light_cdf, &ctx->tmp, &ctx->staging, &ctx->albedo, &ctx->wnodes, &ctx->pbmem, &ctx->mean,
+                    &ctx->lights, &ctx->light_cdf, &ctx->small, &ctx->tmp, &ctx->staging, &ctx->albedo, &ctx->wnodes, &ctx->pbmem, &ctx->mean,
                     &ctx->sum, &ctx->gbuf, &ctx->io_a, &ctx->io_b, &ctx->io_c, &ctx->counters, &ctx->dimg,
                     &ctx->grad, &ctx->world_vox, &ctx->world_matmap, &ctx->wmesh.counts, &ctx->wmesh.vertices,
                     &ctx->wmesh.triangles, &ctx->views, &ctx->pass_state, &ctx->cache_q, &ctx->cache_rec,
@@ -550,6 +571,9 @@ mcrt_status mcrt_upload_scene(mcrt_ctx *ctx, const mcrt_scene_desc *d) {
         }
     } else {
         ctx->n_cnodes = 0;
+        CK(ctx->small.ensure(sizeof(mcrt::SmallScene)), "allocate small scene");
+        CK(cudaMemsetAsync(ctx->small.p, 0, sizeof(mcrt::SmallScene), st), "clear small scene");
+        ctx->small_ok = true;                  // no triangle: the spheres, or nothing
     }
     // ---- albedo texture array (binding 10)
     {
@@ -845,12 +869,25 @@ static mcrt_status render_core(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, ui
         }
         return P;
     };
-    mcrt_status cache_status = MCRT_OK;
+    mcrt_status pass_status = MCRT_OK;
     // one pass: raygen, the bounces, resolve (into the accumulation)
+    const bool small = small_scene(ctx, o, n_slots);
     auto enqueue_pass = [&](const mcrt::RenderParams &P, bool keep_pass, bool timed) {
-        mcrt::launch_raygen(S, P, ctx->pb, st);
+        if (small) {                                  // whole paths in one kernel, counted as closest-hit time
+            size_t a0 = 0;
+            if (timed) { a0 = evi++; cudaEventRecord(ev(ctx, a0), st); }
+            cudaError_t e = mcrt::launch_paths(S, P, ctx->pb, ctx->small.as<mcrt::SmallScene>(), ctx->gbuf.as<float4>(), st);
+            if (e != cudaSuccess) pass_status = cuda_fail(ctx, e, "path kernel");
+            ++extend_launches;
+            if (timed) {
+                cudaEventRecord(ev(ctx, evi++), st);
+                marks.push_back({a0, 1});
+            }
+        } else {
+            mcrt::launch_raygen(S, P, ctx->pb, st);
+        }
         int qi = 0;
-        for (uint32_t b = 0; b < depth; ++b) {
+        for (uint32_t b = 0; b < (small ? 0u : depth); ++b) {
             size_t a0 = 0, a1 = 0, a2 = 0;
             if (timed) { a0 = evi++; cudaEventRecord(ev(ctx, a0), st); }
             mcrt::launch_extend(S, P, ctx->pb, qi, st, b == 0);
@@ -876,7 +913,7 @@ static mcrt_status render_core(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, ui
         if (use_cache) {                              // the terminated paths take the cache's prediction
             cudaError_t e = mcrt::cache_infer_device(ctx->cache, ctx->cache_q.as<float4>(), ctx->pb.counters + 6,
                                                      P.npix * P.spp_pass, nullptr, ctx->pb.L, ctx->pb.thr, st);
-            if (e != cudaSuccess) cache_status = cuda_fail(ctx, e, "cache inference");
+            if (e != cudaSuccess) pass_status = cuda_fail(ctx, e, "cache inference");
         }
         size_t r0 = 0;
         if (timed) { r0 = evi++; cudaEventRecord(ev(ctx, r0), st); }
@@ -885,13 +922,13 @@ static mcrt_status render_core(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, ui
             cudaEventRecord(ev(ctx, evi++), st);
             marks.push_back({r0, 4});
         }
-        if (use_cache && cache_status == MCRT_OK) {   // train on this pass's training paths
+        if (use_cache && pass_status == MCRT_OK) {   // train on this pass's training paths
             const mcrt_cache_params &c = ctx->cache_cfg;
             const uint32_t n_train = (P.npix * P.spp_pass + train_stride - 1) / train_stride;
             cudaError_t e = mcrt::cache_train_records(ctx->cache, ctx->cache_rec.as<float4>(), n_train, depth,
                                                       train_stride, ctx->pb.L, c.train_steps, c.train_batch, c.lr,
                                                       st);
-            if (e != cudaSuccess) cache_status = cuda_fail(ctx, e, "cache training");
+            if (e != cudaSuccess) pass_status = cuda_fail(ctx, e, "cache training");
         }
     };
     uint32_t done = 0;
@@ -914,7 +951,7 @@ static mcrt_status render_core(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, ui
             ccfg = ctx->cache_cfg;
         }
         std::vector<char> key(sizeof(S) + sizeof(P) + sizeof(mcrt::PathBuffers) + 3 * sizeof(void *) + 8 +
-                              sizeof(cbufs) + sizeof(ccfg));
+                              sizeof(cbufs) + sizeof(ccfg) + sizeof(void *));
         {
             char *k = key.data();
             std::memcpy(k, &S, sizeof(S)); k += sizeof(S);
@@ -925,7 +962,9 @@ static mcrt_status render_core(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, ui
             uint32_t extra[2] = {depth, nee ? 1u : 0u};
             std::memcpy(k, extra, sizeof(extra)); k += sizeof(extra);
             std::memcpy(k, cbufs, sizeof(cbufs)); k += sizeof(cbufs);
-            std::memcpy(k, &ccfg, sizeof(ccfg));
+            std::memcpy(k, &ccfg, sizeof(ccfg)); k += sizeof(ccfg);
+            const void *small_scene_ptr = small ? ctx->small.p : nullptr;
+            std::memcpy(k, &small_scene_ptr, sizeof(void *));
         }
         if (!ctx->graph_exec || ctx->graph_key != key) {
             if (ctx->graph_exec) { cudaGraphExecDestroy(ctx->graph_exec); ctx->graph_exec = nullptr; }
@@ -965,7 +1004,7 @@ static mcrt_status render_core(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, ui
     cudaEventRecord(e_end, st);
     CK(cudaGetLastError(), "render launch");
     CK(cudaEventSynchronize(e_end), "render");
-    if (cache_status != MCRT_OK) return cache_status;
+    if (pass_status != MCRT_OK) return pass_status;
     if (use_cache) {                               // the judge's verdict on this render's passes
         double j[8];
         CK(mcrt::cache_judge_read(ctx->cache, j, st), "bias judge");
@@ -1105,6 +1144,7 @@ mcrt_status mcrt_adjoint(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, uint32_t
     A.inv_spp = 1.0f / (float)spp;
     A.grad = ctx->grad.as<double>();
     const bool nee = (o.flags & MCRT_RENDER_NEE) != 0 && (ctx->n_lights > 0 || ctx->has_sun);
+    const bool small = small_scene(ctx, o, npix * spp_pass);
     const unsigned long long launches0 = mcrt::launch_count();
     cudaEvent_t e_begin = ev(ctx, 2), e_end = ev(ctx, 3);
     cudaEventRecord(e_begin, st);
@@ -1121,23 +1161,31 @@ mcrt_status mcrt_adjoint(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, uint32_t
         P.extend_variant = variant;
         A.planes = P.spp_pass;
         // primal pass: the per-path radiance of these samples
-        mcrt::launch_raygen(S, P, ctx->pb, st);
         int qi = 0;
-        for (uint32_t b = 0; b < depth; ++b) {
-            mcrt::launch_extend(S, P, ctx->pb, qi, st, b == 0);
-            mcrt::launch_shade(S, P, ctx->pb, qi, b, nullptr, st);
-            if (nee) mcrt::launch_shadow(S, P, ctx->pb, st);
-            qi ^= 1;
+        if (small) {
+            CK(mcrt::launch_paths(S, P, ctx->pb, ctx->small.as<mcrt::SmallScene>(), nullptr, st), "path kernel");
+        } else {
+            mcrt::launch_raygen(S, P, ctx->pb, st);
+            for (uint32_t b = 0; b < depth; ++b) {
+                mcrt::launch_extend(S, P, ctx->pb, qi, st, b == 0);
+                mcrt::launch_shade(S, P, ctx->pb, qi, b, nullptr, st);
+                if (nee) mcrt::launch_shadow(S, P, ctx->pb, st);
+                qi ^= 1;
+            }
         }
         mcrt::launch_resolve(P, ctx->pb, ctx->mean.as<float4>(), ctx->sum.as<double>(), done > 0, st);
         // adjoint pass: replay the same paths from their seeds
-        mcrt::launch_raygen(S, P, ctx->pb, st, true);
-        qi = 0;
-        for (uint32_t b = 0; b < depth; ++b) {
-            mcrt::launch_extend(S, P, ctx->pb, qi, st, b == 0);
-            mcrt::launch_shade(S, P, ctx->pb, qi, b, nullptr, st, &A);
-            if (nee) mcrt::launch_shadow(S, P, ctx->pb, st, &A);
-            qi ^= 1;
+        if (small) {
+            CK(mcrt::launch_paths(S, P, ctx->pb, ctx->small.as<mcrt::SmallScene>(), nullptr, st, &A), "path kernel");
+        } else {
+            mcrt::launch_raygen(S, P, ctx->pb, st, true);
+            qi = 0;
+            for (uint32_t b = 0; b < depth; ++b) {
+                mcrt::launch_extend(S, P, ctx->pb, qi, st, b == 0);
+                mcrt::launch_shade(S, P, ctx->pb, qi, b, nullptr, st, &A);
+                if (nee) mcrt::launch_shadow(S, P, ctx->pb, st, &A);
+                qi ^= 1;
+            }
         }
         done += P.spp_pass;
     }

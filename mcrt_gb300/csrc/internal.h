@@ -65,6 +65,29 @@ struct PathBuffers {
     float4 *sh_g = nullptr;      // per shadow ray: d log(NEE term) / d(albedo rgb | roughness)
 };
 
+// A mesh of at most kSmallTris triangles as the path kernel of small scenes
+// reads it (built on the device, k_small_scene).  Triangles j and j + 1 of the
+// leaf order, j even, with vertex v, edges e1 and e2 and n = e1 x e2, as the
+// pairs (value of j, value of j + 1) of
+//   n.x n.y n.z v.n  -e2.x -e2.y -e2.z  (e2 x v).xyz  e1.xyz  -(e1 x v).xyz;
+// emax and vmax bound the edges' and the vertices' 1-norms.
+constexpr uint32_t kSmallTris = 64;
+constexpr uint32_t kSmallSpheres = 16;   // the path kernel's limit for a scene's spheres
+// Passes of more paths than this take the path kernel only for scenes of at
+// most kFewTris triangles and no sphere.  512x512, depth 8, path kernel / queue
+// kernels: Cornell box (36 triangles) NEE, 64 spp 14.2 / 20.0 ms; 32 spp: 16
+// triangles 0.61 / 0.84, NEE 0.63 / 0.96; a closed mesh of 32 triangles 2.25 /
+// 2.24, of 64 3.80 / 3.26; 64 triangles and 16 spheres, NEE 14.3 / 9.5; 16
+// spheres, NEE 2.4 / 1.9.  160x120, 1 spp, where the queue kernels' launches
+// count: 64 triangles 0.10 / 0.36 ms, with 16 spheres and NEE 0.23 / 0.67.
+constexpr uint32_t kSmallPass = 2u * 896u * 152u, kFewTris = 40;
+struct SmallScene {
+    float4 pair[8 * (kSmallTris / 2)];
+    uint32_t n;
+    float emax, vmax;
+    uint32_t ok;                         // 0: not for the path kernel
+};
+
 // Adjoint (path-replay backpropagation) inputs of the replay kernels.
 struct AdjointParams {
     const float4 *dimg = nullptr;   // dLoss / d(image), per pixel (rgb)
@@ -123,6 +146,11 @@ void launch_shade(const DeviceScene &S, const RenderParams &P, PathBuffers &B, i
                   float4 *gbuf, cudaStream_t st, const AdjointParams *adj = nullptr);
 void launch_shadow(const DeviceScene &S, const RenderParams &P, PathBuffers &B, cudaStream_t st,
                    const AdjointParams *adj = nullptr);
+// Small scenes: the table of the current mesh (ok = 0: not for the path kernel), into device memory.
+void launch_small_scene(const DeviceScene &S, SmallScene *out, cudaStream_t st);
+// Whole paths of a pass in one kernel (in place of raygen, extend, shade and shadow); adj: the replay.
+cudaError_t launch_paths(const DeviceScene &S, const RenderParams &P, PathBuffers &B, const SmallScene *T,
+                         float4 *gbuf, cudaStream_t st, const AdjointParams *adj = nullptr);
 void launch_resolve(const RenderParams &P, const PathBuffers &B, float4 *mean, double *sum, bool keep,
                     cudaStream_t st);
 void launch_tonemap(const float4 *mean, uint32_t npix, uint32_t mode, uchar4 *out, cudaStream_t st);

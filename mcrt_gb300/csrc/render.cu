@@ -449,14 +449,8 @@ __global__ void k_trace_closest(DeviceScene S, const mcrt_ray *rays, uint32_t n,
     hits[i] = h;
 }
 
-__global__ void k_raygen(DeviceScene S, RenderParams P, PathBuffers B, int keep_radiance) {
-    uint32_t n = P.npix * P.spp_pass;
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) {
-        B.counters[0] = n; B.counters[1] = 0; B.counters[2] = 0; B.counters[3] = 0; B.counters[4] = 0;
-        B.counters[5] = 0; B.counters[6] = 0; B.counters[7] = 0;
-    }
-    if (i >= n) return;
+// The camera ray and random state of path slot i of a pass.
+__device__ __forceinline__ void start_path(const RenderParams &P, uint32_t i, f3 *o, f3 *d, uint32_t *rng_out) {
     if (P.cache_query_vertex && i % P.train_stride == 0u) {        // training path: no vertex recorded yet
         float4 *rec = P.train_records + (size_t)(i / P.train_stride) * P.max_depth * kTrainRecordFloat4;
         for (uint32_t j = 0; j < P.max_depth; ++j) rec[(size_t)j * kTrainRecordFloat4].w = 0.0f;
@@ -482,8 +476,21 @@ __global__ void k_raygen(DeviceScene S, RenderParams P, PathBuffers B, int keep_
         x = p % w; y = p / w;
     }
     uint32_t rng = pcg_hash(pcg_hash(x + y * w) ^ (frame * 2654435761u));   // path_trace.wgsl:636-637
+    camera_ray(*cam, x, y, w, h, rng, o, d);
+    *rng_out = rng;
+}
+
+__global__ void k_raygen(DeviceScene S, RenderParams P, PathBuffers B, int keep_radiance) {
+    uint32_t n = P.npix * P.spp_pass;
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        B.counters[0] = n; B.counters[1] = 0; B.counters[2] = 0; B.counters[3] = 0; B.counters[4] = 0;
+        B.counters[5] = 0; B.counters[6] = 0; B.counters[7] = 0;
+    }
+    if (i >= n) return;
     f3 o, d;
-    camera_ray(*cam, x, y, w, h, rng, &o, &d);
+    uint32_t rng;
+    start_path(P, i, &o, &d, &rng);
     B.thr[i] = make_float4(1.0f, 1.0f, 1.0f, -1.0f);
     if (!keep_radiance) B.L[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (keep_radiance) B.pend_mat[i] = 0u;
@@ -662,6 +669,32 @@ __device__ __forceinline__ uint32_t nth_bit(unsigned mask, uint32_t k) {
     return pos;
 }
 
+// Gradient terms of an unoccluded next-event term c of path `slot` (adjoint
+// replay): dlog = its dlog(f)/d(params) for the vertex's material (bits & 0xff),
+// c / albedo for the emitter's radiance colour (bits 8..15; 0xff: the
+// directional light, which has none), as gadd(material, gradient).
+template <class GAdd>
+__device__ __forceinline__ void shadow_gradient(const DeviceScene &S, const AdjointParams &A, uint32_t slot, f3 c,
+                                                uint32_t bits, float4 dlog, GAdd gadd) {
+    const uint32_t mi = bits & 0xffu, lm = (bits >> 8) & 0xffu;
+    const float4 di = A.dimg[slot / A.planes];
+    const f3 dn = (A.inv_spp * xyz(di)) * c;
+    gadd(mi, make_float4(dn.x * dlog.x, dn.y * dlog.y, dn.z * dlog.z, ((dn.x + dn.y) + dn.z) * dlog.w));
+    if (lm <= kMaxMatIdx) {                    // not the directional light
+        const float *la = S.materials->materials[lm].albedo_fuzz;
+        gadd(lm, make_float4(safe_ratio(dn.x, la[0]), safe_ratio(dn.y, la[1]), safe_ratio(dn.z, la[2]), 0.0f));
+    }
+}
+
+// Adds a material's gradient (albedo rgb, roughness) to the block's sums.
+__device__ __forceinline__ void block_gadd(float *gacc, uint32_t mat, float4 g) {
+    float *a = gacc + 4u * mat;
+    if (g.x != 0.0f) atomicAdd(a, g.x);
+    if (g.y != 0.0f) atomicAdd(a + 1, g.y);
+    if (g.z != 0.0f) atomicAdd(a + 2, g.z);
+    if (g.w != 0.0f) atomicAdd(a + 3, g.w);
+}
+
 // The end of a traced queue entry.  Closest hit: the hit record, in queue
 // order.  Any hit (a shadow ray of path `slot`): an unoccluded ray adds its
 // contribution to the path's radiance; ADJ: the adjoint replay's shadow ray,
@@ -681,24 +714,8 @@ __device__ __forceinline__ void finish_ray(const DeviceScene &S, const PathBuffe
             return;
         }
         B.L[slot] = make_float4(L.x - c.x, L.y - c.y, L.z - c.z, 0.0f);
-        auto gadd = [&](uint32_t k, float v) {
-            if (v != 0.0f) atomicAdd(&gacc[k], v);
-        };
-        const uint32_t bits = __float_as_uint(c.w);
-        const uint32_t mi = bits & 0xffu, lm = (bits >> 8) & 0xffu;
-        const float4 di = A.dimg[slot / A.planes];
-        const f3 dn = (A.inv_spp * xyz(di)) * xyz(c);
-        const float4 g = B.sh_g[ray];
-        gadd(4u * mi + 0, dn.x * g.x);
-        gadd(4u * mi + 1, dn.y * g.y);
-        gadd(4u * mi + 2, dn.z * g.z);
-        gadd(4u * mi + 3, ((dn.x + dn.y) + dn.z) * g.w);
-        if (lm <= kMaxMatIdx) {                    // not the directional light
-            const float *la = S.materials->materials[lm].albedo_fuzz;
-            gadd(4u * lm + 0, safe_ratio(dn.x, la[0]));
-            gadd(4u * lm + 1, safe_ratio(dn.y, la[1]));
-            gadd(4u * lm + 2, safe_ratio(dn.z, la[2]));
-        }
+        shadow_gradient(S, A, slot, xyz(c), __float_as_uint(c.w), B.sh_g[ray],
+                        [&](uint32_t mat, float4 g) { block_gadd(gacc, mat, g); });
     } else {
         if (best.prim == MCRT_HIT_MISS) best.t = -1.0f;
         float u = (best.prim != MCRT_HIT_MISS && (best.prim & MCRT_HIT_SPHERE)) ? __uint_as_float(best.slot) : best.u;
@@ -1191,6 +1208,227 @@ __device__ __forceinline__ void record_end(const RenderParams &P, uint32_t slot,
     rec[5] = make_float4(L.x, L.y, L.z, 0.0f);
 }
 
+// What shading a vertex leaves for the kernel around it.
+struct ShadedVertex {
+    bool cont = false, shadow = false, queried = false;   // the path goes on; a shadow ray; a cache query
+    bool scattered = false, vertex = false;               // the throughput changed; a non-emissive surface was hit
+    f3 no, nd;                                            // continuing ray
+    f3 so, sd, sc;                                        // shadow ray and its contribution
+    float smax;
+    uint32_t rng = 0;                                     // random state: in, of the arriving ray; out, of the next
+    float4 cq[4];                                         // radiance-cache query
+    uint32_t sh_bits = 0;                                 // adjoint: material | light material << 8
+    float4 sh_dlog;
+    float4 pend;                                          // adjoint: the BSDF term left pending, of material
+    uint32_t pend_bits = 0;                               // (pend_bits >> 8) - 1
+};
+
+// Adjoint: the BSDF term of a path's previous vertex, of gradient pend and with
+// the radiance L still ahead of the path.
+__device__ __forceinline__ float4 pending_gradient(f3 delta, float4 L, float4 pend) {
+    const f3 dl = delta * xyz(L);
+    return make_float4(dl.x * pend.x, dl.y * pend.y, dl.z * pend.z, ((dl.x + dl.y) + dl.z) * pend.w);
+}
+
+// One vertex of path `slot`: the hit h of its ray (o, d).  get_L / set_L hold
+// the path's radiance; thr4 is its throughput and the last BSDF pdf.
+template <bool ADJ, class GetL, class SetL, class GAdd>
+__device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderParams &P, f3 o, f3 d, float4 h,
+                                             uint32_t slot, uint32_t pixel, uint32_t bounce, bool nee, float4 *gbuf,
+                                             f3 delta, float4 &thr4, ShadedVertex &v, GetL get_L, SetL set_L,
+                                             GAdd gadd) {
+    f3 thr = xyz(thr4);
+    uint32_t &rng = v.rng;
+    const bool write_g = gbuf && bounce == 0 && (int)(slot % P.spp_pass) == P.gbuf_plane;
+    if (h.x < 0.0f) {                                                   // miss, :592-597
+        if (write_g) gbuf[pixel] = make_float4(0.0f, 0.0f, 0.0f, kTMax);
+        if (!ADJ) {
+            f3 e = thr * sample_env(S, d);
+            if (P.cache_query_vertex && slot % P.train_stride == 0u)   // training path ends here
+                record_end(P, slot, bounce, get_L());
+            float4 L = get_L();
+            if (nee) set_L(make_float4(L.x + e.x, L.y + e.y, L.z + e.z, 0.0f));
+            else set_L(make_float4(e.x, e.y, e.z, 0.0f));
+        }
+    } else {
+        SurfaceHit sh = surface(S, o, d, h);
+        if (write_g) gbuf[pixel] = make_float4(sh.n.x, sh.n.y, sh.n.z, sh.t);   // :599-602
+        const uint32_t mi = min(sh.mat, kMaxMatIdx);
+        const mcrt_gpu_material &m = S.materials->materials[mi];
+        const uint32_t mtype = m.type_pad[0];
+        f3 albedo = ld3(m.albedo_fuzz);
+        if (mtype == kMatEmissive) {                                    // :608-610
+            f3 e = m.ior_pad[0] * (thr * albedo);
+            float wmis = 1.0f;
+            if (nee) {
+                if (thr4.w > 0.0f && S.n_lights > 0) {   // pdf <= 0: specular or camera
+                    float pl = light_pdf_of_hit(S, h, o, d);
+                    float pb = thr4.w;
+                    wmis = (pb * pb) / (pb * pb + pl * pl);
+                }
+            }
+            if (ADJ) {                                                  // d E / d(radiance colour)
+                f3 g = (wmis * m.ior_pad[0]) * (delta * thr);
+                gadd(mi, make_float4(g.x, g.y, g.z, 0.0f));
+            } else {
+                if (P.cache_query_vertex && slot % P.train_stride == 0u)   // training path ends here
+                    record_end(P, slot, bounce, get_L());
+                if (nee) {
+                    float4 L = get_L();
+                    set_L(make_float4(L.x + wmis * e.x, L.y + wmis * e.y, L.z + wmis * e.z, 0.0f));
+                } else {
+                    set_L(make_float4(e.x, e.y, e.z, 0.0f));
+                }
+            }
+        } else {
+            albedo = material_albedo(S, m, sh.p, h);                    // :506-515
+            const f3 tex = ADJ ? material_tex(S, m, sh.p, h) : mk3(1.0f, 1.0f, 1.0f);
+            f3 dir = {0, 0, 0}, atten = {0, 0, 0};
+            bool absorbed = false;
+            float pdf = -1.0f;
+            float4 dlw = make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // adjoint: dlog(weight)/d(params)
+            bool has_params = false;
+            if (!ADJ && P.cache_query_vertex) {                         // radiance cache
+                if (slot % P.train_stride == 0u) {                      // training path: record the vertex
+                    float4 *rec = P.train_records +
+                                  ((size_t)(slot / P.train_stride) * P.max_depth + bounce) * kTrainRecordFloat4;
+                    const float4 Lnow = get_L();
+                    rec[0] = make_float4(sh.p.x, sh.p.y, sh.p.z, 1.0f);
+                    rec[1] = make_float4(-d.x, -d.y, -d.z, 0.0f);
+                    rec[2] = make_float4(sh.n.x, sh.n.y, sh.n.z, 0.0f);
+                    rec[3] = make_float4(albedo.x, albedo.y, albedo.z, 0.0f);
+                    rec[4] = make_float4(thr.x, thr.y, thr.z, 0.0f);
+                    rec[5] = make_float4(Lnow.x, Lnow.y, Lnow.z, 0.0f);
+                } else if (bounce + 1 == P.cache_query_vertex) {        // stop here: ask the cache
+                    v.queried = true;
+                    v.cq[0] = make_float4(sh.p.x, sh.p.y, sh.p.z, __uint_as_float(slot));
+                    v.cq[1] = make_float4(-d.x, -d.y, -d.z, 0.0f);
+                    v.cq[2] = make_float4(sh.n.x, sh.n.y, sh.n.z, 0.0f);
+                    v.cq[3] = make_float4(albedo.x, albedo.y, albedo.z, 0.0f);
+                }
+            }
+            if (mtype == kMatMetal) {                                   // :530-541
+                float fuzz = m.albedo_fuzz[3];
+                f3 refl = reflect_vec(normalize(d), sh.n);
+                f3 pert = refl + fuzz * random_unit_sphere(rng);
+                dir = normalize(dot(pert, pert) >= 1e-6f ? pert : refl);
+                atten = albedo;
+                absorbed = dot(dir, sh.n) <= 0.0f;
+                if (ADJ) {
+                    dlw = make_float4(safe_ratio(tex.x, albedo.x), safe_ratio(tex.y, albedo.y),
+                                      safe_ratio(tex.z, albedo.z), 0.0f);
+                    has_params = true;
+                }
+            } else if (mtype == kMatDielectric) {                       // :543-564
+                atten = mk3(1.0f, 1.0f, 1.0f);
+                float ior = m.ior_pad[0];
+                float eta = sh.front ? 1.0f / ior : ior;
+                float cos_t = fminf(dot(-d, sh.n), 1.0f);
+                float sin_t = sqrtf(fmaxf(0.0f, 1.0f - cos_t * cos_t));
+                bool cannot = eta * sin_t > 1.0f;
+                float scos = (!sh.front && !cannot)
+                                 ? sqrtf(fmaxf(0.0f, 1.0f - (eta * eta) * (1.0f - cos_t * cos_t)))
+                                 : cos_t;
+                float refl = schlick(scos, eta);
+                if (cannot || refl > rand_f32(rng)) dir = reflect_vec(d, sh.n);
+                else dir = normalize(refract_vec(d, sh.n, eta));
+            } else if (mtype == kMatGgx) {
+                f3 t, b;
+                onb(sh.n, &t, &b);
+                f3 wo = mk3(-dot(d, t), -dot(d, b), -dot(d, sh.n));
+                float rough = m.albedo_fuzz[3];
+                float alpha = fmaxf(rough * rough, 1e-4f);
+                const float dadr = rough * rough > 1e-4f ? 2.0f * rough : 0.0f;
+                float r1 = rand_f32(rng), r2 = rand_f32(rng);
+                f3 wi, wgt;
+                float gpdf, mz = 0.0f, fw = 0.0f;
+                if (wo.z > 0.0f && ggx_sample(wo, alpha, albedo, r1, r2, &wi, &wgt, &gpdf, &mz, &fw)) {
+                    dir = normalize((wi.x * t + wi.y * b) + wi.z * sh.n);
+                    atten = wgt;
+                    pdf = gpdf;
+                    if (ADJ) {
+                        const f3 one = mk3(1.0f, 1.0f, 1.0f);
+                        f3 F = albedo + fw * (one - albedo);
+                        dlw = make_float4(safe_ratio((1.0f - fw) * tex.x, F.x),
+                                          safe_ratio((1.0f - fw) * tex.y, F.y),
+                                          safe_ratio((1.0f - fw) * tex.z, F.z),
+                                          ggx_dlog_dalpha(alpha, mz, wo.z, wi.z) * dadr);
+                        has_params = true;
+                    }
+                    if (nee) {                                          // light sample at a GGX vertex
+                        LightSample ls = sample_light(S, sh.p, rng);
+                        if (ls.ok) {
+                            f3 wl = mk3(dot(ls.dir, t), dot(ls.dir, b), dot(ls.dir, sh.n));
+                            float bp, lmz = 0.0f, lfw = 0.0f;
+                            f3 fc = ggx_eval(wo, wl, alpha, albedo, &bp, &lmz, &lfw);
+                            if (wl.z > 0.0f && (fc.x > 0.0f || fc.y > 0.0f || fc.z > 0.0f)) {
+                                float wmis = ls.delta ? 1.0f : (ls.pdf * ls.pdf) / (ls.pdf * ls.pdf + bp * bp);
+                                v.sc = (wmis / ls.pdf) * (thr * (fc * ls.Le));
+                                v.so = sh.p; v.sd = ls.dir; v.smax = ls.dist * (1.0f - 1e-4f);
+                                v.shadow = true;
+                                if (ADJ) {
+                                    const f3 one = mk3(1.0f, 1.0f, 1.0f);
+                                    f3 F = albedo + lfw * (one - albedo);
+                                    v.sh_dlog = make_float4(safe_ratio((1.0f - lfw) * tex.x, F.x),
+                                                          safe_ratio((1.0f - lfw) * tex.y, F.y),
+                                                          safe_ratio((1.0f - lfw) * tex.z, F.z),
+                                                          ggx_dlog_dalpha(alpha, lmz, wo.z, wl.z) * dadr);
+                                    v.sh_bits = mi | (ls.mat << 8);
+                                }
+                            }
+                        }
+                    }
+                } else {
+                    absorbed = true;
+                }
+            } else {                                                    // :521-528
+                if (nee) {
+                    LightSample ls = sample_light(S, sh.p, rng);
+                    float cs = dot(ls.dir, sh.n);
+                    if (ls.ok && cs > 0.0f) {
+                        float bp = cs / kPi;
+                        float wmis = ls.delta ? 1.0f : (ls.pdf * ls.pdf) / (ls.pdf * ls.pdf + bp * bp);
+                        v.sc = (wmis * bp / ls.pdf) * (thr * (albedo * ls.Le));
+                        v.so = sh.p; v.sd = ls.dir; v.smax = ls.dist * (1.0f - 1e-4f);
+                        v.shadow = true;
+                        if (ADJ) {
+                            v.sh_dlog = make_float4(safe_ratio(tex.x, albedo.x), safe_ratio(tex.y, albedo.y),
+                                                  safe_ratio(tex.z, albedo.z), 0.0f);
+                            v.sh_bits = mi | (ls.mat << 8);
+                        }
+                    }
+                }
+                dir = cosine_scatter(rng, sh.n);
+                atten = albedo;
+                pdf = fmaxf(dot(dir, sh.n), 0.0f) / kPi;
+                if (ADJ) {
+                    dlw = make_float4(safe_ratio(tex.x, albedo.x), safe_ratio(tex.y, albedo.y),
+                                      safe_ratio(tex.z, albedo.z), 0.0f);
+                    has_params = true;
+                }
+            }
+            // a cache stop keeps this vertex's light sample (above) and ends
+            // the path: the cache stands for what BSDF sampling would gather
+            if (v.queried) absorbed = true;
+            if (!absorbed) {
+                thr = thr * atten;
+                if (bounce + 1 < P.max_depth) {
+                    v.cont = true;
+                    v.no = sh.p;
+                    v.nd = dir;
+                    if (ADJ && has_params) {
+                        v.pend = dlw;
+                        v.pend_bits = (mi + 1u) << 8;
+                    }
+                }
+                thr4 = make_float4(thr.x, thr.y, thr.z, pdf);
+                v.scattered = true;
+            }
+            v.vertex = true;
+        }
+    }
+}
+
 template <bool ADJ>
 __global__ void __launch_bounds__(256, ADJ ? 2 : 4) k_shade(DeviceScene S, RenderParams P, PathBuffers B, int qi,
                                                 uint32_t bounce, float4 *gbuf, AdjointParams A) {
@@ -1199,9 +1437,6 @@ __global__ void __launch_bounds__(256, ADJ ? 2 : 4) k_shade(DeviceScene S, Rende
         gacc[threadIdx.x] = 0.0f;
         __syncthreads();
     }
-    auto gadd = [&](uint32_t k, float v) {
-        if (ADJ && v != 0.0f) atomicAdd(&gacc[k], v);
-    };
     const uint32_t n = B.counters[qi];
     const bool nee = (P.flags & MCRT_RENDER_NEE) != 0 && (S.n_lights > 0 || S.has_sun);
     const uint32_t lane = threadIdx.x & 31u;
@@ -1211,270 +1446,70 @@ __global__ void __launch_bounds__(256, ADJ ? 2 : 4) k_shade(DeviceScene S, Rende
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t i = base + threadIdx.x;
-        bool cont = false, shadow = false, queried = false;
-        f3 no = {0, 0, 0}, nd = {0, 0, 0}, so = {0, 0, 0}, sd = {0, 0, 0}, sc = {0, 0, 0};
-        float4 cq0, cq1, cq2, cq3;             // radiance-cache query of this path
-        float smax = 0.0f;
+        ShadedVertex v;
         uint32_t slot = 0;
-        uint32_t rng_next = 0;                 // random state of the continuing ray
-        uint32_t sh_bits = 0;                  // adjoint: material | light material << 8
-        float4 sh_dlog = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (i < n) {
             // the queues and hits are streamed once per bounce (GBs per frame):
             // cache-streaming accesses keep them from evicting the BVH in L2
             float4 o4 = __ldcs(B.q_o[qi] + i), d4 = __ldcs(B.q_d[qi] + i);
             float4 h = __ldcs(B.hits + i);
             slot = __float_as_uint(o4.w);
-            f3 o = xyz(o4), d = xyz(d4);
             float4 thr4 = B.thr[slot];
+            v.rng = __float_as_uint(d4.w);
             const uint32_t pixel = slot / P.spp_pass;
-            f3 thr = xyz(thr4);
-            uint32_t rng = __float_as_uint(d4.w);
             f3 delta = {0.0f, 0.0f, 0.0f};
             if (ADJ) {
-                float4 di = A.dimg[pixel];
-                delta = A.inv_spp * xyz(di);
+                delta = A.inv_spp * xyz(A.dimg[pixel]);
                 const uint32_t pm = (B.pend_mat[slot] >> 8) & 0xffu;
-                if (pm) {                                   // BSDF term of the previous vertex
-                    float4 L = B.L[slot], pd = B.pend[slot];
-                    const uint32_t k0 = 4u * (pm - 1u);
-                    f3 dl = delta * xyz(L);
-                    gadd(k0 + 0, dl.x * pd.x);
-                    gadd(k0 + 1, dl.y * pd.y);
-                    gadd(k0 + 2, dl.z * pd.z);
-                    gadd(k0 + 3, ((dl.x + dl.y) + dl.z) * pd.w);
-                }
+                if (pm) block_gadd(gacc, pm - 1u, pending_gradient(delta, B.L[slot], B.pend[slot]));
             }
-            const bool write_g = gbuf && bounce == 0 && (int)(slot % P.spp_pass) == P.gbuf_plane;
-            if (h.x < 0.0f) {                                                   // miss, :592-597
-                if (write_g) gbuf[pixel] = make_float4(0.0f, 0.0f, 0.0f, kTMax);
-                if (!ADJ) {
-                    f3 e = thr * sample_env(S, d);
-                    if (P.cache_query_vertex && slot % P.train_stride == 0u)   // training path ends here
-                        record_end(P, slot, bounce, B.L[slot]);
-                    float4 L = B.L[slot];
-                    if (nee) B.L[slot] = make_float4(L.x + e.x, L.y + e.y, L.z + e.z, 0.0f);
-                    else B.L[slot] = make_float4(e.x, e.y, e.z, 0.0f);
-                }
-            } else {
-                SurfaceHit sh = surface(S, o, d, h);
-                if (write_g) gbuf[pixel] = make_float4(sh.n.x, sh.n.y, sh.n.z, sh.t);   // :599-602
-                const uint32_t mi = min(sh.mat, kMaxMatIdx);
-                const mcrt_gpu_material &m = S.materials->materials[mi];
-                const uint32_t mtype = m.type_pad[0];
-                f3 albedo = ld3(m.albedo_fuzz);
-                if (mtype == kMatEmissive) {                                    // :608-610
-                    f3 e = m.ior_pad[0] * (thr * albedo);
-                    float wmis = 1.0f;
-                    if (nee) {
-                        if (thr4.w > 0.0f && S.n_lights > 0) {   // pdf <= 0: specular or camera
-                            float pl = light_pdf_of_hit(S, h, o, d);
-                            float pb = thr4.w;
-                            wmis = (pb * pb) / (pb * pb + pl * pl);
-                        }
-                    }
-                    if (ADJ) {                                                  // d E / d(radiance colour)
-                        f3 g = (wmis * m.ior_pad[0]) * (delta * thr);
-                        gadd(4u * mi + 0, g.x);
-                        gadd(4u * mi + 1, g.y);
-                        gadd(4u * mi + 2, g.z);
-                    } else {
-                        if (P.cache_query_vertex && slot % P.train_stride == 0u)   // training path ends here
-                            record_end(P, slot, bounce, B.L[slot]);
-                        if (nee) {
-                            float4 L = B.L[slot];
-                            B.L[slot] = make_float4(L.x + wmis * e.x, L.y + wmis * e.y, L.z + wmis * e.z, 0.0f);
-                        } else {
-                            B.L[slot] = make_float4(e.x, e.y, e.z, 0.0f);
-                        }
-                    }
-                } else {
-                    albedo = material_albedo(S, m, sh.p, h);                    // :506-515
-                    const f3 tex = ADJ ? material_tex(S, m, sh.p, h) : mk3(1.0f, 1.0f, 1.0f);
-                    f3 dir = {0, 0, 0}, atten = {0, 0, 0};
-                    bool absorbed = false;
-                    float pdf = -1.0f;
-                    float4 dlw = make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // adjoint: dlog(weight)/d(params)
-                    bool has_params = false;
-                    if (!ADJ && P.cache_query_vertex) {                         // radiance cache
-                        if (slot % P.train_stride == 0u) {                      // training path: record the vertex
-                            float4 *rec = P.train_records +
-                                          ((size_t)(slot / P.train_stride) * P.max_depth + bounce) * kTrainRecordFloat4;
-                            const float4 Lnow = B.L[slot];
-                            rec[0] = make_float4(sh.p.x, sh.p.y, sh.p.z, 1.0f);
-                            rec[1] = make_float4(-d.x, -d.y, -d.z, 0.0f);
-                            rec[2] = make_float4(sh.n.x, sh.n.y, sh.n.z, 0.0f);
-                            rec[3] = make_float4(albedo.x, albedo.y, albedo.z, 0.0f);
-                            rec[4] = make_float4(thr.x, thr.y, thr.z, 0.0f);
-                            rec[5] = make_float4(Lnow.x, Lnow.y, Lnow.z, 0.0f);
-                        } else if (bounce + 1 == P.cache_query_vertex) {        // stop here: ask the cache
-                            queried = true;
-                            cq0 = make_float4(sh.p.x, sh.p.y, sh.p.z, __uint_as_float(slot));
-                            cq1 = make_float4(-d.x, -d.y, -d.z, 0.0f);
-                            cq2 = make_float4(sh.n.x, sh.n.y, sh.n.z, 0.0f);
-                            cq3 = make_float4(albedo.x, albedo.y, albedo.z, 0.0f);
-                        }
-                    }
-                    if (mtype == kMatMetal) {                                   // :530-541
-                        float fuzz = m.albedo_fuzz[3];
-                        f3 refl = reflect_vec(normalize(d), sh.n);
-                        f3 pert = refl + fuzz * random_unit_sphere(rng);
-                        dir = normalize(dot(pert, pert) >= 1e-6f ? pert : refl);
-                        atten = albedo;
-                        absorbed = dot(dir, sh.n) <= 0.0f;
-                        if (ADJ) {
-                            dlw = make_float4(safe_ratio(tex.x, albedo.x), safe_ratio(tex.y, albedo.y),
-                                              safe_ratio(tex.z, albedo.z), 0.0f);
-                            has_params = true;
-                        }
-                    } else if (mtype == kMatDielectric) {                       // :543-564
-                        atten = mk3(1.0f, 1.0f, 1.0f);
-                        float ior = m.ior_pad[0];
-                        float eta = sh.front ? 1.0f / ior : ior;
-                        float cos_t = fminf(dot(-d, sh.n), 1.0f);
-                        float sin_t = sqrtf(fmaxf(0.0f, 1.0f - cos_t * cos_t));
-                        bool cannot = eta * sin_t > 1.0f;
-                        float scos = (!sh.front && !cannot)
-                                         ? sqrtf(fmaxf(0.0f, 1.0f - (eta * eta) * (1.0f - cos_t * cos_t)))
-                                         : cos_t;
-                        float refl = schlick(scos, eta);
-                        if (cannot || refl > rand_f32(rng)) dir = reflect_vec(d, sh.n);
-                        else dir = normalize(refract_vec(d, sh.n, eta));
-                    } else if (mtype == kMatGgx) {
-                        f3 t, b;
-                        onb(sh.n, &t, &b);
-                        f3 wo = mk3(-dot(d, t), -dot(d, b), -dot(d, sh.n));
-                        float rough = m.albedo_fuzz[3];
-                        float alpha = fmaxf(rough * rough, 1e-4f);
-                        const float dadr = rough * rough > 1e-4f ? 2.0f * rough : 0.0f;
-                        float r1 = rand_f32(rng), r2 = rand_f32(rng);
-                        f3 wi, wgt;
-                        float gpdf, mz = 0.0f, fw = 0.0f;
-                        if (wo.z > 0.0f && ggx_sample(wo, alpha, albedo, r1, r2, &wi, &wgt, &gpdf, &mz, &fw)) {
-                            dir = normalize((wi.x * t + wi.y * b) + wi.z * sh.n);
-                            atten = wgt;
-                            pdf = gpdf;
-                            if (ADJ) {
-                                const f3 one = mk3(1.0f, 1.0f, 1.0f);
-                                f3 F = albedo + fw * (one - albedo);
-                                dlw = make_float4(safe_ratio((1.0f - fw) * tex.x, F.x),
-                                                  safe_ratio((1.0f - fw) * tex.y, F.y),
-                                                  safe_ratio((1.0f - fw) * tex.z, F.z),
-                                                  ggx_dlog_dalpha(alpha, mz, wo.z, wi.z) * dadr);
-                                has_params = true;
-                            }
-                            if (nee) {                                          // light sample at a GGX vertex
-                                LightSample ls = sample_light(S, sh.p, rng);
-                                if (ls.ok) {
-                                    f3 wl = mk3(dot(ls.dir, t), dot(ls.dir, b), dot(ls.dir, sh.n));
-                                    float bp, lmz = 0.0f, lfw = 0.0f;
-                                    f3 fc = ggx_eval(wo, wl, alpha, albedo, &bp, &lmz, &lfw);
-                                    if (wl.z > 0.0f && (fc.x > 0.0f || fc.y > 0.0f || fc.z > 0.0f)) {
-                                        float wmis = ls.delta ? 1.0f : (ls.pdf * ls.pdf) / (ls.pdf * ls.pdf + bp * bp);
-                                        sc = (wmis / ls.pdf) * (thr * (fc * ls.Le));
-                                        so = sh.p; sd = ls.dir; smax = ls.dist * (1.0f - 1e-4f);
-                                        shadow = true;
-                                        if (ADJ) {
-                                            const f3 one = mk3(1.0f, 1.0f, 1.0f);
-                                            f3 F = albedo + lfw * (one - albedo);
-                                            sh_dlog = make_float4(safe_ratio((1.0f - lfw) * tex.x, F.x),
-                                                                  safe_ratio((1.0f - lfw) * tex.y, F.y),
-                                                                  safe_ratio((1.0f - lfw) * tex.z, F.z),
-                                                                  ggx_dlog_dalpha(alpha, lmz, wo.z, wl.z) * dadr);
-                                            sh_bits = mi | (ls.mat << 8);
-                                        }
-                                    }
-                                }
-                            }
-                        } else {
-                            absorbed = true;
-                        }
-                    } else {                                                    // :521-528
-                        if (nee) {
-                            LightSample ls = sample_light(S, sh.p, rng);
-                            float cs = dot(ls.dir, sh.n);
-                            if (ls.ok && cs > 0.0f) {
-                                float bp = cs / kPi;
-                                float wmis = ls.delta ? 1.0f : (ls.pdf * ls.pdf) / (ls.pdf * ls.pdf + bp * bp);
-                                sc = (wmis * bp / ls.pdf) * (thr * (albedo * ls.Le));
-                                so = sh.p; sd = ls.dir; smax = ls.dist * (1.0f - 1e-4f);
-                                shadow = true;
-                                if (ADJ) {
-                                    sh_dlog = make_float4(safe_ratio(tex.x, albedo.x), safe_ratio(tex.y, albedo.y),
-                                                          safe_ratio(tex.z, albedo.z), 0.0f);
-                                    sh_bits = mi | (ls.mat << 8);
-                                }
-                            }
-                        }
-                        dir = cosine_scatter(rng, sh.n);
-                        atten = albedo;
-                        pdf = fmaxf(dot(dir, sh.n), 0.0f) / kPi;
-                        if (ADJ) {
-                            dlw = make_float4(safe_ratio(tex.x, albedo.x), safe_ratio(tex.y, albedo.y),
-                                              safe_ratio(tex.z, albedo.z), 0.0f);
-                            has_params = true;
-                        }
-                    }
-                    // a cache stop keeps this vertex's light sample (above) and ends
-                    // the path: the cache stands for what BSDF sampling would gather
-                    if (queried) absorbed = true;
-                    uint32_t pend_bits = 0;
-                    if (!absorbed) {
-                        thr = thr * atten;
-                        if (bounce + 1 < P.max_depth) {
-                            cont = true;
-                            no = sh.p;
-                            nd = dir;
-                            if (ADJ && has_params) {
-                                B.pend[slot] = dlw;
-                                pend_bits = (mi + 1u) << 8;
-                            }
-                        }
-                        B.thr[slot] = make_float4(thr.x, thr.y, thr.z, pdf);
-                    }
-                    if (ADJ) B.pend_mat[slot] = pend_bits;
-                    rng_next = rng;
-                }
+            shade_vertex<ADJ>(S, P, xyz(o4), xyz(d4), h, slot, pixel, bounce, nee, gbuf, delta, thr4, v,
+                              [&]() { return B.L[slot]; }, [&](float4 L) { B.L[slot] = L; },
+                              [&](uint32_t mat, float4 g) { block_gadd(gacc, mat, g); });
+            if (v.scattered) B.thr[slot] = thr4;
+            if (ADJ && v.vertex) {
+                B.pend_mat[slot] = v.pend_bits;
+                if (v.pend_bits) B.pend[slot] = v.pend;
             }
         }
         // warp-aggregated append to the next ray queue
-        unsigned mask = __ballot_sync(0xffffffffu, cont);
+        unsigned mask = __ballot_sync(0xffffffffu, v.cont);
         if (mask) {
             int leader = __ffs(mask) - 1;
             uint32_t basepos = 0;
             if ((int)lane == leader) basepos = atomicAdd(B.counters + (qi ^ 1), (uint32_t)__popc(mask));
             basepos = __shfl_sync(0xffffffffu, basepos, leader);
-            if (cont) {
+            if (v.cont) {
                 uint32_t pos = basepos + __popc(mask & ((1u << lane) - 1u));
-                __stcs(B.q_o[qi ^ 1] + pos, make_float4(no.x, no.y, no.z, __uint_as_float(slot)));
-                __stcs(B.q_d[qi ^ 1] + pos, make_float4(nd.x, nd.y, nd.z, __uint_as_float(rng_next)));
+                __stcs(B.q_o[qi ^ 1] + pos, make_float4(v.no.x, v.no.y, v.no.z, __uint_as_float(slot)));
+                __stcs(B.q_d[qi ^ 1] + pos, make_float4(v.nd.x, v.nd.y, v.nd.z, __uint_as_float(v.rng)));
             }
         }
-        unsigned smask = __ballot_sync(0xffffffffu, shadow);
+        unsigned smask = __ballot_sync(0xffffffffu, v.shadow);
         if (smask) {
             int leader = __ffs(smask) - 1;
             uint32_t basepos = 0;
             if ((int)lane == leader) basepos = atomicAdd(B.counters + 2, (uint32_t)__popc(smask));
             basepos = __shfl_sync(0xffffffffu, basepos, leader);
-            if (shadow) {
+            if (v.shadow) {
                 uint32_t pos = basepos + __popc(smask & ((1u << lane) - 1u));
-                B.sh_o[pos] = make_float4(so.x, so.y, so.z, __uint_as_float(slot));
-                B.sh_d[pos] = make_float4(sd.x, sd.y, sd.z, smax);
-                B.sh_c[pos] = make_float4(sc.x, sc.y, sc.z, __uint_as_float(sh_bits));
-                if (ADJ) B.sh_g[pos] = sh_dlog;
+                B.sh_o[pos] = make_float4(v.so.x, v.so.y, v.so.z, __uint_as_float(slot));
+                B.sh_d[pos] = make_float4(v.sd.x, v.sd.y, v.sd.z, v.smax);
+                B.sh_c[pos] = make_float4(v.sc.x, v.sc.y, v.sc.z, __uint_as_float(v.sh_bits));
+                if (ADJ) B.sh_g[pos] = v.sh_dlog;
             }
         }
         if (!ADJ && P.cache_query_vertex) {
-            unsigned qmask = __ballot_sync(0xffffffffu, queried);
+            unsigned qmask = __ballot_sync(0xffffffffu, v.queried);
             if (qmask) {
                 int leader = __ffs(qmask) - 1;
                 uint32_t basepos = 0;
                 if ((int)lane == leader) basepos = atomicAdd(B.counters + 6, (uint32_t)__popc(qmask));
                 basepos = __shfl_sync(0xffffffffu, basepos, leader);
-                if (queried) {
+                if (v.queried) {
                     uint32_t pos = basepos + __popc(qmask & ((1u << lane) - 1u));
                     float4 *q = P.cache_queries + 4 * (size_t)pos;
-                    q[0] = cq0; q[1] = cq1; q[2] = cq2; q[3] = cq3;
+                    for (int k = 0; k < 4; ++k) q[k] = v.cq[k];
                 }
             }
         }
@@ -1483,6 +1518,441 @@ __global__ void __launch_bounds__(256, ADJ ? 2 : 4) k_shade(DeviceScene S, Rende
         __syncthreads();
         const float v = gacc[threadIdx.x];
         if (v != 0.0f) atomicAdd(A.grad + threadIdx.x, (double)v);
+    }
+}
+
+// ------------------------------------------------------------------ small scenes
+// Scenes of at most kSmallTris triangles and kSmallSpheres spheres: one kernel
+// traces whole paths, one per lane.
+//
+// With so few triangles the tree costs more than it saves: in the Cornell box
+// (36 triangles) a ray of the queue kernels took 4,200 scheduler cycles per
+// warp, most of them in divergent node visits and stack traffic, and every
+// bounce carried 200 bytes of path state through HBM and three launches.
+// Here each lane tests every triangle with a conservative test (15
+// multiply-adds, no division, all lanes together) and takes only the few that
+// can be hit through the exact one, and the state of a path stays in registers.
+// The table of the mesh and whether it may be used: a tree of at most
+// 2 kSmallTris - 1 nodes that reaches every triangle slot once, each box inside
+// its parent's (then a triangle is reached exactly when its leaf's box is
+// entered), and finite coordinates of moderate size.  One block of 2 kSmallTris
+// threads, a node and a triangle each.
+__global__ void __launch_bounds__(2 * kSmallTris) k_small_scene(DeviceScene S, SmallScene *out) {
+    __shared__ uint32_t covered[kSmallTris], parents[2 * kSmallTris];
+    __shared__ uint32_t bad;
+    __shared__ float red[2][kSmallTris];
+    const uint32_t t = threadIdx.x;
+    if (t < kSmallTris) { covered[t] = 0; red[0][t] = red[1][t] = 0.0f; }
+    parents[t] = 0;
+    if (t == 0) bad = (S.n_triangles > kSmallTris || S.n_mesh_nodes >= 2 * kSmallTris) ? 1u : 0u;
+    __syncthreads();
+    const float limit = 1e9f;
+    auto fits = [&](float x) { return fabsf(x) <= limit; };       // false for NaN
+    if (!bad && t < S.n_mesh_nodes) {
+        const mcrt_gpu_bvh_node nd = S.mesh_nodes[t];
+        for (int a = 0; a < 3; ++a)
+            if (!fits(nd.aabb_min[a]) || !fits(nd.aabb_max[a])) bad = 1u;
+        if (nd.prim_count) {
+            for (uint32_t k = 0; k < nd.prim_count; ++k)
+                if (nd.right_or_offset + k < kSmallTris) atomicAdd(&covered[nd.right_or_offset + k], 1u);
+        } else {
+            const uint32_t kids[2] = {t + 1u, nd.right_or_offset};
+            for (int c = 0; c < 2; ++c) {
+                if (kids[c] >= S.n_mesh_nodes) { bad = 1u; continue; }
+                atomicAdd(&parents[kids[c]], 1u);
+                const mcrt_gpu_bvh_node ch = S.mesh_nodes[kids[c]];
+                for (int a = 0; a < 3; ++a)
+                    if (!(ch.aabb_min[a] >= nd.aabb_min[a] && ch.aabb_max[a] <= nd.aabb_max[a])) bad = 1u;
+            }
+        }
+    }
+    float q[16] = {};
+    if (t < S.n_triangles && t < kSmallTris) {
+        const TriRec r = S.tris[t];
+        const double v[3] = {r.v0.x, r.v0.y, r.v0.z}, e1[3] = {r.e1.x, r.e1.y, r.e1.z}, e2[3] = {r.e2.x, r.e2.y, r.e2.z};
+        double k = 0.0;
+        float ve = 0.0f, le1 = 0.0f, le2 = 0.0f;
+        for (int a = 0; a < 3; ++a) {
+            const int b = (a + 1) % 3, c = (a + 2) % 3;
+            const double n = e1[b] * e2[c] - e1[c] * e2[b];
+            k += v[a] * n;
+            q[a] = (float)n;
+            q[4 + a] = (float)-e2[a];
+            q[7 + a] = (float)(e2[b] * v[c] - e2[c] * v[b]);
+            q[10 + a] = (float)e1[a];
+            q[13 + a] = (float)(e1[c] * v[b] - e1[b] * v[c]);
+            if (!fits((float)v[a]) || !fits((float)e1[a]) || !fits((float)e2[a])) bad = 1u;
+            ve += fabsf((float)v[a]); le1 += fabsf((float)e1[a]); le2 += fabsf((float)e2[a]);
+        }
+        q[3] = (float)k;
+        red[0][t] = fmaxf(le1, le2);
+        red[1][t] = ve;
+    }
+    __syncthreads();
+    if (t < S.n_triangles && t < kSmallTris && covered[t] != 1u) bad = 1u;
+    if (t > 0 && t < S.n_mesh_nodes && parents[t] != 1u) bad = 1u;
+    __syncthreads();
+    if (t < kSmallTris) {
+        float *pair = reinterpret_cast<float *>(out->pair + 8u * (t >> 1)) + (t & 1u);
+        for (int k = 0; k < 16; ++k) pair[2 * k] = q[k];
+    }
+    if (t == 0) {
+        float emax = 0.0f, vmax = 0.0f;
+        for (uint32_t k = 0; k < kSmallTris; ++k) { emax = fmaxf(emax, red[0][k]); vmax = fmaxf(vmax, red[1][k]); }
+        out->n = min(S.n_triangles, kSmallTris);
+        out->emax = emax;
+        out->vmax = vmax + emax;
+        out->ok = bad ? 0u : 1u;
+    }
+}
+
+// Two values in one 64-bit register pair: the packed f32x2 instructions.
+__device__ __forceinline__ uint64_t pk2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// One ray of the conservative test: direction and moment o x d, each doubled.
+struct PackedRay {
+    uint64_t d[3], m[3];
+    float tol;
+};
+__device__ __forceinline__ PackedRay pack_ray(f3 o, f3 d, float emax, float vmax) {
+    const f3 m = cross(o, d);
+    const float ov = ((fabsf(o.x) + fabsf(o.y)) + fabsf(o.z)) + vmax;
+    const float dl = (fabsf(d.x) + fabsf(d.y)) + fabsf(d.z);
+    PackedRay r;
+    r.d[0] = pk2(d.x, d.x); r.d[1] = pk2(d.y, d.y); r.d[2] = pk2(d.z, d.z);
+    r.m[0] = pk2(m.x, m.x); r.m[1] = pk2(m.y, m.y); r.m[2] = pk2(m.z, m.z);
+    r.tol = (3.814697265625e-6f * emax) * (dl * ov + emax * (dl + ov));
+    return r;
+}
+
+// The triangles that the exact test (tri_test) can accept for the rays (o, d0)
+// and, with TWO, the shadow ray (o, d1) up to tmax, as two words of bits each.
+// Cramer's rule without the division: with m = o x d,
+//   a = d.n,  u a = d.(e2 x v) - m.e2,  v a = m.e1 - d.(e1 x v),  t a = v.n - o.n
+// (n = e1 x e2; all four signs turned), each within tol of what the exact test
+// has before its divisions: both sides sum at most 12 products whose rounding
+// errors are relative 2^-24 of terms bounded by |d| emax (|o| + vmax), |d| emax^2
+// and emax^2 (|o| + vmax) (1-norms), with at most 28 roundings in all; 2^-18 is
+// 2.3 times those.  Accepted means u >= 0, v >= 0, u + v <= 1,
+// t >= t_min > 0 (and t < tmax), each after one rounded product, which the
+// 1e-5 |a| covers.  A NaN keeps its triangle.
+// Two triangles go through each packed instruction, and a triangle pair's 128
+// bytes of shared memory serve both rays: with the table in the constant bank
+// and one ray at a time the constant loads alone kept the kernel at 54 % of its
+// issue slots (21.8 ms for the Cornell box of k_paths).  The loop stays rolled:
+// unrolled twice it took 18.5 ms against 16.8.
+template <bool TWO>
+__device__ __forceinline__ void small_candidates(const float4 *s_pair, uint32_t n, const uint64_t no[3],
+                                                 const PackedRay &r0, const PackedRay &r1, float tmax, uint2 *c0,
+                                                 uint2 *c1) {
+    auto outside = [](float a, float u, float v, float t, float tol, bool any, float tmax) {
+        const uint32_t sign = __float_as_uint(a) & 0x80000000u;
+        const float us = __uint_as_float(__float_as_uint(u) ^ sign), vs = __uint_as_float(__float_as_uint(v) ^ sign);
+        const float ts = __uint_as_float(__float_as_uint(t) ^ sign);
+        const float aa = fabsf(a), slack = fmaf(aa, 1e-5f, tol);
+        float low = fminf(min3(us, vs, (aa - us) - vs), ts);
+        if (any) low = fminf(low, fmaf(aa + slack, tmax, -ts));
+        return low < -slack;
+    };
+    uint32_t w0[2] = {0u, 0u}, w1[2] = {0u, 0u};
+#pragma unroll
+    for (uint32_t w = 0; w < 2; ++w) {
+        const uint32_t cnt = n > 32u * w ? min(n - 32u * w, 32u) : 0u;
+        uint32_t b0 = 0u, b1 = 0u;
+#pragma unroll 1
+        for (uint32_t k = 0; k < cnt; k += 2) {
+            const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(s_pair + 4u * (32u * w + k));
+            const ulonglong2 nxy = q[0], nzk = q[1], e2xy = q[2], e2zc2x = q[3], c2yz = q[4], e1xy = q[5], e1zc1x = q[6],
+                             c1yz = q[7];
+            const uint64_t t = fma2(no[0], nxy.x, fma2(no[1], nxy.y, fma2(no[2], nzk.x, nzk.y)));
+            auto one = [&](const PackedRay &r, bool any) {
+                const uint64_t a = fma2(r.d[0], nxy.x, fma2(r.d[1], nxy.y, mul2(r.d[2], nzk.x)));
+                const uint64_t u = fma2(r.d[0], e2zc2x.y, fma2(r.d[1], c2yz.x, fma2(r.d[2], c2yz.y,
+                                   fma2(r.m[0], e2xy.x, fma2(r.m[1], e2xy.y, mul2(r.m[2], e2zc2x.x))))));
+                const uint64_t v = fma2(r.d[0], e1zc1x.y, fma2(r.d[1], c1yz.x, fma2(r.d[2], c1yz.y,
+                                   fma2(r.m[0], e1xy.x, fma2(r.m[1], e1xy.y, mul2(r.m[2], e1zc1x.x))))));
+                uint32_t bits = 0u;
+                if (!outside(lo2(a), lo2(u), lo2(v), lo2(t), r.tol, any, tmax)) bits |= 1u << k;
+                if (!outside(hi2(a), hi2(u), hi2(v), hi2(t), r.tol, any, tmax)) bits |= 2u << k;
+                return bits;
+            };
+            b0 |= one(r0, false);
+            if (TWO) b1 |= one(r1, true);
+        }
+        const uint32_t valid = cnt == 32u ? 0xffffffffu : (1u << cnt) - 1u;      // an odd triangle's partner
+        w0[w] = b0 & valid;
+        w1[w] = b1 & valid;
+    }
+    *c0 = make_uint2(w0[0], w0[1]);
+    *c1 = make_uint2(w1[0], w1[1]);
+}
+
+// Gradients of a warp's lanes (mat: the lane's material, or 64 for none), the
+// lanes of a material summed first: one addition per material and component
+// instead of one per lane on the same few addresses.
+__device__ __forceinline__ void warp_gadd(float *gacc, uint32_t mat, float4 g, uint32_t lane) {
+    unsigned left = __ballot_sync(0xffffffffu, mat <= kMaxMatIdx);
+    while (left) {
+        const uint32_t m = __shfl_sync(0xffffffffu, mat, __ffs(left) - 1);
+        const bool mine = mat == m;
+        left &= ~__ballot_sync(0xffffffffu, mine);
+        float4 x = mine ? g : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int h = 16; h >= 1; h >>= 1) {
+            x.x += __shfl_xor_sync(0xffffffffu, x.x, h);
+            x.y += __shfl_xor_sync(0xffffffffu, x.y, h);
+            x.z += __shfl_xor_sync(0xffffffffu, x.z, h);
+            x.w += __shfl_xor_sync(0xffffffffu, x.w, h);
+        }
+        if (lane == 0) block_gadd(gacc, m, x);
+    }
+}
+
+// The exact tests of the candidates, under the cull of their leaves' boxes as
+// in the tree walk.  ANY: whether one is accepted before tmax (best.t).
+template <bool ANY>
+__device__ __forceinline__ bool small_hit(const DeviceScene &S, const float4 *s_tri, const float4 *s_box,
+                                          const RayInv &r, uint2 cand, Closest &best) {
+    while (cand.x | cand.y) {
+        uint32_t j;
+        if (cand.x) {
+            j = (uint32_t)__ffs(cand.x) - 1u;
+            cand.x &= cand.x - 1u;
+        } else {
+            j = (uint32_t)__ffs(cand.y) + 31u;
+            cand.y &= cand.y - 1u;
+        }
+        const float4 a = s_tri[3u * j], b = s_tri[3u * j + 1u], c = s_tri[3u * j + 2u];
+        float t, u, v;
+        if (!tri_test(r, xyz(a), xyz(b), xyz(c), kTMin, &t, &u, &v)) continue;
+        const uint32_t id = __float_as_uint(a.w);
+        if (ANY ? !(t < best.t) : !tie_better_tri(t, id, best)) continue;
+        const float4 mn = s_box[2u * j], mx = s_box[2u * j + 1u];
+        float te;
+        if (!slab(r, mn.x, mn.y, mn.z, mx.x, mx.y, mx.z, kTMin, best.t, &te)) continue;
+        if (__float_as_uint(b.w) & MCRT_BACKFACE_CULL_FLAG) {       // path_trace.wgsl:438-452
+            f3 n = tri_shading_normal(S, id, u, v);
+            if (!(dot(r.d, n) < 0.0f)) continue;
+        }
+        if (ANY) return true;
+        best.t = t; best.prim = id; best.slot = id; best.u = u; best.v = v;
+    }
+    return false;
+}
+
+// One path per lane from its camera ray to its end; a lane whose path ends
+// takes the next slot of the warp's chunk.  A vertex's shadow ray and the ray
+// that continues its path start at the same point and are traced together.
+// The order of a path's radiance terms is the queue kernels' (emission or
+// environment at a vertex, then its next-event sample), so its radiance has
+// the same bits.  ADJ: the replay of the same paths, each starting from its
+// forward radiance in B.L (k_shade); the block's gradient sums go to the
+// double sums every kFlush steps of a warp, so that no float sum grows long.
+// counters[4] hands out chunks of slots, counters[6] collects cache queries.
+//
+// Bound by instruction fetch and issue: a step is some 5,000 instructions of
+// straight-line code.  One block per SM whose warps meet at a barrier each step
+// keeps them in the same part of it: Cornell box, 512x512, 64 spp, next-event
+// estimation: five blocks of 128 threads 16.8 ms, the same with the barrier
+// 16.4, one of 640 15.0, of 768 14.7, of 896 14.2 (72 registers), of 1024 14.3;
+// the queue kernels 20.0.  Passes of at most kSmallPass paths use 128
+// threads: 160x120, 1 spp: 0.11 ms a call against 0.16 (queue kernels 0.37).
+constexpr int kPathsBlock = 896, kPathsSmallBlock = 128;
+constexpr uint32_t kFlush = 16;
+template <bool ADJ>
+__global__ void __launch_bounds__(kPathsBlock, 1)
+    k_paths(DeviceScene S, RenderParams P, PathBuffers B, const SmallScene *T, uint32_t chunk, float4 *gbuf,
+            AdjointParams A) {
+    __shared__ float gacc[ADJ ? 256 : 1];
+    __shared__ float4 s_pair[4 * kSmallTris], s_tri[3 * kSmallTris], s_box[2 * kSmallTris];
+    const uint32_t nt = T->n;
+    const float emax = T->emax, vmax = T->vmax;
+    if (ADJ)
+        for (uint32_t k = threadIdx.x; k < 256u; k += blockDim.x) gacc[k] = 0.0f;
+    for (uint32_t k = threadIdx.x; k < 8u * ((nt + 1u) / 2u); k += blockDim.x) s_pair[k] = __ldg(T->pair + k);
+    for (uint32_t k = threadIdx.x; k < 3u * nt; k += blockDim.x)
+        s_tri[k] = __ldg(reinterpret_cast<const float4 *>(S.tris) + k);
+    if (threadIdx.x < S.n_mesh_nodes) {
+        const mcrt_gpu_bvh_node nd = S.mesh_nodes[threadIdx.x];
+        for (uint32_t k = 0; k < nd.prim_count; ++k) {
+            s_box[2u * (nd.right_or_offset + k)] = make_float4(nd.aabb_min[0], nd.aabb_min[1], nd.aabb_min[2], 0.0f);
+            s_box[2u * (nd.right_or_offset + k) + 1u] = make_float4(nd.aabb_max[0], nd.aabb_max[1], nd.aabb_max[2], 0.0f);
+        }
+    }
+    __syncthreads();
+    const uint32_t n = P.npix * P.spp_pass;
+    const bool nee = (P.flags & MCRT_RENDER_NEE) != 0 && (S.n_lights > 0 || S.has_sun);
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t next = 0, limit = 0;              // the warp's slots not yet started
+    bool exhausted = false;
+    bool go = false, shadow = false;           // the path has a ray to trace; its last vertex a shadow ray
+    f3 o = {0, 0, 0}, d = {0, 0, 0}, sd = {0, 0, 0}, sc = {0, 0, 0};
+    float smax = 0.0f;
+    uint32_t slot = 0, bounce = 0, rng = 0, pend_bits = 0, sh_bits = 0;
+    float4 thr4, L, pend, sh_dlog;
+    uint32_t rays = 0, shadow_rays = 0, nn = 0, steps = 0;
+    for (;;) {
+        // ---- idle lanes take the next slots
+        const unsigned idle = __ballot_sync(0xffffffffu, !go && !shadow);
+        if (idle && next == limit && !exhausted) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(B.counters + 4, chunk);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            next = min(base, n);
+            limit = min(base + chunk, n);
+            exhausted = limit == n;
+        }
+        if (idle && next < limit) {
+            const uint32_t mine = next + __popc(idle & below);
+            if (!go && !shadow && mine < limit) {
+                slot = mine;
+                start_path(P, slot, &o, &d, &rng);
+                thr4 = make_float4(1.0f, 1.0f, 1.0f, -1.0f);
+                L = ADJ ? B.L[slot] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                bounce = 0;
+                pend_bits = 0;
+                go = true;
+            }
+            next = min(limit, next + __popc(idle));
+        }
+        // the block's warps step together (see above); all done: the queue is empty
+        if (!__syncthreads_or(go || shadow || !(exhausted && next == limit))) break;
+        // ---- the path's ray (closest hit) and its last vertex's shadow ray (any hit)
+        float4 h = make_float4(-1.0f, 0.0f, 0.0f, 0.0f);
+        bool occl = false;
+        {
+            const uint64_t no[3] = {pk2(-o.x, -o.x), pk2(-o.y, -o.y), pk2(-o.z, -o.z)};
+            const PackedRay r0 = pack_ray(o, d, emax, vmax);
+            uint2 c0, c1;
+            if (__any_sync(0xffffffffu, shadow)) {
+                const PackedRay r1 = pack_ray(o, sd, emax, vmax);
+                small_candidates<true>(s_pair, nt, no, r0, r1, smax, &c0, &c1);
+                if (shadow) {
+                    const RayInv r = make_ray(o, sd);
+                    Closest best{smax, MCRT_HIT_MISS, 0u, 0.0f, 0.0f};
+                    spheres_hit(S, r, kTMin, smax, best, &nn);
+                    occl = best.prim != MCRT_HIT_MISS;
+                    best.t = smax;
+                    if (!occl) occl = small_hit<true>(S, s_tri, s_box, r, c1, best);
+                    ++shadow_rays;
+                }
+            } else {
+                small_candidates<false>(s_pair, nt, no, r0, r0, 0.0f, &c0, &c1);
+            }
+            if (go) {
+                const RayInv r = make_ray(o, d);
+                Closest best{kTMax, MCRT_HIT_MISS, 0u, 0.0f, 0.0f};
+                spheres_hit(S, r, kTMin, kTMax, best, &nn);          // path_trace.wgsl:472-474
+                small_hit<false>(S, s_tri, s_box, r, c0, best);
+                ++rays;
+                if (best.prim != MCRT_HIT_MISS)
+                    h = make_float4(best.t, __uint_as_float(best.prim),
+                                    (best.prim & MCRT_HIT_SPHERE) ? __uint_as_float(best.slot) : best.u, best.v);
+            }
+        }
+        // ---- next-event term
+        {
+            const bool lit = shadow && !occl;
+            if (!ADJ) {
+                if (lit) L = make_float4(L.x + sc.x, L.y + sc.y, L.z + sc.z, 0.0f);
+            } else if (__any_sync(0xffffffffu, lit)) {
+                uint32_t m0 = 64u, m1 = 64u;
+                float4 g0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), g1 = g0;
+                if (lit) {
+                    L = make_float4(L.x - sc.x, L.y - sc.y, L.z - sc.z, 0.0f);
+                    shadow_gradient(S, A, slot, sc, sh_bits, sh_dlog, [&](uint32_t mat, float4 g) {
+                        if (m0 == 64u) { m0 = mat; g0 = g; } else { m1 = mat; g1 = g; }
+                    });
+                }
+                warp_gadd(gacc, m0, g0, lane);
+                warp_gadd(gacc, m1, g1, lane);
+            }
+        }
+        // ---- shading
+        ShadedVertex v;
+        uint32_t m0 = 64u, m1 = 64u;           // ADJ: the pending term's and an emitter's gradients
+        float4 g0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), g1 = g0;
+        if (go) {
+            v.rng = rng;
+            const uint32_t pixel = slot / P.spp_pass;
+            f3 delta = {0.0f, 0.0f, 0.0f};
+            if (ADJ) {
+                delta = A.inv_spp * xyz(A.dimg[pixel]);
+                if (pend_bits) {
+                    m0 = (pend_bits >> 8) - 1u;
+                    g0 = pending_gradient(delta, L, pend);
+                }
+            }
+            shade_vertex<ADJ>(S, P, o, d, h, slot, pixel, bounce, nee, gbuf, delta, thr4, v, [&]() { return L; },
+                              [&](float4 x) { L = x; }, [&](uint32_t mat, float4 g) { m1 = mat; g1 = g; });
+            rng = v.rng;
+            if (ADJ) {
+                pend = v.pend;
+                pend_bits = v.pend_bits;
+                sh_bits = v.sh_bits;
+                sh_dlog = v.sh_dlog;
+            }
+        }
+        if (ADJ) {
+            warp_gadd(gacc, m0, g0, lane);
+            warp_gadd(gacc, m1, g1, lane);
+            if (++steps % kFlush == 0u)
+                for (uint32_t k = lane; k < 256u; k += 32u) {
+                    const float x = gacc[k] != 0.0f ? atomicExch(&gacc[k], 0.0f) : 0.0f;
+                    if (x != 0.0f) atomicAdd(A.grad + k, (double)x);
+                }
+        }
+        if (!ADJ && P.cache_query_vertex) {
+            const unsigned qmask = __ballot_sync(0xffffffffu, v.queried);
+            if (qmask) {
+                const int leader = __ffs(qmask) - 1;
+                uint32_t base = 0;
+                if ((int)lane == leader) base = atomicAdd(B.counters + 6, (uint32_t)__popc(qmask));
+                base = __shfl_sync(0xffffffffu, base, leader);
+                if (v.queried) {
+                    float4 *q = P.cache_queries + 4 * (size_t)(base + __popc(qmask & below));
+                    for (int k = 0; k < 4; ++k) q[k] = v.cq[k];
+                    B.thr[slot] = thr4;                               // read by the inference kernel
+                }
+            }
+        }
+        // ---- the next rays, or the path's end
+        const bool was = go || shadow;
+        go = v.cont;
+        shadow = v.shadow;
+        if (go) { o = v.no; d = v.nd; ++bounce; }
+        if (shadow) { o = v.so; sd = v.sd; sc = v.sc; smax = v.smax; }
+        if (!ADJ && was && !go && !shadow) __stcs(B.L + slot, L);
+    }
+    rays = __reduce_add_sync(0xffffffffu, rays);
+    shadow_rays = __reduce_add_sync(0xffffffffu, shadow_rays);
+    if (lane == 0) {
+        if (rays) atomicAdd(B.stats, (unsigned long long)rays);
+        if (shadow_rays) atomicAdd(B.stats + 1, (unsigned long long)shadow_rays);
+    }
+    if (ADJ) {
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < 256u; k += blockDim.x) {
+            const float x = gacc[k];
+            if (x != 0.0f) atomicAdd(A.grad + k, (double)x);
+        }
     }
 }
 
@@ -1629,7 +2099,7 @@ const ExtendKernel kCountKernels[kExtendVariants] = {
 int g_extend_per_sm[kExtendVariants] = {0, 0, 0, 0, 0, 0, 0, 0};
 int g_shadow_per_sm[kExtendVariants] = {0, 0, 0, 0, 0, 0, 0, 0};
 int g_shadow_adj_per_sm[kExtendVariants] = {0, 0, 0, 0, 0, 0, 0, 0};
-int g_packet_per_sm = 0;
+int g_packet_per_sm = 0, g_paths_per_sm = 0, g_paths_adj_per_sm = 0;
 int g_count_per_sm[kExtendVariants] = {0, 0, 0, 0, 0, 0, 0, 0};
 }  // namespace
 
@@ -1645,6 +2115,12 @@ void prepare_extend_variants() {
         int n = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_extend_packet<false>, kPacketBlock, 0);
         g_packet_per_sm = n > 0 ? n : 1;
+        n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_paths<false>, kPathsSmallBlock, 0);
+        g_paths_per_sm = n > 0 ? n : 1;
+        n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_paths<true>, kPathsSmallBlock, 0);
+        g_paths_adj_per_sm = n > 0 ? n : 1;
     }
     for (int v = 0; v < kExtendVariants; ++v) {
         if (g_extend_per_sm[v] == 0) {
@@ -1735,6 +2211,29 @@ void launch_shadow(const DeviceScene &S, const RenderParams &P, PathBuffers &B, 
     else kShadowKernels[v]<<<blocks, block, 0, st>>>(S, B, 0, AdjointParams{});
     ::mcrt::note_launch();
     launch_retry(S, B, 0, true, adj, st);
+}
+
+void launch_small_scene(const DeviceScene &S, SmallScene *out, cudaStream_t st) {
+    k_small_scene<<<1, 2 * kSmallTris, 0, st>>>(S, out); ::mcrt::note_launch();
+}
+
+cudaError_t launch_paths(const DeviceScene &S, const RenderParams &P, PathBuffers &B, const SmallScene *T,
+                         float4 *gbuf, cudaStream_t st, const AdjointParams *adj) {
+    prepare_extend_variants();
+    const uint32_t n = P.npix * P.spp_pass;
+    const bool large = n > kSmallPass;
+    const int block = large ? kPathsBlock : kPathsSmallBlock;
+    const int per_sm = large ? 1 : adj ? g_paths_adj_per_sm : g_paths_per_sm;
+    const int blocks = min(grid_blocks_for(n, block), sm_count() * per_sm);
+    // slots per fetch: about eight fetches per warp, at most 256 slots
+    const uint32_t warps = (uint32_t)blocks * (uint32_t)(block / 32);
+    const uint32_t chunk = max(32u, min(256u, n / (8u * warps) / 32u * 32u));
+    cudaError_t e = cudaMemsetAsync(B.counters, 0, 8 * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    if (adj) k_paths<true><<<blocks, block, 0, st>>>(S, P, B, T, chunk, gbuf, *adj);
+    else k_paths<false><<<blocks, block, 0, st>>>(S, P, B, T, chunk, gbuf, AdjointParams{});
+    ::mcrt::note_launch();
+    return cudaGetLastError();
 }
 
 void launch_resolve(const RenderParams &P, const PathBuffers &B, float4 *mean, double *sum, bool keep,
