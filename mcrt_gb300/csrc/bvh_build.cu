@@ -92,12 +92,13 @@ void exclusive_scan_u32(const uint32_t *d_in, uint32_t *d_out, uint32_t n, uint3
 
 // ------------------------------------------------------------------ float atomics
 namespace {
+// (decided by the sign bit: -0 is below +0 and must not be compared as the integer INT_MIN)
 __device__ __forceinline__ void atomic_min_f(float *a, float v) {
-    if (v >= 0.0f) atomicMin(reinterpret_cast<int *>(a), __float_as_int(v));
+    if (__float_as_int(v) >= 0) atomicMin(reinterpret_cast<int *>(a), __float_as_int(v));
     else atomicMax(reinterpret_cast<unsigned *>(a), __float_as_uint(v));
 }
 __device__ __forceinline__ void atomic_max_f(float *a, float v) {
-    if (v >= 0.0f) atomicMax(reinterpret_cast<int *>(a), __float_as_int(v));
+    if (__float_as_int(v) >= 0) atomicMax(reinterpret_cast<int *>(a), __float_as_int(v));
     else atomicMin(reinterpret_cast<unsigned *>(a), __float_as_uint(v));
 }
 

@@ -1,0 +1,48 @@
+"""The GPU builder's trees against the reference builder's (oracle), at shapes where it can go wrong."""
+import numpy as np
+import pytest
+
+import mcrt_gb300 as M
+from test_gpu_parity import bits, leaf_sets
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = M.Context(0)
+    yield c
+    c.close()
+
+
+def mesh(points):
+    n = len(points)
+    v = np.zeros(3 * n, M.VERTEX)
+    v["position"][:, :3] = points.reshape(-1, 3)
+    v["position"][:, 3] = 1
+    v["normal"][:, 1] = 1
+    t = np.zeros(n, M.TRIANGLE)
+    t["v"] = np.arange(3 * n).reshape(-1, 3)
+    return v, t
+
+
+def build_both(ctx, oracle, points):
+    v, t = mesh(points)
+    ctx.upload_scene(vertices=v, triangles=t, materials=M.materials([(0, (0.5, 0.5, 0.5), 0, 1)]))
+    nodes, order = ctx.mesh_bvh()
+    want, _, ids = oracle.build_mesh_bvh(v, t)
+    assert len(nodes) == len(want)
+    for f in ("right_or_offset", "prim_count"):
+        assert np.array_equal(nodes[f], want[f])
+    assert leaf_sets(nodes, order) == leaf_sets(want, ids)
+    return nodes, want
+
+
+@pytest.mark.parametrize("n", [7, 40, 300, 4000])
+def test_bvh_of_negative_zero_coordinates(ctx, oracle, n):
+    """-0 is one of the smallest values a box can have, not the largest integer."""
+    p = np.random.default_rng(n).integers(-2, 3, (n, 3, 3)).astype(np.float32)
+    p[p == 0] *= np.float32(-1)
+    nodes, want = build_both(ctx, oracle, p)
+    for f in ("aabb_min", "aabb_max"):       # by value: which zero a box keeps is the order of its primitives
+        assert np.array_equal(nodes[f], want[f])
