@@ -115,9 +115,6 @@ constexpr unsigned kOrdPosInf = 0xff800000u;     // f2ord(+inf): empty minimum
 constexpr unsigned kOrdNegInf = 0x007fffffu;     // f2ord(-inf): empty maximum
 constexpr unsigned kFull = 0xffffffffu;
 
-// Positions per block of the whole-array passes (4 per thread).
-constexpr uint32_t kPosPerBlock = 1024;
-
 constexpr int kBins = 8;
 constexpr uint32_t kLeafMax = 4;
 constexpr int kBinStride = 7;                    // count, min xyz, max xyz
@@ -158,16 +155,15 @@ struct BuildState {
     uint32_t *n_a, *n_b;              // internal: left bfs, right bfs; leaf: start, count
     uint32_t *n_leaf;                 // 1 = leaf
     uint32_t *n_size, *n_pre;         // subtree size, pre-order index
-    // Tasks of a level: large ones (above kSmallTask primitives) at indices
-    // 0, 1, ... of a task buffer, built by the whole-array passes; small ones
-    // at tcap - 1, tcap - 2, ... of the same buffer, one warp each; tiny ones
-    // (at most kTinyTask) in their own buffers, one thread each.
-    uint32_t tcap;                    // task buffer capacity (a level has at most nt / 5 tasks)
-    uint32_t *y_start[2], *y_count[2], *y_node[2];
-    float *y_bounds[2];               // tiny tasks (double-buffered), 6 bounds each
-    uint32_t *counters;               // [0] large tasks of the next level, [1] bfs node count,
-                                      // [4] small tasks of the next level, [5] of the current level,
-                                      // [6] tiny tasks of the next level, [7] of the current level
+    // Large tasks (above kSub primitives) are split level by level by the
+    // whole-array passes; the tasks their splits leave at kSub primitives and
+    // below go to this list and are built whole, one block each.
+    uint32_t *sub_start, *sub_count, *sub_node;
+    float4 *sub_rec;                  // their nodes: 3 float4 each (min, max, link | count | pre-order index), the
+                                      // nodes of a subtree from index 2 * its first position
+    uint32_t *counters;               // [0] large tasks of the next level, [1] bfs node count, [4] subtrees,
+                                      // [8] large tasks of the current level, [9] error word (a look-back wait
+                                      // gave up), [10] levels of the deepest subtree
     uint32_t *level_end;              // bfs node count at the start of each level
     // spatial order: primitives are built in the order of their centroids'
     // Morton codes (radix-sorted), so a warp's positions are neighbours
@@ -175,15 +171,23 @@ struct BuildState {
     uint32_t *rhist, *roffs;          // digit counts per tile and their exclusive scan
     float4 *qmin, *qmax, *qcen;       // second set of primitive bounds: the reordering target
     // single-pass partition scan of a level (k_flag_scan): [0] tile ticket,
-    // [1] error word (a look-back wait gave up), [2 + t] status of tile t:
+    // [2 + t] status of tile t:
     // flag << 32 | value (flag 1: the tile's own sum, 2: inclusive prefix)
     unsigned long long *part;
 };
-constexpr uint32_t kFlagThreads = 256, kFlagItems = 8;   // k_flag_scan: positions per thread, per block
-constexpr uint32_t kFlagTile = kFlagThreads * kFlagItems;
+constexpr uint32_t kFlagThreads = 256;                     // k_flag_scan: threads per tile
+constexpr uint32_t kMinFlagTile = kFlagThreads * 2;
 constexpr uint32_t kLookbackPolls = 1u << 20;              // polls of one predecessor before giving up
-constexpr uint32_t kSmallTask = 256;       // tasks up to this size are built by one warp each
-constexpr uint32_t kTinyTask = 8;          // and up to this size by one thread each
+// Subtrees up to this size are built by one block in shared memory: the
+// primitives' 36 bytes, their order and the nodes take 70 KB at 1024, so three
+// blocks share an SM.
+constexpr uint32_t kSub = 1024;
+constexpr uint32_t kSubThreads = 256, kSubWarps = kSubThreads / 32;
+constexpr uint32_t kSubCoop = 256;         // within a subtree: larger tasks by the whole block, others by a warp
+constexpr uint32_t kSubTasks = kSub / 5 + 4;   // a level's tasks hold more than 4 primitives each
+// Below this many primitives the whole-array passes take 256 positions per block
+// instead of 1024, so that there are more blocks than SMs.
+constexpr uint32_t kWideBlocks = 1u << 19;
 constexpr uint32_t kMaxLevels = 4096;
 }  // namespace
 
@@ -250,16 +254,25 @@ __global__ void k_root_init(BuildState S) {
             S.t_bounds[0][3 + a] = __int_as_float(0xff800000);
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x < 16) S.counters[threadIdx.x] = threadIdx.x == 1 ? 1u : 0u;
+    if (blockIdx.x == 0 && threadIdx.x < 16) S.counters[threadIdx.x] = threadIdx.x <= 1 ? 1u : 0u;   // the root
 }
 
-// Root bounds: per-thread min / max over 4 primitives, warp and block
+// A build of at most kSub primitives: the root is the one subtree.
+__global__ void k_root_subtree(BuildState S) {
+    S.sub_start[0] = 0;
+    S.sub_count[0] = S.nt;
+    S.sub_node[0] = 0;
+    S.n_leaf[0] = 2u;
+    S.level_end[0] = 1;
+}
+
+// Root bounds: per-thread min / max over the block's primitives, warp and block
 // reductions on the ordered integers, six global atomics per block.
-__global__ void __launch_bounds__(256) k_root_bounds(BuildState S) {
+__global__ void __launch_bounds__(256) k_root_bounds(BuildState S, uint32_t per) {
     __shared__ unsigned sh[6];
     if (threadIdx.x < 6) sh[threadIdx.x] = threadIdx.x < 3 ? kOrdPosInf : kOrdNegInf;
     __syncthreads();
-    const uint32_t first = blockIdx.x * kPosPerBlock, end = min(first + kPosPerBlock, S.nt);
+    const uint32_t first = blockIdx.x * per, end = min(first + per, S.nt);
     unsigned o[6] = {kFull, kFull, kFull, 0u, 0u, 0u};
     for (uint32_t i = first + threadIdx.x; i < end; i += 256) {
         const float4 a = S.pmin[i], b = S.pmax[i];
@@ -389,21 +402,18 @@ __global__ void k_final_order(const uint32_t *perm, const uint32_t *sorted_ids, 
     if (i < n) out[i] = sorted_ids[perm[i]];
 }
 
-// The start of a level: the current level's small and tiny task counts (those
-// of the level before), the node count at its start, and fresh child-task
-// counters.  One thread.
+// The start of a level: its number of large tasks, a fresh count of their
+// large children, and the node count.  One thread.
 __device__ __forceinline__ void level_advance(BuildState &S, uint32_t level) {
+    S.counters[8] = S.counters[0];
     S.counters[0] = 0;
-    S.counters[5] = S.counters[4];
-    S.counters[4] = 0;
-    S.counters[7] = S.counters[6];
-    S.counters[6] = 0;
     S.level_end[level] = S.counters[1];
 }
 
 // The start of a level with large tasks, in one launch: level_advance, the
 // status words of the level's partition scan zeroed (n_part), and the large
 // tasks' centroid bounds and bins set to empty.
+// ntasks: at least the number of large tasks.
 __global__ void k_task_reset(BuildState S, uint32_t level, uint32_t ntasks, uint32_t n_part) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) level_advance(S, level);
@@ -430,11 +440,11 @@ __device__ __forceinline__ int block_single_task(const BuildState &S, int cur, u
 // Centroid bounds per task.  Lanes reduce first (one pass per distinct task in
 // the warp, redux.sync on the ordered integers); a block inside one task
 // combines its warps in shared memory and issues six global atomics.
-__global__ void __launch_bounds__(256) k_centroid_bounds(BuildState S, int cur) {
+__global__ void __launch_bounds__(256) k_centroid_bounds(BuildState S, int cur, uint32_t per) {
     __shared__ unsigned sh[6];
     __shared__ int block_task;
-    const uint32_t first = blockIdx.x * kPosPerBlock;
-    const uint32_t end = min(first + kPosPerBlock, S.nt);
+    const uint32_t first = blockIdx.x * per;
+    const uint32_t end = min(first + per, S.nt);
     const uint32_t lane = threadIdx.x & 31u;
     if (threadIdx.x == 0) block_task = block_single_task(S, cur, first, end);
     if (threadIdx.x < 6) sh[threadIdx.x] = threadIdx.x < 3 ? kOrdPosInf : kOrdNegInf;
@@ -570,11 +580,11 @@ __device__ __forceinline__ void bins_warp(BuildState &S, unsigned *sh, int task,
 // Bin accumulation (count and primitive-bounds union per bin and axis).  Warps
 // reduce lanes of equal (task, bin) first; a block inside one task collects
 // its warps in shared memory and adds the block's bins to the global ones.
-__global__ void __launch_bounds__(256) k_bins(BuildState S, int cur) {
+__global__ void __launch_bounds__(256) k_bins(BuildState S, int cur, uint32_t per) {
     __shared__ unsigned sh[kTaskBinWords];
     __shared__ int block_task;
-    const uint32_t first = blockIdx.x * kPosPerBlock;
-    const uint32_t end = min(first + kPosPerBlock, S.nt);
+    const uint32_t first = blockIdx.x * per;
+    const uint32_t end = min(first + per, S.nt);
     const uint32_t lane = threadIdx.x & 31u;
     if (threadIdx.x == 0) block_task = block_single_task(S, cur, first, end);
     for (int k = threadIdx.x; k < kTaskBinWords; k += blockDim.x) {
@@ -615,159 +625,119 @@ __global__ void __launch_bounds__(256) k_bins(BuildState S, int cur) {
     }
 }
 
-// SAH split choice of one task (bvh.rs:388-463) from its node bounds tb,
-// centroid bounds cb and bins.  Returns the split (axis * 16 + bin), or -1 when
-// the task stays a leaf; *lcount = primitives going left, *bl / *br = the
-// children's bounds.
-// Best split so far of the serial SAH sweep.
-struct SplitBest {
-    float cost;                    // starts at the leaf cost n
-    int axis = 0, bin = 0;
-    uint32_t l = 0;
-    bool found = false;
-    Aabb lb, rb;
-};
-__device__ __forceinline__ SplitBest split_best_init(uint32_t n) {
-    SplitBest b;
-    b.cost = (float)n;
-    b.lb = aabb_empty();
-    b.rb = aabb_empty();
-    return b;
-}
-
-// One axis of the SAH sweep (bvh.rs:388-463): prefix unions of bins 0..s,
-// suffix unions of bins 7..s+1, cost (A_l * n_l + A_r * n_r) / A_parent,
-// replaced only on a strictly smaller cost.  get(k, f) = field f of bin k
-// (0: count as bits, 1-3: min, 4-6: max).
-template <class Get>
-__device__ __forceinline__ void split_axis(int axis, float parent, Get get, SplitBest &best) {
-    Aabb bb[kBins];
-    uint32_t bc[kBins];
-    for (int k = 0; k < kBins; ++k) {
-        bc[k] = __float_as_uint(get(k, 0));
-        for (int a = 0; a < 3; ++a) { bb[k].mn[a] = get(k, 1 + a); bb[k].mx[a] = get(k, 4 + a); }
-    }
-    Aabb lb[kBins];
-    uint32_t lc[kBins];
-    lb[0] = bb[0]; lc[0] = bc[0];
-    for (int k = 1; k < kBins; ++k) { lb[k] = aabb_union(lb[k - 1], bb[k]); lc[k] = lc[k - 1] + bc[k]; }
-    Aabb rb = aabb_empty();
-    uint32_t rc = 0;
-    for (int s = kBins - 2; s >= 0; --s) {
-        rb = aabb_union(rb, bb[s + 1]);
-        rc += bc[s + 1];
-        const uint32_t l = lc[s];
-        if (l == 0 || rc == 0) continue;
-        const float cost = (half_area(lb[s]) * (float)l + half_area(rb) * (float)rc) / parent;
-        if (cost < best.cost) {
-            best.cost = cost; best.axis = axis; best.bin = s; best.l = l; best.found = true;
-            best.lb = lb[s]; best.rb = rb;
-        }
-    }
-}
-
-// The split of a finished sweep: axis * 16 + bin, or -1 for a leaf.
-__device__ __forceinline__ int split_result(const SplitBest &best, uint32_t n, uint32_t *lcount, Aabb *bl, Aabb *br) {
-    if (!(best.found && best.l > 0 && best.l < n)) return -1;
-    *lcount = best.l;
-    *bl = best.lb;
-    *br = best.rb;
-    return best.axis * 16 + best.bin;
-}
-
+// ---- SAH split choice (bvh.rs:388-463): per axis, prefix unions of bins 0..s and
+// suffix unions of bins 7..s+1, cost (A_l * n_l + A_r * n_r) / A_parent, taken in
+// the serial order (axes ascending, s descending) and replaced only on a strictly
+// smaller cost, starting from the leaf's cost n.  Evaluated by a warp, or by two or
+// four groups of its lanes for small tasks: a lane holds one bin of one axis.
 __device__ __forceinline__ float node_half_area(const float *tb) {
     Aabb nb;
     for (int a = 0; a < 3; ++a) { nb.mn[a] = tb[a]; nb.mx[a] = tb[3 + a]; }
     return fmaxf(half_area(nb), 1e-8f);
 }
 
-__device__ int choose_split(uint32_t n, const float *tb, const float *cb, const float *bins, uint32_t *lcount,
-                            Aabb *bl, Aabb *br) {
-    const float parent = node_half_area(tb);
-    SplitBest best = split_best_init(n);
-    for (int axis = 0; axis < 3; ++axis) {
-        const float len = cb[3 + axis] - cb[axis];
-        if (len < 1e-8f) continue;
-        const float *q = bins + axis * kBins * kBinStride;
-        split_axis(axis, parent, [&](int k, int f) { return q[k * kBinStride + f]; }, best);
-    }
-    return split_result(best, n, lcount, bl, br);
-}
+// One lane's bin of one axis: its primitives' number and box.
+struct LaneBin { uint32_t n; Aabb b; };
 
-// choose_split evaluated by a warp.  Lane j < 21 takes the serial loop's j-th
-// candidate (axis j / 7, split 6 - j % 7) and forms its left union over bins
-// 0..s ascending and its right union over bins 7..s+1 descending — the serial
-// loop's operation order, so every cost has the same bits — and the cheapest
-// candidate below the leaf cost wins, ties to the earliest (the serial loop
-// replaces only on a strictly smaller cost).  Every lane gets the result.
-__device__ int choose_split_warp(uint32_t n, const float *tb, const float *cb, const float *bins, uint32_t lane,
-                                 uint32_t *lcount, Aabb *bl, Aabb *br) {
-    Aabb nb;
-    for (int a = 0; a < 3; ++a) { nb.mn[a] = tb[a]; nb.mx[a] = tb[3 + a]; }
-    const float parent = fmaxf(half_area(nb), 1e-8f);
-    const int axis = (int)lane / 7, s = 6 - (int)lane % 7;
-    bool ok = lane < 21u;
-    float cost = 0.0f;
-    uint32_t l = 0, rc = 0;
-    Aabb lb = aabb_empty(), rb = aabb_empty();
-    if (ok) {
-        const float len = cb[3 + axis] - cb[axis];
-        if (len < 1e-8f) {
-            ok = false;
-        } else {
-            const float *q = bins + axis * kBins * kBinStride;
-            auto box = [&](int k) {
-                Aabb b;
-                for (int a = 0; a < 3; ++a) { b.mn[a] = q[k * kBinStride + 1 + a]; b.mx[a] = q[k * kBinStride + 4 + a]; }
-                return b;
-            };
-            lb = box(0);
-            l = __float_as_uint(q[0]);
-            for (int k = 1; k <= s; ++k) { lb = aabb_union(lb, box(k)); l += __float_as_uint(q[k * kBinStride]); }
-            for (int k = kBins - 1; k > s; --k) { rb = aabb_union(rb, box(k)); rc += __float_as_uint(q[k * kBinStride]); }
-            if (l == 0 || rc == 0) ok = false;
-            else cost = (half_area(lb) * (float)l + half_area(rb) * (float)rc) / parent;
-            ok = ok && cost < (float)n;
+// Adds to a lane's bin (axis, bin) those of cnt staged primitives (two float4
+// each: box, then the bins of the three axes in 4 bits each) that fall into it.
+__device__ __forceinline__ void bin_add(LaneBin &acc, const float4 *stage, uint32_t cnt, uint32_t axis, uint32_t bin) {
+    const float inf = __int_as_float(0x7f800000);
+#pragma unroll 4
+    for (uint32_t i = 0; i < cnt; ++i) {
+        const float4 q0 = stage[2 * i], q1 = stage[2 * i + 1];
+        const bool in = ((__float_as_uint(q1.z) >> (4u * axis)) & 15u) == bin;
+        const float qn[3] = {q0.x, q0.y, q0.z}, qx[3] = {q0.w, q1.x, q1.y};
+        acc.n += in ? 1u : 0u;
+        for (int a = 0; a < 3; ++a) {
+            acc.b.mn[a] = fminf(acc.b.mn[a], in ? qn[a] : inf);
+            acc.b.mx[a] = fmaxf(acc.b.mx[a], in ? qx[a] : -inf);
         }
     }
-    const unsigned oc = ok ? f2ord(cost) : kFull;
-    const unsigned best = __reduce_min_sync(kFull, oc);
-    if (best == kFull) return -1;
-    const int win = (int)__reduce_min_sync(kFull, (ok && oc == best) ? lane : kFull);
-    *lcount = __shfl_sync(kFull, l, win);
-    for (int a = 0; a < 3; ++a) {
-        bl->mn[a] = __shfl_sync(kFull, lb.mn[a], win); bl->mx[a] = __shfl_sync(kFull, lb.mx[a], win);
-        br->mn[a] = __shfl_sync(kFull, rb.mn[a], win); br->mx[a] = __shfl_sync(kFull, rb.mx[a], win);
+}
+
+// A candidate split of the serial order: k = axis * 7 + 6 - bin.
+struct LaneSplit {
+    unsigned cost = kFull;                 // ordered cost, kFull: none
+    uint32_t k = 32u, l = 0;
+    Aabb lb = aabb_empty(), rb = aabb_empty();
+};
+// The lane's candidate (left: bins up to its own of its axis), from the bins of
+// the eight lanes of the axis by a prefix and a suffix scan; kept in best when it
+// is cheaper than the leaf and than best.  Same costs, bit for bit, as the serial
+// sweep: the unions are the same sets, and min and max do not depend on order.
+__device__ __forceinline__ void bin_candidate(const LaneBin &mine, uint32_t axis, uint32_t bin, bool flat, uint32_t n,
+                                              float parent, LaneSplit &best) {
+    LaneBin p = mine, q = mine;
+#pragma unroll
+    for (uint32_t h = 1; h < 8; h <<= 1) {
+        LaneBin a, b;
+        a.n = __shfl_up_sync(kFull, p.n, h, 8);
+        b.n = __shfl_down_sync(kFull, q.n, h, 8);
+        for (int c = 0; c < 3; ++c) {
+            a.b.mn[c] = __shfl_up_sync(kFull, p.b.mn[c], h, 8); a.b.mx[c] = __shfl_up_sync(kFull, p.b.mx[c], h, 8);
+            b.b.mn[c] = __shfl_down_sync(kFull, q.b.mn[c], h, 8); b.b.mx[c] = __shfl_down_sync(kFull, q.b.mx[c], h, 8);
+        }
+        if (bin >= h) { p.n += a.n; p.b = aabb_union(p.b, a.b); }
+        if (bin + h < 8u) { q.n += b.n; q.b = aabb_union(q.b, b.b); }
     }
-    return (win / 7) * 16 + (6 - win % 7);
+    Aabb rb;
+    const uint32_t rc = __shfl_down_sync(kFull, q.n, 1, 8);
+    for (int c = 0; c < 3; ++c) {
+        rb.mn[c] = __shfl_down_sync(kFull, q.b.mn[c], 1, 8);
+        rb.mx[c] = __shfl_down_sync(kFull, q.b.mx[c], 1, 8);
+    }
+    const float cost = (half_area(p.b) * (float)p.n + half_area(rb) * (float)rc) / parent;
+    const bool ok = axis < 3u && bin < 7u && !flat && p.n != 0u && rc != 0u && cost < (float)n;
+    const unsigned oc = ok ? f2ord(cost) : kFull;
+    if (oc < best.cost || (oc == best.cost && oc != kFull && axis * 7u + 6u - bin < best.k)) {
+        best.cost = oc;
+        best.k = axis * 7u + 6u - bin;
+        best.l = p.n;
+        best.lb = p.b;
+        best.rb = rb;
+    }
 }
 
-// Child tasks a split creates, by class: large (above kSmallTask primitives),
-// small (above kTinyTask) and tiny (above the leaf size).
+// The cheapest candidate of a group of G lanes, ties to the earliest; every
+// lane of the group gets it.  Returns whether there is one.
+template <uint32_t G>
+__device__ __forceinline__ bool best_split(LaneSplit &v, uint32_t lane) {
+    unsigned cost = v.cost;
+#pragma unroll
+    for (uint32_t h = G / 2; h; h >>= 1) cost = min(cost, __shfl_xor_sync(kFull, cost, h));
+    uint32_t key = v.cost == cost ? (v.k << 8) | lane : kFull;
+#pragma unroll
+    for (uint32_t h = G / 2; h; h >>= 1) key = min(key, __shfl_xor_sync(kFull, key, h));
+    const int from = (int)(key & 31u);
+    v.cost = cost;
+    v.k = key >> 8;
+    v.l = __shfl_sync(kFull, v.l, from);
+    for (int a = 0; a < 3; ++a) {
+        v.lb.mn[a] = __shfl_sync(kFull, v.lb.mn[a], from); v.lb.mx[a] = __shfl_sync(kFull, v.lb.mx[a], from);
+        v.rb.mn[a] = __shfl_sync(kFull, v.rb.mn[a], from); v.rb.mx[a] = __shfl_sync(kFull, v.rb.mx[a], from);
+    }
+    return cost != kFull;
+}
+
+// Child tasks of a split: large (above kSub primitives) and subtrees (above the
+// leaf size).
 __device__ __forceinline__ uint32_t child_large(uint32_t n, uint32_t lcount) {
-    return (lcount > kSmallTask ? 1u : 0u) + (n - lcount > kSmallTask ? 1u : 0u);
+    return (lcount > kSub ? 1u : 0u) + (n - lcount > kSub ? 1u : 0u);
 }
-__device__ __forceinline__ uint32_t child_small(uint32_t n, uint32_t lcount) {
-    auto small = [](uint32_t c) { return c > kTinyTask && c <= kSmallTask; };
-    return (small(lcount) ? 1u : 0u) + (small(n - lcount) ? 1u : 0u);
+__device__ __forceinline__ uint32_t child_sub(uint32_t n, uint32_t lcount) {
+    auto sub = [](uint32_t c) { return c > kLeafMax && c <= kSub; };
+    return (sub(lcount) ? 1u : 0u) + (sub(n - lcount) ? 1u : 0u);
 }
-__device__ __forceinline__ uint32_t child_tiny(uint32_t n, uint32_t lcount) {
-    auto tiny = [](uint32_t c) { return c > kLeafMax && c <= kTinyTask; };
-    return (tiny(lcount) ? 1u : 0u) + (tiny(n - lcount) ? 1u : 0u);
-}
-constexpr uint32_t kSmallFlag = 0x80000000u;     // task map: the child is a small or tiny task
+constexpr uint32_t kSubMark = 2u;                // n_leaf of a subtree's root
 
-// Node records of a task.  A leaf (sp < 0) keeps its range.  A split gets the
-// BFS ids child0, child0 + 1 for its children; its large children get the task
-// ids large0, large0 + 1, its small children small0, small0 + 1 (a small task
-// k is stored at index tcap - 1 - k) and its tiny children tiny0, tiny0 + 1
-// (in child order) in buffer nxt.  child_task[c] = -1 for a leaf child.  Ids
-// come from the caller, which reserves them for a whole warp with one atomic
-// each (same-address atomics per task serialise at the L2).
+// Node records of a large task.  A leaf (sp < 0) keeps its range.  A split gets
+// the BFS ids child0, child0 + 1 for its children; its large children get the
+// task ids large0, large0 + 1 and its subtrees the list entries sub0, sub0 + 1
+// (in child order).
 __device__ void record_task(BuildState &S, int nxt, uint32_t start, uint32_t n, uint32_t node, int sp,
                             uint32_t lcount, const Aabb &bl, const Aabb &br, uint32_t child0, uint32_t large0,
-                            uint32_t small0, uint32_t tiny0, int child_task[2]) {
-    child_task[0] = child_task[1] = -1;
+                            uint32_t sub0) {
     if (sp < 0) {
         S.n_leaf[node] = 1; S.n_a[node] = start; S.n_b[node] = n;
         return;
@@ -784,22 +754,16 @@ __device__ void record_task(BuildState &S, int nxt, uint32_t start, uint32_t n, 
             S.n_leaf[id] = 1; S.n_a[id] = starts[c]; S.n_b[id] = counts[c];
             continue;
         }
-        S.n_leaf[id] = 0;
-        if (counts[c] <= kTinyTask) {
-            const uint32_t task = tiny0++;
-            S.y_start[nxt][task] = starts[c];
-            S.y_count[nxt][task] = counts[c];
-            S.y_node[nxt][task] = id;
-            for (int a = 0; a < 3; ++a) {
-                S.y_bounds[nxt][6 * task + a] = cbx[c]->mn[a];
-                S.y_bounds[nxt][6 * task + 3 + a] = cbx[c]->mx[a];
-            }
-            S.n_size[id] = kSmallFlag;
-            child_task[c] = (int)task;
+        if (counts[c] <= kSub) {
+            const uint32_t k = sub0++;
+            S.sub_start[k] = starts[c];
+            S.sub_count[k] = counts[c];
+            S.sub_node[k] = id;
+            S.n_leaf[id] = kSubMark;
             continue;
         }
-        const bool small = counts[c] <= kSmallTask;
-        const uint32_t task = small ? S.tcap - 1u - small0++ : large0++;
+        S.n_leaf[id] = 0;
+        const uint32_t task = large0++;
         S.t_start[nxt][task] = starts[c];
         S.t_count[nxt][task] = counts[c];
         S.t_node[nxt][task] = id;
@@ -807,315 +771,504 @@ __device__ void record_task(BuildState &S, int nxt, uint32_t start, uint32_t n, 
             S.t_bounds[nxt][6 * task + a] = cbx[c]->mn[a];
             S.t_bounds[nxt][6 * task + 3 + a] = cbx[c]->mx[a];
         }
-        // the child's positions learn their new task id in k_scatter through this map
-        S.n_size[id] = small ? kSmallFlag : task;      // temporary: child node -> task id
-        child_task[c] = (int)task;
+        S.n_size[id] = task;               // temporary: child node -> task id, for k_scatter
     }
     S.n_a[node] = child0;
     S.n_b[node] = child0 + 1;
 }
 
-// One thread per task: split choice, then ids for the children reserved per
-// warp (prefix sums by shuffles, one atomic per counter).
-__global__ void k_split(BuildState S, int cur, uint32_t ntasks) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per large task: split choice from its 24 bins, then the node records
+// and the children's ids by lane 0.  (A thread per task ran the sweep in 10 us a
+// level, for one task as for a thousand, and the 80,000-triangle build 0.80 ms
+// instead of 0.74.)
+__global__ void __launch_bounds__(128) k_split(BuildState S, int cur) {
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31u;
-    if ((t & ~31u) >= ntasks) return;                     // whole warps
-    const bool active = t < ntasks;
-    uint32_t start = 0, n = 0, node = 0, lcount = 0;
-    int sp = -1;
-    Aabb bl = aabb_empty(), br = aabb_empty();
-    if (active) {
-        start = S.t_start[cur][t]; n = S.t_count[cur][t]; node = S.t_node[cur][t];
-        sp = choose_split(n, S.t_bounds[cur] + 6 * t, S.t_cb + 6 * t, S.t_bins + (size_t)t * kTaskBinWords, &lcount,
-                          &bl, &br);
+    if (t >= S.counters[8]) return;                       // whole warps
+    const uint32_t start = S.t_start[cur][t], n = S.t_count[cur][t], node = S.t_node[cur][t];
+    const uint32_t axis = lane >> 3, bin = lane & 7u;
+    LaneBin mine{0u, aabb_empty()};
+    bool flat = true;
+    if (axis < 3u) {
+        const float *q = S.t_bins + (size_t)t * kTaskBinWords + lane * kBinStride;
+        mine.n = __float_as_uint(q[0]);
+        for (int a = 0; a < 3; ++a) { mine.b.mn[a] = q[1 + a]; mine.b.mx[a] = q[4 + a]; }
+        flat = S.t_cb[6 * t + 3 + axis] - S.t_cb[6 * t + axis] < 1e-8f;
     }
-    const uint32_t my_nodes = sp >= 0 ? 2u : 0u;
-    const uint32_t my_large = sp >= 0 ? child_large(n, lcount) : 0u;
-    const uint32_t my_small = sp >= 0 ? child_small(n, lcount) : 0u;
-    const uint32_t my_tiny = sp >= 0 ? child_tiny(n, lcount) : 0u;
-    uint32_t pn = my_nodes, pl = my_large, ps = my_small, py = my_tiny;   // inclusive prefix sums over the warp
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t a = __shfl_up_sync(kFull, pn, off), b = __shfl_up_sync(kFull, pl, off);
-        const uint32_t c = __shfl_up_sync(kFull, ps, off), d = __shfl_up_sync(kFull, py, off);
-        if ((int)lane >= off) { pn += a; pl += b; ps += c; py += d; }
-    }
-    const uint32_t tn = __shfl_sync(kFull, pn, 31), tl = __shfl_sync(kFull, pl, 31);
-    const uint32_t ts = __shfl_sync(kFull, ps, 31), ty = __shfl_sync(kFull, py, 31);
-    uint32_t bn = 0, bl0 = 0, bs = 0, by = 0;
-    if (lane == 0) {
-        if (tn) bn = atomicAdd(S.counters + 1, tn);
-        if (tl) bl0 = atomicAdd(S.counters, tl);
-        if (ts) bs = atomicAdd(S.counters + 4, ts);
-        if (ty) by = atomicAdd(S.counters + 6, ty);
-    }
-    bn = __shfl_sync(kFull, bn, 0);
-    bl0 = __shfl_sync(kFull, bl0, 0);
-    bs = __shfl_sync(kFull, bs, 0);
-    by = __shfl_sync(kFull, by, 0);
-    if (!active) return;
-    int ct[2];
-    record_task(S, cur ^ 1, start, n, node, sp, lcount, bl, br, bn + pn - my_nodes, bl0 + pl - my_large,
-                bs + ps - my_small, by + py - my_tiny, ct);
+    LaneSplit best;
+    bin_candidate(mine, axis, bin, flat, n, node_half_area(S.t_bounds[cur] + 6 * t), best);
+    const bool split = best_split<32>(best, lane);
+    if (lane != 0) return;
+    const int sp = split ? (int)(best.k / 7u) * 16 + (int)(6u - best.k % 7u) : -1;
+    const uint32_t large = split ? child_large(n, best.l) : 0u, sub = split ? child_sub(n, best.l) : 0u;
+    const uint32_t child0 = split ? atomicAdd(S.counters + 1, 2u) : 0u;
+    const uint32_t large0 = large ? atomicAdd(S.counters, large) : 0u;
+    const uint32_t sub0 = sub ? atomicAdd(S.counters + 4, sub) : 0u;
+    record_task(S, cur ^ 1, start, n, node, sp, best.l, best.lb, best.rb, child0, large0, sub0);
     S.t_split[t] = sp;
-    if (sp >= 0) S.t_lcount[t] = lcount;
+    if (split) S.t_lcount[t] = best.l;
 }
 
-// Levels whose tasks are all small: one warp per task does what the per-level
-// kernels above do for the whole array — centroid bounds (warp reduction),
-// bins (shared-memory atomics private to the warp), the split of lane 0, and a
-// stable partition by ballot — so a level is one launch.  Positions that land
-// in a leaf are written to both permutation buffers (they never move again).
-__global__ void __launch_bounds__(256) k_small_level(BuildState S, int cur) {
-    __shared__ float wbins[8][kTaskBinWords];
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (k >= S.counters[5]) return;                            // whole warps leave together
-    const uint32_t t = S.tcap - 1u - k;                        // small tasks from the top of the buffer
-    const uint32_t start = S.t_start[cur][t], n = S.t_count[cur][t], node = S.t_node[cur][t];
-    const uint32_t *perm_in = S.perm[cur];
-    // A task of at most 32 primitives keeps one per lane in registers for all
-    // passes (one load each); a larger one streams chunks of 32 per pass.
-    const bool one = n <= 32u;                                 // warp-uniform
-    const bool in0 = one && lane < n;
-    uint32_t id0 = 0;
-    float4 c0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), mn0 = c0, mx0 = c0;
-    if (in0) {
-        id0 = perm_in[start + lane];
-        c0 = S.pcen[id0]; mn0 = S.pmin[id0]; mx0 = S.pmax[id0];
+// ------------------------------------------------------------------ subtrees
+// A task of at most kSub primitives is built whole by one block: the same
+// level-synchronous algorithm (centroid bounds, 8 bins per axis, the cheapest
+// split, a stable partition) on primitives, order and nodes in shared memory.
+// Within a level, a task above kSubCoop primitives is split by the whole block,
+// one of 33 to kSubCoop by a warp, and two or four of at most 16 or 8 by a warp.
+// A lane first holds a primitive and computes its bins, then it holds a bin of
+// one axis and runs over the staged primitives, taking those of its bin: 18
+// instructions per primitive and warp.  (Groups of lanes of equal bin by
+// match.any and redux.sync on their masks, as the whole-array passes have them,
+// took 12,000 cycles per 32 primitives here: each mask is its own instruction.)
+//
+// The smaller levels hold most of a tree's nodes.  As launches over all tasks
+// of a level (a warp per task, a thread per task of at most 8) they took 1.64 of
+// the 4.2 ms of the 1.3M-triangle build and 0.61 of the 1.9 ms of an 80,000
+// triangle build, in 25 launches, and another 46 launches found the subtree sizes
+// and pre-order indices.  Now k_subtrees takes 0.70 and 0.14 ms and the builds
+// 2.54 and 0.74 ms, in 118 launches (206 before) and 94 (173).  It is bound by
+// the instructions of bin_add and by a block's idle warps on a subtree's first
+// and last levels; blocks of 512 threads, two to an SM, take the same time.
+struct SubShared {
+    float c[3][kSub], mn[3][kSub], mx[3][kSub];       // centroids and boxes by local index
+    uint16_t perm[2][kSub];                           // position -> local index
+    unsigned scratch[kSubWarps][256];                 // per warp: 32 staged primitives of 8 words, or bins
+    uint16_t t_start[2][kSubTasks], t_count[2][kSubTasks], t_node[2][kSubTasks];
+    float t_area[2][kSubTasks];                       // the tasks' half areas, clamped as the cost wants them
+    uint16_t a[2 * kSub], b[2 * kSub];                // node: left child (b = 0), or first position and count
+    uint16_t size[2 * kSub], pre[2 * kSub];
+    uint16_t level_end[kSub + 2];
+    unsigned red[6];
+    uint32_t warp_left[kSubWarps];
+    uint32_t n_nodes, n_tasks[2], lcount;
+    uint32_t n_class[2][3];                           // tasks of at most 8, at most 16, and more primitives
+    uint8_t of_class[2][3][kSubTasks];
+    int split, leaf_child[2];
+};
+static_assert(kSubTasks < 256, "task indices are bytes");
+static_assert(kTaskBinWords <= 256, "a warp's bins fit its scratch");
+
+__device__ __forceinline__ void sub_box(const BuildState &S, size_t rec, const Aabb &b) {
+    S.sub_rec[3 * rec] = make_float4(b.mn[0], b.mn[1], b.mn[2], 0.0f);
+    S.sub_rec[3 * rec + 1] = make_float4(b.mx[0], b.mx[1], b.mx[2], 0.0f);
+}
+
+// Node records of a subtree's task and its children (one thread); rec0: the
+// subtree's first record; *leaf0, *leaf1: whether the children are leaves.
+__device__ void sub_record(const BuildState &S, SubShared &sh, int nxt, size_t rec0, uint32_t start, uint32_t n,
+                           uint32_t node, int sp, uint32_t lcount, const Aabb &bl, const Aabb &br, int *leaf0,
+                           int *leaf1) {
+    if (sp < 0) {
+        sh.a[node] = (uint16_t)start;
+        sh.b[node] = (uint16_t)n;
+        return;
     }
-    // centroid bounds
+    const uint32_t kid = atomicAdd(&sh.n_nodes, 2u);
+    sh.a[node] = (uint16_t)kid;
+    sh.b[node] = 0;
+    sub_box(S, rec0 + kid, bl);
+    sub_box(S, rec0 + kid + 1, br);
+    const uint32_t counts[2] = {lcount, n - lcount}, starts[2] = {start, start + lcount};
+    for (int c = 0; c < 2; ++c) {
+        const bool leaf = counts[c] <= kLeafMax;
+        *(c ? leaf1 : leaf0) = leaf;
+        if (leaf) {
+            sh.a[kid + c] = (uint16_t)starts[c];
+            sh.b[kid + c] = (uint16_t)counts[c];
+        } else {
+            const uint32_t t = atomicAdd(&sh.n_tasks[nxt], 1u);
+            sh.t_start[nxt][t] = (uint16_t)starts[c];
+            sh.t_count[nxt][t] = (uint16_t)counts[c];
+            sh.t_node[nxt][t] = (uint16_t)(kid + c);
+            sh.t_area[nxt][t] = fmaxf(half_area(c ? br : bl), 1e-8f);
+            const uint32_t k = counts[c] <= 8u ? 0u : (counts[c] <= 16u ? 1u : 2u);
+            sh.of_class[nxt][k][atomicAdd(&sh.n_class[nxt][k], 1u)] = (uint8_t)t;
+        }
+    }
+}
+
+// A primitive's bins on the three axes, 4 bits each (0 on a flat axis).
+__device__ __forceinline__ uint32_t bins_of(const float c[3], const float cb[6]) {
+    uint32_t bits = 0;
+    for (int a = 0; a < 3; ++a) {
+        const float len = cb[3 + a] - cb[a];
+        if (!(len < 1e-8f)) bits |= bin_of(c[a], cb[a], len) << (4 * a);
+    }
+    return bits;
+}
+constexpr uint32_t kNoBins = 0xfffu;       // staged place without a primitive
+
+// Tasks of at most G primitives, 32 / G of them by one warp, a group of G lanes
+// each (have_task: the group has one).  A lane holds a primitive, then a bin:
+// with G = 8 the bins of one axis per round, with G = 16 of two.
+template <uint32_t G>
+__device__ void sub_task_group(BuildState &S, SubShared &sh, int cur, bool have_task, uint32_t t, size_t rec0,
+                               uint32_t lane, unsigned *scratch) {
+    const uint32_t gl = lane & (G - 1u), g0 = lane & ~(G - 1u);
+    const unsigned group = G == 32u ? kFull : ((1u << (G & 31u)) - 1u) << g0;
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t start = 0, n = 0, node = 0;
+    float parent = 1.0f;
+    if (have_task) {
+        start = sh.t_start[cur][t]; n = sh.t_count[cur][t]; node = sh.t_node[cur][t];
+        parent = sh.t_area[cur][t];
+    }
+    const bool have = gl < n;
+    const uint32_t p = have ? sh.perm[cur][start + gl] : 0u;
+    float c[3], cb[6];
+    for (int a = 0; a < 3; ++a) {
+        c[a] = sh.c[a][p];
+        const unsigned o = f2ord(c[a]);
+        unsigned lo = have ? o : kFull, hi = have ? o : 0u;
+#pragma unroll
+        for (uint32_t h = G / 2; h; h >>= 1) {
+            lo = min(lo, __shfl_xor_sync(kFull, lo, h));
+            hi = max(hi, __shfl_xor_sync(kFull, hi, h));
+        }
+        cb[a] = ord2f(lo);
+        cb[3 + a] = ord2f(hi);
+    }
+    const uint32_t bits = bins_of(c, cb);
+    float4 *stage = reinterpret_cast<float4 *>(scratch);
+    __syncwarp();
+    stage[2 * lane] = make_float4(sh.mn[0][p], sh.mn[1][p], sh.mn[2][p], sh.mx[0][p]);
+    stage[2 * lane + 1] = make_float4(sh.mx[1][p], sh.mx[2][p], __uint_as_float(have ? bits : kNoBins), 0.0f);
+    __syncwarp();
+    LaneSplit best;
+    const uint32_t longest = __reduce_max_sync(kFull, n);
+#pragma unroll
+    for (uint32_t r = 0; r < (G == 8u ? 3u : (G == 16u ? 2u : 1u)); ++r) {
+        const uint32_t axis = r * (G / 8u) + (gl >> 3), bin = gl & 7u;
+        LaneBin mine{0u, aabb_empty()};
+        bin_add(mine, stage + 2 * g0, longest, axis, bin);
+        const float lo = axis == 0 ? cb[0] : (axis == 1 ? cb[1] : cb[2]);
+        const float hi = axis == 0 ? cb[3] : (axis == 1 ? cb[4] : cb[5]);
+        bin_candidate(mine, axis, bin, hi - lo < 1e-8f, n, parent, best);
+    }
+    const bool split = best_split<G>(best, lane);
+    int leaf0 = 0, leaf1 = 0;
+    if (gl == 0 && have_task)
+        sub_record(S, sh, cur ^ 1, rec0, start, n, node, split ? 0 : -1, best.l, best.lb, best.rb, &leaf0, &leaf1);
+    leaf0 = __shfl_sync(kFull, leaf0, (int)g0);
+    leaf1 = __shfl_sync(kFull, leaf1, (int)g0);
+    // stable partition; positions in a leaf are final in both orders
+    uint16_t *out0 = sh.perm[cur ^ 1], *out1 = sh.perm[cur];
+    const bool left = have && split && ((bits >> (4u * (best.k / 7u))) & 15u) <= 6u - best.k % 7u;
+    const unsigned lm = __ballot_sync(kFull, left) & group, rm = __ballot_sync(kFull, have && !left) & group;
+    if (have) {
+        const uint32_t pos = !split ? start + gl : left ? start + __popc(lm & below) : start + best.l + __popc(rm & below);
+        out0[pos] = (uint16_t)p;
+        if (split && (left ? leaf0 : leaf1)) out1[pos] = (uint16_t)p;
+    }
+}
+
+// Stages the primitive of position i (none: i >= end) in the warp's scratch.
+__device__ __forceinline__ void stage_position(const SubShared &sh, const uint16_t *in, uint32_t i, uint32_t end,
+                                               const float cb[6], uint32_t lane, float4 *stage) {
+    const bool have = i < end;
+    const uint32_t p = have ? in[i] : 0u;
+    const float c[3] = {sh.c[0][p], sh.c[1][p], sh.c[2][p]};
+    const uint32_t bits = bins_of(c, cb);
+    __syncwarp();
+    stage[2 * lane] = make_float4(sh.mn[0][p], sh.mn[1][p], sh.mn[2][p], sh.mx[0][p]);
+    stage[2 * lane + 1] = make_float4(sh.mx[1][p], sh.mx[2][p], __uint_as_float(have ? bits : kNoBins), 0.0f);
+    __syncwarp();
+}
+__device__ __forceinline__ bool axis_flat(const float cb[6], uint32_t axis) {
+    const float lo = axis == 0 ? cb[0] : (axis == 1 ? cb[1] : cb[2]);
+    const float hi = axis == 0 ? cb[3] : (axis == 1 ? cb[4] : cb[5]);
+    return hi - lo < 1e-8f;
+}
+
+// A task of 33 to kSubCoop primitives, by one warp.
+__device__ void sub_task_warp(BuildState &S, SubShared &sh, int cur, uint32_t t, size_t rec0, uint32_t lane,
+                              unsigned *scratch) {
+    const uint32_t start = sh.t_start[cur][t], n = sh.t_count[cur][t], node = sh.t_node[cur][t];
+    const uint16_t *in = sh.perm[cur];
+    uint16_t *out0 = sh.perm[cur ^ 1], *out1 = sh.perm[cur];
+    const unsigned below = (1u << lane) - 1u;
     unsigned co[6] = {kFull, kFull, kFull, 0u, 0u, 0u};
-    auto add_centroid = [&](float4 c) {
-        const unsigned q[3] = {f2ord(c.x), f2ord(c.y), f2ord(c.z)};
-        for (int a = 0; a < 3; ++a) { co[a] = min(co[a], q[a]); co[3 + a] = max(co[3 + a], q[a]); }
-    };
-    if (one) {
-        if (in0) add_centroid(c0);
-    } else {
-        for (uint32_t i = start + lane; i < start + n; i += 32) add_centroid(S.pcen[perm_in[i]]);
+    for (uint32_t i = start + lane; i < start + n; i += 32u) {
+        const uint32_t p = in[i];
+        for (int a = 0; a < 3; ++a) {
+            const unsigned o = f2ord(sh.c[a][p]);
+            co[a] = min(co[a], o);
+            co[3 + a] = max(co[3 + a], o);
+        }
     }
     float cb[6];
     for (int a = 0; a < 3; ++a) {
         cb[a] = ord2f(__reduce_min_sync(kFull, co[a]));
         cb[3 + a] = ord2f(__reduce_max_sync(kFull, co[3 + a]));
     }
-    // bins (ordered-integer form while accumulating, then floats for the split);
-    // lane j < 24 initialises and converts bin j
-    unsigned *ubins = reinterpret_cast<unsigned *>(wbins[w]);
-    if (lane < 3u * kBins) {
-        unsigned *q = ubins + lane * kBinStride;
-        q[0] = 0u;
-        for (int a = 0; a < 3; ++a) { q[1 + a] = kOrdPosInf; q[4 + a] = kOrdNegInf; }
+    float4 *stage = reinterpret_cast<float4 *>(scratch);
+    LaneBin mine{0u, aabb_empty()};
+    for (uint32_t base = start; base < start + n; base += 32u) {
+        stage_position(sh, in, base + lane, start + n, cb, lane, stage);
+        bin_add(mine, stage, 32u, lane >> 3, lane & 7u);
     }
-    __syncwarp();
-    uint32_t b0[3] = {0u, 0u, 0u};                             // one: the lane's bins
-    if (one) {
-        const unsigned mn[3] = {f2ord(mn0.x), f2ord(mn0.y), f2ord(mn0.z)};
-        const unsigned mx[3] = {f2ord(mx0.x), f2ord(mx0.y), f2ord(mx0.z)};
-        bins_warp(S, ubins, in0 ? 0 : -1, c0, cb, mn, mx, lane, b0);
-    } else {
-        for (uint32_t base = start; base < start + n; base += 32) {     // warp-uniform
-            const uint32_t i = base + lane;
-            const bool in = i < start + n;
-            float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f), bmn = c, bmx = c;
-            if (in) {
-                const uint32_t id = perm_in[i];
-                c = S.pcen[id]; bmn = S.pmin[id]; bmx = S.pmax[id];
-            }
-            const unsigned mn[3] = {f2ord(bmn.x), f2ord(bmn.y), f2ord(bmn.z)};
-            const unsigned mx[3] = {f2ord(bmx.x), f2ord(bmx.y), f2ord(bmx.z)};
-            uint32_t b[3];
-            bins_warp(S, ubins, in ? 0 : -1, c, cb, mn, mx, lane, b);
-        }
-    }
-    __syncwarp();
-    if (lane < 3u * kBins) {
-        unsigned *q = ubins + lane * kBinStride;
-        for (int j = 1; j < kBinStride; ++j) q[j] = __float_as_uint(ord2f(q[j]));
-    }
-    __syncwarp();
-    const float *bins = wbins[w];
-    // split (the whole warp), child ids (lane 0)
-    int ct0 = -1, ct1 = -1;
-    uint32_t lcount = 0;
-    Aabb bl = aabb_empty(), br = aabb_empty();
-    const int sp = choose_split_warp(n, S.t_bounds[cur] + 6 * t, cb, bins, lane, &lcount, &bl, &br);
-    if (lane == 0) {
-        uint32_t c0 = 0, s0 = 0, y0 = 0;
-        if (sp >= 0) {
-            c0 = atomicAdd(S.counters + 1, 2u);
-            const uint32_t m = child_small(n, lcount);           // a small task has no large child
-            if (m) s0 = atomicAdd(S.counters + 4, m);
-            const uint32_t q = child_tiny(n, lcount);
-            if (q) y0 = atomicAdd(S.counters + 6, q);
-        }
-        int ct[2];
-        record_task(S, cur ^ 1, start, n, node, sp, lcount, bl, br, c0, 0u, s0, y0, ct);
-        ct0 = ct[0];
-        ct1 = ct[1];
-    }
-    ct0 = __shfl_sync(0xffffffffu, ct0, 0);
-    ct1 = __shfl_sync(0xffffffffu, ct1, 0);
-    uint32_t *out0 = S.perm[cur ^ 1], *out1 = S.perm[cur];
-    const unsigned below = (1u << lane) - 1u;
-    const int axis = sp >> 4, bin = sp & 15;
-    if (one) {
-        if (sp < 0) {                                          // a leaf: positions stay
-            if (in0) out0[start + lane] = id0;
-            return;
-        }
-        // the split axis has an extent, so b0[axis] is the lane's bin on it
-        const uint32_t my_bin = axis == 0 ? b0[0] : (axis == 1 ? b0[1] : b0[2]);
-        const bool left = in0 && my_bin <= (uint32_t)bin;
-        const unsigned lm = __ballot_sync(kFull, left);
-        const unsigned rm = __ballot_sync(kFull, in0 && !left);
-        if (in0) {
-            const uint32_t pos = left ? start + __popc(lm & below) : start + lcount + __popc(rm & below);
-            out0[pos] = id0;
-            if ((left ? ct0 : ct1) < 0) out1[pos] = id0;       // in a leaf: final in both buffers
-        }
+    LaneSplit best;
+    bin_candidate(mine, lane >> 3, lane & 7u, axis_flat(cb, lane >> 3), n, sh.t_area[cur][t], best);
+    const bool split = best_split<32>(best, lane);
+    int leaf0 = 0, leaf1 = 0;
+    if (lane == 0) sub_record(S, sh, cur ^ 1, rec0, start, n, node, split ? 0 : -1, best.l, best.lb, best.rb, &leaf0, &leaf1);
+    leaf0 = __shfl_sync(kFull, leaf0, 0);
+    leaf1 = __shfl_sync(kFull, leaf1, 0);
+    if (!split) {
+        for (uint32_t i = start + lane; i < start + n; i += 32u) out0[i] = in[i];
         return;
     }
-    if (sp < 0) {                                              // a leaf: positions stay
-        for (uint32_t i = start + lane; i < start + n; i += 32) out0[i] = perm_in[i];
-        return;
-    }
-    // stable partition by ballot, in position order
-    const float len = cb[3 + axis] - cb[axis];
+    const uint32_t axis = best.k / 7u, bin = 6u - best.k % 7u, lcount = best.l;
+    const float lo = axis == 0 ? cb[0] : (axis == 1 ? cb[1] : cb[2]);
+    const float len = (axis == 0 ? cb[3] : (axis == 1 ? cb[4] : cb[5])) - lo;
     uint32_t lbase = start, rbase = start + lcount;
-    for (uint32_t base = start; base < start + n; base += 32) {
+    for (uint32_t base = start; base < start + n; base += 32u) {
         const uint32_t i = base + lane;
-        const bool valid = i < start + n;
-        uint32_t id = 0;
-        bool left = false;
-        if (valid) {
-            id = perm_in[i];
-            const float4 c = S.pcen[id];
-            const float cc = axis == 0 ? c.x : (axis == 1 ? c.y : c.z);
-            left = bin_of(cc, cb[axis], len) <= (uint32_t)bin;
-        }
-        const unsigned lm = __ballot_sync(0xffffffffu, valid && left);
-        const unsigned rm = __ballot_sync(0xffffffffu, valid && !left);
-        if (valid) out0[left ? lbase + __popc(lm & below) : rbase + __popc(rm & below)] = id;
+        const bool have = i < start + n;
+        const uint32_t p = have ? in[i] : 0u;
+        const bool left = have && bin_of(sh.c[axis][p], lo, len) <= bin;
+        const unsigned lm = __ballot_sync(kFull, left), rm = __ballot_sync(kFull, have && !left);
+        if (have) out0[left ? lbase + __popc(lm & below) : rbase + __popc(rm & below)] = (uint16_t)p;
         lbase += __popc(lm);
         rbase += __popc(rm);
     }
-    // a child that is a leaf: its positions are final, copy them into the input
-    // buffer too (after every read of that buffer above)
-    __syncwarp();
-    if (ct0 < 0)
-        for (uint32_t i = start + lane; i < start + lcount; i += 32) out1[i] = out0[i];
-    if (ct1 < 0)
-        for (uint32_t i = start + lcount + lane; i < start + n; i += 32) out1[i] = out0[i];
+    __syncwarp();                                              // every read of this order is done
+    if (leaf0)
+        for (uint32_t i = start + lane; i < start + lcount; i += 32u) out1[i] = out0[i];
+    if (leaf1)
+        for (uint32_t i = start + lcount + lane; i < start + n; i += 32u) out1[i] = out0[i];
 }
 
-constexpr int kTinyThreads = 128;
-
-// Tiny tasks (at most kTinyTask primitives): one thread each runs the serial
-// algorithm — centroid bounds, the 8 bins of one axis at a time in its own
-// column of shared memory (a column per thread, so lanes never share a bank),
-// the sweep of split_axis, and the stable partition.  Child ids are reserved
-// per warp; every child of a tiny task is a leaf or tiny.
-__global__ void __launch_bounds__(kTinyThreads) k_tiny_level(BuildState S, int cur) {
-    __shared__ unsigned sb[kBins * kBinStride][kTinyThreads];
-    const uint32_t tid = threadIdx.x, lane = tid & 31u;
-    const uint32_t k = blockIdx.x * kTinyThreads + tid;
-    const uint32_t ntiny = S.counters[7];
-    if ((k & ~31u) >= ntiny) return;                           // whole warps
-    const bool active = k < ntiny;
-    uint32_t start = 0, n = 0, node = 0;
-    if (active) { start = S.y_start[cur][k]; n = S.y_count[cur][k]; node = S.y_node[cur][k]; }
-    const uint32_t *perm_in = S.perm[cur];
+// A task above kSubCoop primitives, by the whole block.
+__device__ void sub_task_block(BuildState &S, SubShared &sh, int cur, uint32_t t, size_t rec0) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+    const uint32_t start = sh.t_start[cur][t], n = sh.t_count[cur][t], node = sh.t_node[cur][t];
+    const uint16_t *in = sh.perm[cur];
+    if (tid < 6u) sh.red[tid] = tid < 3u ? kOrdPosInf : kOrdNegInf;
+    __syncthreads();
     unsigned co[6] = {kFull, kFull, kFull, 0u, 0u, 0u};
-    for (uint32_t j = 0; j < n; ++j) {
-        const float4 c = S.pcen[perm_in[start + j]];
-        const unsigned q[3] = {f2ord(c.x), f2ord(c.y), f2ord(c.z)};
-        for (int a = 0; a < 3; ++a) { co[a] = min(co[a], q[a]); co[3 + a] = max(co[3 + a], q[a]); }
-    }
-    float cb[6], tb[6];
-    for (int a = 0; a < 6; ++a) {
-        cb[a] = ord2f(co[a]);
-        tb[a] = active ? S.y_bounds[cur][6 * k + a] : 0.0f;
-    }
-    const float parent = node_half_area(tb);
-    SplitBest best = split_best_init(n);
-    for (int axis = 0; axis < 3; ++axis) {
-        const float len = cb[3 + axis] - cb[axis];
-        if (!active || len < 1e-8f) continue;
-        for (int b = 0; b < kBins; ++b) {
-            sb[b * kBinStride][tid] = 0u;
-            for (int a = 0; a < 3; ++a) {
-                sb[b * kBinStride + 1 + a][tid] = kOrdPosInf;
-                sb[b * kBinStride + 4 + a][tid] = kOrdNegInf;
-            }
+    for (uint32_t i = start + tid; i < start + n; i += kSubThreads) {
+        const uint32_t p = in[i];
+        for (int a = 0; a < 3; ++a) {
+            const unsigned o = f2ord(sh.c[a][p]);
+            co[a] = min(co[a], o);
+            co[3 + a] = max(co[3 + a], o);
         }
-        for (uint32_t j = 0; j < n; ++j) {
-            const uint32_t id = perm_in[start + j];
-            const float4 c = S.pcen[id], bmn = S.pmin[id], bmx = S.pmax[id];
-            const float cc = axis == 0 ? c.x : (axis == 1 ? c.y : c.z);
-            const uint32_t o = bin_of(cc, cb[axis], len) * kBinStride;
-            const unsigned mn[3] = {f2ord(bmn.x), f2ord(bmn.y), f2ord(bmn.z)};
-            const unsigned mx[3] = {f2ord(bmx.x), f2ord(bmx.y), f2ord(bmx.z)};
-            sb[o][tid] += 1u;
-            for (int a = 0; a < 3; ++a) {
-                sb[o + 1 + a][tid] = min(sb[o + 1 + a][tid], mn[a]);
-                sb[o + 4 + a][tid] = max(sb[o + 4 + a][tid], mx[a]);
-            }
+    }
+    for (int a = 0; a < 3; ++a) {
+        co[a] = __reduce_min_sync(kFull, co[a]);
+        co[3 + a] = __reduce_max_sync(kFull, co[3 + a]);
+    }
+    if (lane == 0)
+        for (int a = 0; a < 3; ++a) { atomicMin(&sh.red[a], co[a]); atomicMax(&sh.red[3 + a], co[3 + a]); }
+    __syncthreads();
+    float cb[6];
+    for (int a = 0; a < 6; ++a) cb[a] = ord2f(sh.red[a]);
+    float4 *stage = reinterpret_cast<float4 *>(sh.scratch[w]);
+    LaneBin mine{0u, aabb_empty()};
+    for (uint32_t base = start + 32u * w; base < start + n; base += kSubThreads) {
+        stage_position(sh, in, base + lane, start + n, cb, lane, stage);
+        bin_add(mine, stage, 32u, lane >> 3, lane & 7u);
+    }
+    __syncwarp();
+    if (lane < 24u) {                                          // the warp's bins over its staged primitives
+        unsigned *q = sh.scratch[w] + lane * kBinStride;
+        q[0] = mine.n;
+        for (int a = 0; a < 3; ++a) {
+            q[1 + a] = __float_as_uint(mine.b.mn[a]);
+            q[4 + a] = __float_as_uint(mine.b.mx[a]);
         }
-        split_axis(axis, parent, [&](int b, int f) {
-            const unsigned v = sb[b * kBinStride + f][tid];
-            return f == 0 ? __uint_as_float(v) : ord2f(v);
-        }, best);
     }
-    uint32_t lcount = 0;
-    Aabb bl = aabb_empty(), br = aabb_empty();
-    const int sp = active ? split_result(best, n, &lcount, &bl, &br) : -1;
-    // child ids for the warp: prefix sums by shuffles, one atomic per counter
-    const uint32_t my_nodes = sp >= 0 ? 2u : 0u;
-    const uint32_t my_tiny = sp >= 0 ? child_tiny(n, lcount) : 0u;
-    uint32_t pn = my_nodes, py = my_tiny;
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t a = __shfl_up_sync(kFull, pn, off), b = __shfl_up_sync(kFull, py, off);
-        if ((int)lane >= off) { pn += a; py += b; }
+    __syncthreads();
+    if (w == 0) {
+        mine = LaneBin{0u, aabb_empty()};
+        if (lane < 24u)
+            for (uint32_t k = 0; k < kSubWarps; ++k) {
+                const unsigned *q = sh.scratch[k] + lane * kBinStride;
+                mine.n += q[0];
+                for (int a = 0; a < 3; ++a) {
+                    mine.b.mn[a] = fminf(mine.b.mn[a], __uint_as_float(q[1 + a]));
+                    mine.b.mx[a] = fmaxf(mine.b.mx[a], __uint_as_float(q[4 + a]));
+                }
+            }
+        LaneSplit best;
+        bin_candidate(mine, lane >> 3, lane & 7u, axis_flat(cb, lane >> 3), n, sh.t_area[cur][t], best);
+        const bool split = best_split<32>(best, lane);
+        if (lane == 0) {
+            sh.split = split ? (int)best.k : -1;
+            sh.lcount = best.l;
+            sub_record(S, sh, cur ^ 1, rec0, start, n, node, split ? 0 : -1, best.l, best.lb, best.rb,
+                       &sh.leaf_child[0], &sh.leaf_child[1]);
+        }
     }
-    const uint32_t tn = __shfl_sync(kFull, pn, 31), ty = __shfl_sync(kFull, py, 31);
-    uint32_t bn = 0, by = 0;
-    if (lane == 0) {
-        if (tn) bn = atomicAdd(S.counters + 1, tn);
-        if (ty) by = atomicAdd(S.counters + 6, ty);
-    }
-    bn = __shfl_sync(kFull, bn, 0);
-    by = __shfl_sync(kFull, by, 0);
-    if (!active) return;
-    int ct[2];
-    record_task(S, cur ^ 1, start, n, node, sp, lcount, bl, br, bn + pn - my_nodes, 0u, 0u, by + py - my_tiny, ct);
-    uint32_t *out0 = S.perm[cur ^ 1], *out1 = S.perm[cur];
-    if (sp < 0) {                                              // a leaf: positions stay
-        for (uint32_t j = 0; j < n; ++j) out0[start + j] = perm_in[start + j];
+    __syncthreads();
+    const int k = sh.split;
+    uint16_t *out0 = sh.perm[cur ^ 1], *out1 = sh.perm[cur];
+    if (k < 0) {
+        for (uint32_t i = start + tid; i < start + n; i += kSubThreads) out0[i] = in[i];
+        __syncthreads();
         return;
     }
-    // stable partition, then the positions of leaf children into the input
-    // buffer too (after every read of it)
-    const int axis = sp >> 4, bin = sp & 15;
-    const float len = cb[3 + axis] - cb[axis];
-    uint32_t lp = start, rp = start + lcount;
-    for (uint32_t j = 0; j < n; ++j) {
-        const uint32_t id = perm_in[start + j];
-        const float4 c = S.pcen[id];
-        const float cc = axis == 0 ? c.x : (axis == 1 ? c.y : c.z);
-        const bool left = bin_of(cc, cb[axis], len) <= (uint32_t)bin;
-        out0[left ? lp++ : rp++] = id;
+    // stable partition: a contiguous share of the positions per warp
+    const int axis = k / 7;
+    const uint32_t bin = (uint32_t)(6 - k % 7), lcount = sh.lcount;
+    const float lo = ord2f(sh.red[axis]), len = ord2f(sh.red[3 + axis]) - lo;
+    const uint32_t share = (n + kSubThreads - 1u) / kSubThreads * 32u;
+    const uint32_t first = start + min(w * share, n), last = start + min((w + 1u) * share, n);
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t lefts = 0;
+    for (uint32_t base = first; base < last; base += 32u) {
+        const uint32_t i = base + lane;
+        const bool left = i < last && bin_of(sh.c[axis][in[i]], lo, len) <= bin;
+        lefts += __popc(__ballot_sync(kFull, left));
     }
-    if (ct[0] < 0)
-        for (uint32_t p = start; p < start + lcount; ++p) out1[p] = out0[p];
-    if (ct[1] < 0)
-        for (uint32_t p = start + lcount; p < start + n; ++p) out1[p] = out0[p];
+    if (lane == 0) sh.warp_left[w] = lefts;
+    __syncthreads();
+    uint32_t lbase = start;
+    for (uint32_t j = 0; j < w; ++j) lbase += sh.warp_left[j];
+    uint32_t rbase = start + lcount + (first - start) - (lbase - start);
+    for (uint32_t base = first; base < last; base += 32u) {
+        const uint32_t i = base + lane;
+        const bool have = i < last;
+        const uint32_t p = have ? in[i] : 0u;
+        const bool left = have && bin_of(sh.c[axis][p], lo, len) <= bin;
+        const unsigned lm = __ballot_sync(kFull, left), rm = __ballot_sync(kFull, have && !left);
+        if (have) out0[left ? lbase + __popc(lm & below) : rbase + __popc(rm & below)] = (uint16_t)p;
+        lbase += __popc(lm);
+        rbase += __popc(rm);
+    }
+    __syncthreads();
+    if (sh.leaf_child[0])
+        for (uint32_t i = start + tid; i < start + lcount; i += kSubThreads) out1[i] = out0[i];
+    if (sh.leaf_child[1])
+        for (uint32_t i = start + lcount + tid; i < start + n; i += kSubThreads) out1[i] = out0[i];
+    __syncthreads();
 }
 
-// The start of a level without large tasks (level_advance alone).
-__global__ void k_level_advance(BuildState S, uint32_t level) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) level_advance(S, level);
+// One block per subtree: its nodes into sub_rec (links and pre-order indices
+// local to the subtree), the final order of its positions into perm[buf], its
+// size into n_size of its root.
+__global__ void __launch_bounds__(kSubThreads, 3) k_subtrees(BuildState S, int buf) {
+    extern __shared__ __align__(16) unsigned char sub_smem[];
+    SubShared &sh = *reinterpret_cast<SubShared *>(sub_smem);
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+    const uint32_t start = S.sub_start[blockIdx.x], n = S.sub_count[blockIdx.x], node = S.sub_node[blockIdx.x];
+    const size_t rec0 = 2 * (size_t)start;
+    for (uint32_t i = tid; i < n; i += kSubThreads) {
+        const uint32_t id = S.perm[buf][start + i];
+        const float4 c = S.pcen[id], mn = S.pmin[id], mx = S.pmax[id];
+        sh.c[0][i] = c.x; sh.c[1][i] = c.y; sh.c[2][i] = c.z;
+        sh.mn[0][i] = mn.x; sh.mn[1][i] = mn.y; sh.mn[2][i] = mn.z;
+        sh.mx[0][i] = mx.x; sh.mx[1][i] = mx.y; sh.mx[2][i] = mx.z;
+        sh.perm[0][i] = (uint16_t)i;
+    }
+    if (tid == 0) {
+        const float4 mn = S.n_min[node], mx = S.n_max[node];
+        Aabb b;
+        b.mn[0] = mn.x; b.mn[1] = mn.y; b.mn[2] = mn.z;
+        b.mx[0] = mx.x; b.mx[1] = mx.y; b.mx[2] = mx.z;
+        sub_box(S, rec0, b);
+        sh.t_start[0][0] = 0; sh.t_count[0][0] = (uint16_t)n; sh.t_node[0][0] = 0;
+        sh.t_area[0][0] = fmaxf(half_area(b), 1e-8f);
+        sh.n_nodes = 1;
+        sh.n_tasks[0] = 1; sh.n_tasks[1] = 0;
+        for (int k = 0; k < 3; ++k) sh.n_class[0][k] = sh.n_class[1][k] = 0;
+        const uint32_t k = n <= 8u ? 0u : (n <= 16u ? 1u : 2u);
+        sh.n_class[0][k] = 1;
+        sh.of_class[0][k][0] = 0;
+        sh.level_end[0] = 1;
+    }
+    int cur = 0;
+    uint32_t levels = 0;
+    for (;;) {
+        __syncthreads();
+        const uint32_t tasks = sh.n_tasks[cur];
+        if (tasks == 0) break;
+        bool wide = false;                                     // uniform: every thread reads the same counts
+        if (tasks <= kSub / kSubCoop)
+            for (uint32_t t = 0; t < tasks; ++t)
+                if (sh.t_count[cur][t] > kSubCoop) { sub_task_block(S, sh, cur, t, rec0); wide = true; }
+        if (wide) __syncthreads();
+        // the level's remaining tasks: the larger ones first, then two and four of the smaller ones per warp
+        const uint32_t n2 = sh.n_class[cur][2], n1 = sh.n_class[cur][1], n0 = sh.n_class[cur][0];
+        const uint32_t items = n2 + (n1 + 1u) / 2u + (n0 + 3u) / 4u;
+        for (uint32_t k = w; k < items; k += kSubWarps) {
+            if (k < n2) {
+                const uint32_t t = sh.of_class[cur][2][k], cnt = sh.t_count[cur][t];
+                if (cnt <= 32u) sub_task_group<32>(S, sh, cur, true, t, rec0, lane, sh.scratch[w]);
+                else if (cnt <= kSubCoop || tasks > kSub / kSubCoop) sub_task_warp(S, sh, cur, t, rec0, lane, sh.scratch[w]);
+            } else if (k < n2 + (n1 + 1u) / 2u) {
+                const uint32_t j = 2u * (k - n2) + (lane >> 4);
+                sub_task_group<16>(S, sh, cur, j < n1, j < n1 ? sh.of_class[cur][1][j] : 0u, rec0, lane, sh.scratch[w]);
+            } else {
+                const uint32_t j = 4u * (k - n2 - (n1 + 1u) / 2u) + (lane >> 3);
+                sub_task_group<8>(S, sh, cur, j < n0, j < n0 ? sh.of_class[cur][0][j] : 0u, rec0, lane, sh.scratch[w]);
+            }
+        }
+        __syncthreads();
+        ++levels;
+        if (tid == 0) {
+            sh.n_tasks[cur] = 0;
+            for (int k = 0; k < 3; ++k) sh.n_class[cur][k] = 0;
+            sh.level_end[levels] = (uint16_t)sh.n_nodes;
+        }
+        cur ^= 1;
+    }
+    // subtree sizes bottom-up, pre-order indices top-down: level k holds the nodes [level_end[k - 1], level_end[k])
+    for (uint32_t k = levels + 1; k-- > 0;) {
+        for (uint32_t i = (k ? sh.level_end[k - 1] : 0u) + tid; i < sh.level_end[k]; i += kSubThreads)
+            sh.size[i] = sh.b[i] ? 1u : (uint16_t)(1u + sh.size[sh.a[i]] + sh.size[sh.a[i] + 1u]);
+        __syncthreads();
+    }
+    if (tid == 0) sh.pre[0] = 0;
+    __syncthreads();
+    for (uint32_t k = 0; k <= levels; ++k) {
+        for (uint32_t i = (k ? sh.level_end[k - 1] : 0u) + tid; i < sh.level_end[k]; i += kSubThreads)
+            if (!sh.b[i]) {
+                const uint32_t l = sh.a[i];
+                sh.pre[l] = (uint16_t)(sh.pre[i] + 1u);
+                sh.pre[l + 1u] = (uint16_t)(sh.pre[i] + 1u + sh.size[l]);
+            }
+        __syncthreads();
+    }
+    for (uint32_t i = tid; i < sh.n_nodes; i += kSubThreads) {
+        const uint32_t count = sh.b[i], link = count ? start + sh.a[i] : (uint32_t)sh.pre[sh.a[i] + 1u];
+        S.sub_rec[3 * (rec0 + i) + 2] = make_float4(__uint_as_float(link), __uint_as_float(count),
+                                                    __uint_as_float((uint32_t)sh.pre[i]), 0.0f);
+    }
+    uint32_t id[kSub / kSubThreads];
+    for (uint32_t k = 0; k < kSub / kSubThreads; ++k) {
+        const uint32_t i = k * kSubThreads + tid;
+        if (i < n) id[k] = S.perm[buf][start + sh.perm[cur][i]];
+    }
+    __syncthreads();
+    for (uint32_t k = 0; k < kSub / kSubThreads; ++k) {
+        const uint32_t i = k * kSubThreads + tid;
+        if (i < n) S.perm[buf][start + i] = id[k];
+    }
+    if (tid == 0) {
+        S.n_size[node] = sh.n_nodes;
+        S.n_a[node] = start;
+        atomicMax(S.counters + 10, levels);
+    }
+}
+
+// The subtrees' nodes into their places, one block per subtree.
+__global__ void __launch_bounds__(256) k_emit_subtrees(BuildState S, mcrt_gpu_bvh_node *out) {
+    const uint32_t start = S.sub_start[blockIdx.x], node = S.sub_node[blockIdx.x];
+    const uint32_t base = S.n_pre[node], size = S.n_size[node];
+    const float4 *rec = S.sub_rec + 6 * (size_t)start;
+    for (uint32_t i = threadIdx.x; i < size; i += 256u) {
+        const float4 mn = rec[3 * (size_t)i], mx = rec[3 * (size_t)i + 1];
+        float4 link = rec[3 * (size_t)i + 2];
+        const uint32_t pre = __float_as_uint(link.z);
+        if (__float_as_uint(link.y) == 0u) link.x = __uint_as_float(__float_as_uint(link.x) + base);
+        link.z = 0.0f;
+        float4 *o = reinterpret_cast<float4 *>(out + base + pre);
+        o[0] = mn;
+        o[1] = mx;
+        o[2] = link;
+    }
 }
 
 // Partition flag of position i: 1 when its primitive goes to the left child of
@@ -1143,7 +1296,9 @@ __device__ __forceinline__ uint32_t partition_flag(const BuildState &S, int cur,
 // else their sums are added and the window moves back.  Every wait is bounded:
 // after kLookbackPolls polls of a predecessor the tile records the error word
 // and goes on (the host fails the build).
+template <uint32_t kFlagItems>
 __global__ void __launch_bounds__(kFlagThreads) k_flag_scan(BuildState S, int cur) {
+    constexpr uint32_t kFlagTile = kFlagThreads * kFlagItems;
     __shared__ uint32_t s_tile, s_excl, s_warp[kFlagThreads / 32];
     const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
     unsigned long long *status = S.part + 2;
@@ -1206,7 +1361,7 @@ __global__ void __launch_bounds__(kFlagThreads) k_flag_scan(BuildState S, int cu
                 j -= 32;
             }
             if (lane == 0) {
-                if (gave_up) atomicExch(reinterpret_cast<unsigned int *>(S.part + 1), 1u);
+                if (gave_up) atomicExch(S.counters + 9, 1u);
                 __threadfence();
                 atomicExch(status + tile, (2ull << 32) | (excl + block_total));
             }
@@ -1229,7 +1384,6 @@ __global__ void k_scatter(BuildState S, int cur) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= S.nt) return;
     int task = S.ptask[cur][i];
-    if (task == -2) { S.ptask[cur ^ 1][i] = -2; return; }     // a small task's position: k_small_level moves it
     uint32_t id = S.perm[cur][i];
     if (task < 0) { S.perm[cur ^ 1][i] = id; S.ptask[cur ^ 1][i] = -1; return; }
     int sp = S.t_split[task];
@@ -1242,29 +1396,43 @@ __global__ void k_scatter(BuildState S, int cur) {
     if (S.flags[i]) { pos = start + left_rank; child = S.n_a[node]; }
     else { pos = start + lcount + ((i - start) - left_rank); child = S.n_b[node]; }
     S.perm[cur ^ 1][pos] = id;
-    const uint32_t map = S.n_size[child];
-    S.ptask[cur ^ 1][pos] = S.n_leaf[child] ? -1 : (map == kSmallFlag ? -2 : (int)map);
+    S.ptask[cur ^ 1][pos] = S.n_leaf[child] ? -1 : (int)S.n_size[child];   // -1: in a leaf or a subtree
 }
 
-// subtree sizes, bottom-up over a BFS id range
-__global__ void k_sizes(BuildState S, uint32_t begin, uint32_t end) {
-    uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= end) return;
-    S.n_size[i] = S.n_leaf[i] ? 1u : 1u + S.n_size[S.n_a[i]] + S.n_size[S.n_b[i]];
-}
-// pre-order indices, top-down
-__global__ void k_preorder(BuildState S, uint32_t begin, uint32_t end) {
-    uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= end) return;
-    if (S.n_leaf[i]) return;
-    uint32_t p = S.n_pre[i];
-    uint32_t l = S.n_a[i], r = S.n_b[i];
-    S.n_pre[l] = p + 1;
-    S.n_pre[r] = p + 1 + S.n_size[l];
+// Subtree sizes (bottom-up) and pre-order indices (top-down) of the nodes above
+// the subtrees, one block: a level is a few hundred to a few thousand nodes, and
+// a launch per level and direction cost 3.6 us each.
+__global__ void __launch_bounds__(1024) k_upper_order(BuildState S, uint32_t levels) {
+    const uint32_t tid = threadIdx.x;
+    auto begin = [&](uint32_t k) { return k ? S.level_end[k - 1] : 0u; };
+    for (uint32_t k = levels + 1; k-- > 0;) {
+        const uint32_t end = k < levels ? S.level_end[k] : S.counters[1];
+        for (uint32_t i = begin(k) + tid; i < end; i += 1024u) {
+            const uint32_t kind = S.n_leaf[i];
+            if (kind == 1u) S.n_size[i] = 1u;
+            else if (kind == 0u) S.n_size[i] = 1u + S.n_size[S.n_a[i]] + S.n_size[S.n_b[i]];
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        S.n_pre[0] = 0;
+        S.counters[11] = S.n_size[0];
+    }
+    __syncthreads();
+    for (uint32_t k = 0; k <= levels; ++k) {
+        const uint32_t end = k < levels ? S.level_end[k] : S.counters[1];
+        for (uint32_t i = begin(k) + tid; i < end; i += 1024u) {
+            if (S.n_leaf[i] != 0u) continue;
+            const uint32_t p = S.n_pre[i], l = S.n_a[i];
+            S.n_pre[l] = p + 1;
+            S.n_pre[S.n_b[i]] = p + 1 + S.n_size[l];
+        }
+        __syncthreads();
+    }
 }
 __global__ void k_emit(BuildState S, uint32_t n_bfs, mcrt_gpu_bvh_node *out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_bfs) return;
+    if (i >= n_bfs || S.n_leaf[i] == kSubMark) return;        // a subtree's root: k_emit_subtrees
     mcrt_gpu_bvh_node nd;
     float4 mn = S.n_min[i], mx = S.n_max[i];
     nd.aabb_min[0] = mn.x; nd.aabb_min[1] = mn.y; nd.aabb_min[2] = mn.z; nd.aabb_min[3] = 0.0f;
@@ -1312,8 +1480,8 @@ static cudaError_t gpu_build(const mcrt_gpu_vertex *d_verts, const mcrt_gpu_tria
         acc(n * 4); acc(n * 4); acc(n * 4); acc(n * 4);      // sort keys, ids (ping-pong)
         acc(256 * tiles * 4); acc(256 * tiles * 4);          // digit counts, offsets
         acc(n * 16); acc(n * 16); acc(n * 16);               // reordered bounds
-        for (int k = 0; k < 2; ++k) { acc(tc * 4); acc(tc * 4); acc(tc * 4); acc(tc * 24); }   // tiny tasks
-        acc((2 + (n + kFlagTile - 1) / kFlagTile) * 8);     // partition scan state
+        acc(tc * 4); acc(tc * 4); acc(tc * 4); acc(nn * 48);  // subtrees and their nodes
+        acc((2 + (n + kMinFlagTile - 1) / kMinFlagTile) * 8);   // partition scan state
         cudaError_t e = cudaMalloc(&sc->mem, bytes);
         if (e != cudaSuccess) { if (err) *err = "BVH scratch allocation failed"; return e; }
         sc->cap = nt;
@@ -1339,22 +1507,20 @@ static cudaError_t gpu_build(const mcrt_gpu_vertex *d_verts, const mcrt_gpu_tria
         S.rval[0] = carve<uint32_t>(p, n); S.rval[1] = carve<uint32_t>(p, n);
         S.rhist = carve<uint32_t>(p, 256 * tiles); S.roffs = carve<uint32_t>(p, 256 * tiles);
         S.qmin = carve<float4>(p, n); S.qmax = carve<float4>(p, n); S.qcen = carve<float4>(p, n);
-        for (int k = 0; k < 2; ++k) {
-            S.y_start[k] = carve<uint32_t>(p, tc); S.y_count[k] = carve<uint32_t>(p, tc);
-            S.y_node[k] = carve<uint32_t>(p, tc); S.y_bounds[k] = carve<float>(p, 6 * tc);
-        }
-        S.part = carve<unsigned long long>(p, 2 + (n + kFlagTile - 1) / kFlagTile);
+        S.sub_start = carve<uint32_t>(p, tc); S.sub_count = carve<uint32_t>(p, tc); S.sub_node = carve<uint32_t>(p, tc);
+        S.sub_rec = carve<float4>(p, 3 * nn);
+        S.part = carve<unsigned long long>(p, 2 + (n + kMinFlagTile - 1) / kMinFlagTile);
     }
     BuildState S = sc->s;
     S.nt = nt;
-    S.tcap = nt / 4 + 1;                                 // tasks hold > 4 primitives
+    const uint32_t per = nt < kWideBlocks ? 256u : 1024u;    // positions per block of the whole-array passes
     const uint32_t TB = 256;
     const uint32_t nb = (nt + TB - 1) / TB;
     if (d_sph) k_sphere_bounds<<<nb, TB, 0, st>>>(d_sph, S);
     else k_prim_bounds<<<nb, TB, 0, st>>>(d_verts, d_tris, S);
     ::mcrt::note_launch();
     k_root_init<<<1, 32, 0, st>>>(S); ::mcrt::note_launch();
-    k_root_bounds<<<(nt + kPosPerBlock - 1) / kPosPerBlock, 256, 0, st>>>(S); ::mcrt::note_launch();
+    k_root_bounds<<<(nt + per - 1) / per, 256, 0, st>>>(S, per); ::mcrt::note_launch();
     if (nt <= kLeafMax) {
         // the root is a single leaf (bvh.rs:301-304)
         std::vector<float> tb(6);
@@ -1392,113 +1558,75 @@ static cudaError_t gpu_build(const mcrt_gpu_vertex *d_verts, const mcrt_gpu_tria
     // BFS node 0 = root
     cudaMemcpyAsync(S.n_min, S.t_bounds[0], 12, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(S.n_max, S.t_bounds[0] + 3, 12, cudaMemcpyDeviceToDevice, st);
-    // Levels.  Round r builds the tasks of level r: the large ones by the
-    // whole-array passes (while any exist; the host reads their count after
-    // each round), the small ones by k_small_level in the same round.  Once no
-    // large task is left, rounds run in batches of 8 with one host round trip
-    // per batch.  level_end[r] = the BFS node count when round r starts, so
-    // round r creates the nodes [level_end[r], level_end[r + 1]).
-    const uint32_t tcap = S.tcap;
-    const uint32_t nbp = (nt + kPosPerBlock - 1) / kPosPerBlock;
-    uint32_t n_large = 1, n_small = 0, n_tiny = 0;       // tasks of the current level
-    uint32_t level = 0;
+    // Levels of large tasks, by the whole-array passes; level_end[r] = the BFS
+    // node count when level r starts, so level r creates the nodes
+    // [level_end[r], level_end[r + 1]).  A level at most halves the largest task,
+    // so the first log2(nt / kSub) levels run without a look at the count of
+    // large tasks; after those the host reads it once per level.
+    const uint32_t nbp = (nt + per - 1) / per;
+    const uint32_t flag_tile = nt < kWideBlocks ? kMinFlagTile : 4u * kMinFlagTile;
+    const uint32_t n_flag_tiles = (nt + flag_tile - 1) / flag_tile, n_part = 2 + n_flag_tiles;
+    uint32_t host_counters[16] = {};
+    uint32_t level = 0, n_large = nt > kSub ? 1u : 0u, n_sub = 0, n_bfs = 1;
+    uint32_t unseen = 0;                                 // levels to run before the next look
+    while ((uint64_t)kSub << (unseen + 1) <= nt) ++unseen;
     int cur = 0;
-    uint32_t host_counters[8] = {};
-    uint32_t scan_error = 0;
-    const uint32_t n_flag_tiles = (nt + kFlagTile - 1) / kFlagTile;
-    auto level_ok = [&]() -> bool {
+    while (n_large > 0) {
         if (level + 1 >= kMaxLevels) {
             if (err) *err = "BVH build exceeded 4096 levels";
-            return false;
+            return cudaErrorUnknown;
         }
-        return true;
-    };
-    auto advance = [&]() -> bool {
-        if (!level_ok()) return false;
-        k_level_advance<<<1, 1, 0, st>>>(S, level++); ::mcrt::note_launch();
-        return true;
-    };
-    // small and tiny tasks of the current level (bounds: at least their counts)
-    auto small_round = [&](uint64_t small_bound, uint64_t tiny_bound) {
-        const uint32_t warps = (uint32_t)std::min<uint64_t>(small_bound, tcap);
-        if (warps) { k_small_level<<<(warps + 7) / 8, 256, 0, st>>>(S, cur); ::mcrt::note_launch(); }
-        const uint32_t threads = (uint32_t)std::min<uint64_t>(tiny_bound, tcap);
-        if (threads) {
-            k_tiny_level<<<(threads + kTinyThreads - 1) / kTinyThreads, kTinyThreads, 0, st>>>(S, cur);
-            ::mcrt::note_launch();
-        }
-    };
-    const uint32_t n_part = 2 + n_flag_tiles;
-    while (n_large > 0) {
-        if (!level_ok()) return cudaErrorUnknown;
         const uint32_t nw = std::max(n_large * (6 + kTaskBinWords), n_part);
         k_task_reset<<<(nw + TB - 1) / TB, TB, 0, st>>>(S, level++, n_large, n_part); ::mcrt::note_launch();
-        k_centroid_bounds<<<nbp, 256, 0, st>>>(S, cur); ::mcrt::note_launch();
-        k_bins<<<nbp, 256, 0, st>>>(S, cur); ::mcrt::note_launch();
-        k_split<<<(n_large + 127) / 128, 128, 0, st>>>(S, cur, n_large); ::mcrt::note_launch();
-        k_flag_scan<<<n_flag_tiles, kFlagThreads, 0, st>>>(S, cur); ::mcrt::note_launch();
+        k_centroid_bounds<<<nbp, 256, 0, st>>>(S, cur, per); ::mcrt::note_launch();
+        k_bins<<<nbp, 256, 0, st>>>(S, cur, per); ::mcrt::note_launch();
+        k_split<<<(n_large + 3) / 4, 128, 0, st>>>(S, cur); ::mcrt::note_launch();
+        if (nt < kWideBlocks) k_flag_scan<2><<<n_flag_tiles, kFlagThreads, 0, st>>>(S, cur);
+        else k_flag_scan<8><<<n_flag_tiles, kFlagThreads, 0, st>>>(S, cur);
+        ::mcrt::note_launch();
         k_scatter<<<nb, TB, 0, st>>>(S, cur); ::mcrt::note_launch();
-        small_round(n_small, n_tiny);
         cur ^= 1;
+        if (unseen > 1) {                                // at most twice as many, each above kSub primitives
+            --unseen;
+            n_large = std::min(2u * n_large, nt / (kSub + 1u));
+            continue;
+        }
         cudaMemcpyAsync(host_counters, S.counters, sizeof(host_counters), cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&scan_error, S.part + 1, 4, cudaMemcpyDeviceToHost, st);
         cudaError_t e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) { if (err) *err = "BVH build level failed"; return e; }
-        if (scan_error) { if (err) *err = "BVH build: partition scan look-back gave up"; return cudaErrorUnknown; }
+        if (host_counters[9]) { if (err) *err = "BVH build: partition scan look-back gave up"; return cudaErrorUnknown; }
         n_large = host_counters[0];
-        n_small = host_counters[4];
-        n_tiny = host_counters[6];
+        n_bfs = host_counters[1];
+        n_sub = host_counters[4];
     }
-    // positions the whole-array passes finished (leaves) are in perm[cur] only
-    cudaMemcpyAsync(S.perm[cur ^ 1], S.perm[cur], 4 * (size_t)nt, cudaMemcpyDeviceToDevice, st);
-    // upper bounds of a level's small and tiny tasks: a small task has at most
-    // two small or tiny children, a tiny one at most two tiny children
-    uint64_t small_bound = n_small, tiny_bound = n_tiny;
-    while (n_small > 0 || n_tiny > 0) {
-        for (int k = 0; k < 8; ++k) {
-            if (!advance()) return cudaErrorUnknown;
-            small_round(small_bound, tiny_bound);
-            cur ^= 1;
-            tiny_bound = std::min<uint64_t>(2 * (small_bound + tiny_bound), tcap);
-            small_bound = std::min<uint64_t>(2 * small_bound, tcap);
+    if (nt <= kSub) {                                    // the root is a subtree itself
+        k_root_subtree<<<1, 1, 0, st>>>(S); ::mcrt::note_launch();
+        n_sub = 1;
+    }
+    if (n_sub) {
+        static bool configured[64] = {};                 // per device: 70 KB of dynamic shared memory
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev >= 64 || !configured[dev]) {
+            cudaError_t e = cudaFuncSetAttribute(k_subtrees, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)sizeof(SubShared));
+            if (e != cudaSuccess) { if (err) *err = "BVH subtree kernel"; return e; }
+            if (dev < 64) configured[dev] = true;
         }
-        cudaMemcpyAsync(host_counters, S.counters, sizeof(host_counters), cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) { if (err) *err = "BVH build level failed"; return e; }
-        n_small = host_counters[4];
-        n_tiny = host_counters[6];
-        small_bound = n_small;
-        tiny_bound = n_tiny;
+        k_subtrees<<<n_sub, kSubThreads, sizeof(SubShared), st>>>(S, cur); ::mcrt::note_launch();
     }
-    if (!advance()) return cudaErrorUnknown;             // the node count after the last level
-    std::vector<uint32_t> level_begin(level + 1);
-    level_begin[0] = 0;                                  // level 0 is the root alone: [0, 1)
-    cudaMemcpyAsync(level_begin.data() + 1, S.level_end, 4 * (size_t)level, cudaMemcpyDeviceToHost, st);
-    {
-        cudaError_t e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) { if (err) *err = "BVH build level failed"; return e; }
-    }
-    const uint32_t n_bfs = level_begin[level];
-    // BFS ids are allocated level by level: the children of the nodes created by
-    // one level are all created by the next, so subtree sizes are exact when the
-    // levels are swept bottom-up and pre-order indices when swept top-down.
-    {
-        const size_t nl = level_begin.size() - 1;
-        for (size_t k = nl; k-- > 0;) {
-            const uint32_t b = level_begin[k], e = level_begin[k + 1];
-            if (e > b) { k_sizes<<<(e - b + TB - 1) / TB, TB, 0, st>>>(S, b, e); ::mcrt::note_launch(); }
-        }
-        cudaMemsetAsync(S.n_pre, 0, 4, st);
-        for (size_t k = 0; k < nl; ++k) {
-            const uint32_t b = level_begin[k], e = level_begin[k + 1];
-            if (e > b) { k_preorder<<<(e - b + TB - 1) / TB, TB, 0, st>>>(S, b, e); ::mcrt::note_launch(); }
-        }
-    }
+    k_upper_order<<<1, 1024, 0, st>>>(S, level); ::mcrt::note_launch();
     k_emit<<<(n_bfs + TB - 1) / TB, TB, 0, st>>>(S, n_bfs, d_nodes); ::mcrt::note_launch();
+    if (n_sub) { k_emit_subtrees<<<n_sub, 256, 0, st>>>(S, d_nodes); ::mcrt::note_launch(); }
     k_final_order<<<nb, TB, 0, st>>>(S.perm[cur], S.rval[0], nt, d_order); ::mcrt::note_launch();
+    cudaMemcpyAsync(host_counters, S.counters, sizeof(host_counters), cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { if (err) *err = "BVH emit failed"; return e; }
-    *n_nodes_out = n_bfs;
+    if (level + host_counters[10] + 1 >= kMaxLevels) {
+        if (err) *err = "BVH build exceeded 4096 levels";
+        return cudaErrorUnknown;
+    }
+    *n_nodes_out = host_counters[11];
     return cudaSuccess;
 }
 

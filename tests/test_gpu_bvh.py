@@ -46,3 +46,25 @@ def test_bvh_of_negative_zero_coordinates(ctx, oracle, n):
     nodes, want = build_both(ctx, oracle, p)
     for f in ("aabb_min", "aabb_max"):       # by value: which zero a box keeps is the order of its primitives
         assert np.array_equal(nodes[f], want[f])
+
+
+def shape(kind, n, rng):
+    if kind == "cloud":                      # balanced splits
+        c = rng.uniform(-5, 5, (n, 1, 3))
+    elif kind == "chain":                    # a few primitives leave per split: deep trees
+        c = np.zeros((n, 1, 3))
+        c[:, 0, 0] = 1.2 ** (np.arange(n) % 400)
+        c[:, 0, 1] = 4 * (np.arange(n) // 400)
+    else:                                    # clusters of equal triangles: leaves above the leaf size
+        return rng.integers(0, 3, (max(n // 40, 1), 3, 3)).repeat(40, axis=0)[:n].astype(np.float32)
+    return (c + rng.uniform(-0.4, 0.4, (n, 3, 3))).astype(np.float32)
+
+
+# 4 | 5: leaf and smallest subtree; up to 8, 16, 32: tasks of a part of a warp; 256: of a warp; 1024: of one block;
+# 2049 and above: two levels and more above the subtrees
+@pytest.mark.parametrize("kind", ["cloud", "chain", "equal"])
+@pytest.mark.parametrize("n", [4, 5, 8, 9, 16, 17, 32, 33, 128, 129, 257, 1023, 1024, 1025, 2049, 5000])
+def test_bvh_sizes_around_the_subtree_limits(ctx, oracle, n, kind):
+    nodes, want = build_both(ctx, oracle, shape(kind, n, np.random.default_rng(n)))
+    for f in ("aabb_min", "aabb_max"):
+        assert np.array_equal(bits(nodes[f]), bits(want[f]))
