@@ -243,7 +243,7 @@ cudaError_t cache_train_host(CacheState *c, const float *samples16, uint32_t n, 
                              float lr, float *out_loss, float *out_grad, cudaStream_t st, bool *timed_out);
 cudaError_t cache_infer_device(CacheState *c, const float4 *q, const uint32_t *d_count, uint32_t max_n, float *out,
                                float4 *L, const float4 *thr, cudaStream_t st);
-cudaError_t cache_step_device(CacheState *c, const float *d_samples, uint32_t n, uint32_t n_valid, float lr,
+cudaError_t cache_step_device(CacheState *c, const float *d_samples, uint32_t n, uint32_t n_valid, bool count, float lr,
                               cudaStream_t st);
 // Samples from the training paths' records (L: final path radiance per slot), the bias judge, then
 // `steps` Adam steps; no host round trip (capturable once cache_prepare has run for the capacity).

@@ -161,31 +161,31 @@ __device__ __forceinline__ void store_chunk(uint8_t *tile, uint32_t row, int c, 
     *reinterpret_cast<uint4 *>(tile + tc::op_offset(row, 8 * c, kTile)) =
         make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
 }
-__device__ void encode_row_streamed(const NetDev &net, const float q[12], bool valid, uint8_t *tile, uint32_t row) {
-    float u[3];
-    for (int a = 0; a < 3; ++a) {
-        float s = 0.0f, c = 0.0f;
-        if (valid) {
-            const float v = (q[a] - net.lo[a]) * net.inv_ext[a];
-            u[a] = v < 0.0f ? 0.0f : (v > 1.0f ? 1.0f : v);
-            fm_sincos(u[a] * band_freq(0), &s, &c);
-        } else {
-            u[a] = 0.0f;
-        }
+// A coordinate of the query on axis a of the encoding's box, in [0, 1].
+__device__ __forceinline__ float encode_unit(const NetDev &net, float qa, int a) {
+    const float v = (qa - net.lo[a]) * net.inv_ext[a];
+    return v < 0.0f ? 0.0f : (v > 1.0f ? 1.0f : v);
+}
+// The three chunks of axis a.
+__device__ __forceinline__ void encode_axis(float u, bool valid, uint8_t *tile, uint32_t row, int a) {
+    float s = 0.0f, c = 0.0f;
+    if (valid) fm_sincos(u * band_freq(0), &s, &c);
 #pragma unroll
-        for (int ch = 0; ch < 3; ++ch) {
-            float f[8];
+    for (int ch = 0; ch < 3; ++ch) {
+        float f[8];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                f[2 * k] = valid ? s : 0.0f;
-                f[2 * k + 1] = valid ? c : 0.0f;
-                const float s2 = (2.0f * s) * c, c2 = c * c - s * s;
-                s = s2;
-                c = c2;
-            }
-            store_chunk(tile, row, 3 * a + ch, f);
+        for (int k = 0; k < 4; ++k) {
+            f[2 * k] = valid ? s : 0.0f;
+            f[2 * k + 1] = valid ? c : 0.0f;
+            const float s2 = (2.0f * s) * c, c2 = c * c - s * s;
+            s = s2;
+            c = c2;
         }
+        store_chunk(tile, row, 3 * a + ch, f);
     }
+}
+// The three chunks after the bands: directions, albedo, the unit coordinates.
+__device__ __forceinline__ void encode_rest(const float q[12], const float u[3], bool valid, uint8_t *tile, uint32_t row) {
     const float z = 0.0f;
     float f9[8] = {q[3], q[4], q[5], q[6], q[7], q[8], q[9], q[10]};
     float f10[8] = {q[11], u[0], u[1], u[2], z, z, z, z};
@@ -195,6 +195,14 @@ __device__ void encode_row_streamed(const NetDev &net, const float q[12], bool v
     store_chunk(tile, row, 9, f9);
     store_chunk(tile, row, 10, f10);
     store_chunk(tile, row, 11, f11);
+}
+__device__ void encode_row_streamed(const NetDev &net, const float q[12], bool valid, uint8_t *tile, uint32_t row) {
+    float u[3];
+    for (int a = 0; a < 3; ++a) {
+        u[a] = valid ? encode_unit(net, q[a], a) : 0.0f;
+        encode_axis(u[a], valid, tile, row, a);
+    }
+    encode_rest(q, u, valid, tile, row);
 }
 
 // Issue D = A * B for a K-major activation tile A (128 rows) and the K-major
@@ -217,6 +225,15 @@ __device__ __forceinline__ void operand_sync() {
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+}
+
+// The same, and whether v held in every thread.
+__device__ __forceinline__ bool operand_sync_and(bool v) {
+    tc::fence_proxy_async();
+    tc::fence_before_sync();
+    const bool all = __syncthreads_and(v ? 1 : 0) != 0;
+    tc::fence_after_sync();
+    return all;
 }
 
 struct InferIO {
@@ -341,13 +358,14 @@ __global__ void __launch_bounds__(128 * kInferGroups) k_cache_infer(NetDev net, 
 }
 
 // Column sums over a warp's 32 rows: x[k] = the calling lane's value in column
-// k.  A reduce-scatter butterfly (31 shuffles, each round's exchanges
+// k of 16.  A reduce-scatter butterfly (15 shuffles, each round's exchanges
 // independent): after the round of distance h a lane keeps the half of its
-// columns on its side of bit h, plus its partner's values of them; in the end
-// lane c holds the sum of column c.  The order of additions is fixed.
-__device__ __forceinline__ float warp_column_sums32(float x[32], uint32_t lane) {
+// columns on its side of bit h, plus its partner's values of them; the lanes c
+// and c + 16 then hold halves of column c, and both get the sum.  The order of
+// additions is fixed.
+__device__ __forceinline__ float warp_column_sums16(float x[16], uint32_t lane) {
 #pragma unroll
-    for (int h = 16; h >= 1; h >>= 1) {
+    for (int h = 8; h >= 1; h >>= 1) {
         const bool upper = (lane & (uint32_t)h) != 0u;
 #pragma unroll
         for (int k = 0; k < h; ++k) {
@@ -356,7 +374,7 @@ __device__ __forceinline__ float warp_column_sums32(float x[32], uint32_t lane) 
             x[k] = keep + __shfl_xor_sync(0xffffffffu, send, h);
         }
     }
-    return x[0];
+    return x[0] + __shfl_xor_sync(0xffffffffu, x[0], 16);
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -367,7 +385,9 @@ __device__ __forceinline__ float warp_sum(float v) {
 struct TrainIO {
     const float *samples;     // 16 floats per sample: query (12), target (3), weight (0 or 1)
     uint32_t n;
-    float loss_scale;         // 1 / (3 * valid samples)
+    uint32_t n_valid;         // samples of weight > 0, when d_valid is null
+    const uint32_t *d_valid;
+    uint32_t *adam_step;      // the Adam step that follows, advanced here (kept on the device; null: none follows)
     float *partial;           // per CTA: kParams floats (weight and bias gradients)
     float *loss;              // per CTA: sum of the relative L2 terms
 };
@@ -379,11 +399,22 @@ struct TrainIO {
 //                          G's rows padded to 128 with zeros; the sums stay in
 //                          TMEM across the CTA's tiles)
 //   G    <- (G * W_l) .* [H_l > 0]    (tensor cores; W_l read MN-major)
-// Bias gradients are column sums of G: per warp by warp_column_sums32, kept in
-// registers across tiles (lane c: columns c and c + 32 of every layer), and
-// combined over the warps in a fixed order at the end.  The CTA then writes
-// its partial gradients; k_cache_reduce sums them in a fixed order.
-__global__ void __launch_bounds__(128, 1) k_cache_train(NetDev net, TrainIO io, uint32_t *status) {
+// Bias gradients are column sums of G: per warp by warp_column_sums16, kept in
+// registers across tiles, and combined over the warps in a fixed order at the
+// end.  The CTA then writes its partial gradients; k_cache_reduce sums them in
+// a fixed order.
+//
+// A tile is a chain of 12 products with an epilogue each, one after the other,
+// and shared memory holds one tile's layers per SM: the time is the chain's,
+// not the tensor cores'.  So a row's 64 columns are split over four warps
+// (kTrainSplit; warp w: rows 32 (w % 4) .. + 31, the TMEM lanes it can read,
+// columns 16 (w / 4) .. + 15), which cuts every epilogue and the encoding to a
+// quarter.  131,072 samples: 162 us with one thread per row, 125 us split, 109 us
+// with one barrier per product less (the wait's result joins the next barrier's);
+// a tile costs 12.4 us instead of 17.1.
+constexpr uint32_t kTrainSplit = 4, kTrainThreads = kTile * kTrainSplit, kTrainCols = kHid / kTrainSplit;
+static_assert(kTrainCols == 16, "columns of a warp: one TMEM load, one warp_column_sums16");
+__global__ void __launch_bounds__(kTrainThreads, 1) k_cache_train(NetDev net, TrainIO io, uint32_t *status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *x0 = smem + kTrainX0;
     uint8_t *G = smem + kTrainG;
@@ -393,19 +424,22 @@ __global__ void __launch_bounds__(128, 1) k_cache_train(NetDev net, TrainIO io, 
     float *loss_acc = reinterpret_cast<float *>(smem + kTrainMisc + 16);
     const float *bias = reinterpret_cast<const float *>(smem + kSmemBias);
     auto H = [&](int l) { return smem + kTrainH + (uint32_t)(l - 1) * kTileHid; };   // input of layer l >= 1
-    const uint32_t t = threadIdx.x, warp = t >> 5, row = t;
+    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31u, quad = warp & 3u, part_id = warp >> 2;
+    const uint32_t row = quad * 32u + lane, col = part_id * kTrainCols;
     load_net(net, smem);
     for (uint32_t k = t; k < 2 * kTileHid / 16; k += blockDim.x) reinterpret_cast<uint4 *>(G)[k] = make_uint4(0, 0, 0, 0);
     for (uint32_t k = t; k < (uint32_t)kBiasFloats; k += blockDim.x) dbias[k] = 0.0f;
     if (t == 0) *loss_acc = 0.0f;
     if (warp == 0) tc::tmem_alloc(tslot, 512);
     if (t == 0) tc::mbar_init(mbar, 1);
+    if (t == 0 && blockIdx.x == 0 && io.adam_step) *io.adam_step += 1u;
     operand_sync();
     const uint32_t taddr = *tslot;
-    const uint32_t lane_base = (warp * 32u) << 16;
-    const uint32_t lane = t & 31u;
-    float db[kLayers - 1][2];                    // bias-gradient column sums of this warp's rows
-    for (int l = 0; l < kLayers - 1; ++l) db[l][0] = db[l][1] = 0.0f;
+    const uint32_t lane_base = (quad * 32u) << 16;
+    const uint32_t n_valid = io.d_valid ? *io.d_valid : io.n_valid;
+    const float loss_scale = 1.0f / (3.0f * (float)max(n_valid, 1u));
+    float db[kLayers - 1];                       // bias-gradient sums of this warp's rows, column col + lane % 16
+    for (int l = 0; l < kLayers - 1; ++l) db[l] = 0.0f;
     float db_out = 0.0f;                         // output layer: column = lane (lanes < 3)
     float loss_sum = 0.0f;                       // lane 0
     uint32_t phase = 0;
@@ -414,63 +448,71 @@ __global__ void __launch_bounds__(128, 1) k_cache_train(NetDev net, TrainIO io, 
         const uint32_t i = tile * kTile + row;
         const float *s = io.samples + 16 * (size_t)min(i, io.n - 1);
         const float wgt = i < io.n ? s[15] : 0.0f;
-        float q[12];
-        for (int k = 0; k < 12; ++k) q[k] = s[k];
-        const float tg0 = s[12], tg1 = s[13], tg2 = s[14];
-        encode_row_streamed(net, q, wgt > 0.0f, x0, row);
+        float tg[3] = {0.0f, 0.0f, 0.0f};
+        if (part_id == 0)
+            for (int c = 0; c < 3; ++c) tg[c] = s[12 + c];
+        if (part_id < 3u) {
+            encode_axis(wgt > 0.0f ? encode_unit(net, s[part_id], (int)part_id) : 0.0f, wgt > 0.0f, x0, row, (int)part_id);
+        } else {
+            float q[12], u[3];
+            for (int k = 0; k < 12; ++k) q[k] = s[k];
+            for (int a = 0; a < 3; ++a) u[a] = wgt > 0.0f ? encode_unit(net, q[a], a) : 0.0f;
+            encode_rest(q, u, wgt > 0.0f, x0, row);
+        }
         operand_sync();
         // ---- forward
-        for (int l = 0; l < kLayers && ok; ++l) {
+#pragma unroll
+        for (int l = 0; l < kLayers; ++l) {
+            if (!ok) break;
             const uint8_t *in = l == 0 ? x0 : H(l);
             if (t == 0) issue_forward(taddr, in, smem + kSmemImg + img_off(l), l, mbar);
-            ok = __syncthreads_and(tc::mbar_wait(mbar, phase & 1u, kPollLimit) ? 1 : 0) != 0;   // uniform
+            ok = tc::mbar_wait(mbar, phase & 1u, kPollLimit);
             ++phase;
             tc::fence_after_sync();
-            if (!ok) break;
             if (l < kLayers - 1) {
                 uint8_t *out = H(l + 1);
+                float v[16];
+                tc::tmem_ld16(taddr + lane_base + col, v);
 #pragma unroll
-                for (uint32_t c = 0; c < (uint32_t)kHid; c += 32) {
-                    float v[32];
-                    tc::tmem_ld32(taddr + lane_base + c, v);
-#pragma unroll
-                    for (uint32_t k = 0; k < 32; k += 8) {
-                        const float *bb = bias + bias_idx(l) + c + k;
-                        *reinterpret_cast<uint4 *>(out + tc::op_offset(row, c + k, kTile)) = make_uint4(
-                            pack2_relu(v[k] + bb[0], v[k + 1] + bb[1]),
-                            pack2_relu(v[k + 2] + bb[2], v[k + 3] + bb[3]),
-                            pack2_relu(v[k + 4] + bb[4], v[k + 5] + bb[5]),
-                            pack2_relu(v[k + 6] + bb[6], v[k + 7] + bb[7]));
-                    }
+                for (uint32_t k = 0; k < kTrainCols; k += 8) {
+                    const float *bb = bias + bias_idx(l) + col + k;
+                    *reinterpret_cast<uint4 *>(out + tc::op_offset(row, col + k, kTile)) = make_uint4(
+                        pack2_relu(v[k] + bb[0], v[k + 1] + bb[1]),
+                        pack2_relu(v[k + 2] + bb[2], v[k + 3] + bb[3]),
+                        pack2_relu(v[k + 4] + bb[4], v[k + 5] + bb[5]),
+                        pack2_relu(v[k + 6] + bb[6], v[k + 7] + bb[7]));
                 }
-            } else {
+            } else if (part_id == 0) {
                 float v[16];
                 tc::tmem_ld16(taddr + lane_base, v);
                 const float y[3] = {v[0] + bias[bias_idx(l)], v[1] + bias[bias_idx(l) + 1],
                                     v[2] + bias[bias_idx(l) + 2]};
-                const float tg[3] = {tg0, tg1, tg2};
                 float g[3], lsum = 0.0f;
                 for (int c = 0; c < 3; ++c) {
                     const float e = y[c] - tg[c], den = y[c] * y[c] + 0.01f;
                     lsum += wgt * ((e * e) / den);
-                    g[c] = bf16_float(bf16_bits(wgt * (2.0f * e / den) * io.loss_scale));
+                    g[c] = bf16_float(bf16_bits(wgt * (2.0f * e / den) * loss_scale));
                 }
                 lsum = warp_sum(lsum);
                 if (lane == 0) loss_sum += lsum;
                 for (int c = 0; c < 3; ++c) {
-                    const float s = warp_sum(g[c]);
-                    if (lane == (uint32_t)c) db_out += s;
+                    const float gs = warp_sum(g[c]);
+                    if (lane == (uint32_t)c) db_out += gs;
                 }
                 *reinterpret_cast<uint4 *>(G + tc::op_offset(row, 0, kTile)) =
                     make_uint4(pack2(g[0], g[1]), pack2(g[2], 0.0f), 0u, 0u);
-                for (uint32_t c = 8; c < (uint32_t)kHid; c += 8)
+                *reinterpret_cast<uint4 *>(G + tc::op_offset(row, 8, kTile)) = make_uint4(0, 0, 0, 0);
+            } else {
+                for (uint32_t c = col; c < col + kTrainCols; c += 8)
                     *reinterpret_cast<uint4 *>(G + tc::op_offset(row, c, kTile)) = make_uint4(0, 0, 0, 0);
             }
-            operand_sync();
+            ok = operand_sync_and(ok);
         }
         if (!ok) break;
         // ---- backward
-        for (int l = kLayers - 1; l >= 0 && ok; --l) {
+#pragma unroll
+        for (int l = kLayers - 1; l >= 0; --l) {
+            if (!ok) break;
             const uint8_t *in = l == 0 ? x0 : H(l);
             if (t == 0) {
                 // dW_l += G^T * H_l: M = 128 (out rows, zero beyond out_of(l)), N = in_of(l), K = 128 samples
@@ -494,52 +536,41 @@ __global__ void __launch_bounds__(128, 1) k_cache_train(NetDev net, TrainIO io, 
                 }
                 tc::commit(mbar);
             }
-            ok = __syncthreads_and(tc::mbar_wait(mbar, phase & 1u, kPollLimit) ? 1 : 0) != 0;   // uniform
+            ok = tc::mbar_wait(mbar, phase & 1u, kPollLimit);
             ++phase;
             tc::fence_after_sync();
-            if (!ok) break;
             if (l > 0) {
                 const uint8_t *hl = H(l);
+                float v[16], g[16];
+                tc::tmem_ld16(taddr + lane_base + col, v);
+                const uint4 ha = *reinterpret_cast<const uint4 *>(hl + tc::op_offset(row, col, kTile));
+                const uint4 hb = *reinterpret_cast<const uint4 *>(hl + tc::op_offset(row, col + 8, kTile));
+                const uint32_t hw[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
 #pragma unroll
-                for (uint32_t half = 0; half < 2; ++half) {
-                    float g[32];
-#pragma unroll
-                    for (uint32_t q = 0; q < 2; ++q) {
-                        const uint32_t c = half * 32u + q * 16u;
-                        float v[16];
-                        tc::tmem_ld16(taddr + lane_base + c, v);
-                        const uint4 ha = *reinterpret_cast<const uint4 *>(hl + tc::op_offset(row, c, kTile));
-                        const uint4 hb = *reinterpret_cast<const uint4 *>(hl + tc::op_offset(row, c + 8, kTile));
-                        const uint32_t hw[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
-                        float *gq = g + q * 16u;
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const uint32_t hbits = (hw[j >> 1] >> (16 * (j & 1))) & 0xffffu;
-                            gq[j] = bf16_float(bf16_bits(hbits != 0u ? v[j] : 0.0f));   // ReLU output > 0 <=> bits != 0
-                        }
-                        *reinterpret_cast<uint4 *>(G + tc::op_offset(row, c, kTile)) =
-                            make_uint4(pack2(gq[0], gq[1]), pack2(gq[2], gq[3]), pack2(gq[4], gq[5]), pack2(gq[6], gq[7]));
-                        *reinterpret_cast<uint4 *>(G + tc::op_offset(row, c + 8, kTile)) =
-                            make_uint4(pack2(gq[8], gq[9]), pack2(gq[10], gq[11]), pack2(gq[12], gq[13]),
-                                       pack2(gq[14], gq[15]));
-                    }
-                    db[l - 1][half] += warp_column_sums32(g, lane);      // column half * 32 + lane
+                for (int j = 0; j < 16; ++j) {
+                    const uint32_t hbits = (hw[j >> 1] >> (16 * (j & 1))) & 0xffffu;
+                    g[j] = bf16_float(bf16_bits(hbits != 0u ? v[j] : 0.0f));   // ReLU output > 0 <=> bits != 0
                 }
-                operand_sync();
+                *reinterpret_cast<uint4 *>(G + tc::op_offset(row, col, kTile)) =
+                    make_uint4(pack2(g[0], g[1]), pack2(g[2], g[3]), pack2(g[4], g[5]), pack2(g[6], g[7]));
+                *reinterpret_cast<uint4 *>(G + tc::op_offset(row, col + 8, kTile)) =
+                    make_uint4(pack2(g[8], g[9]), pack2(g[10], g[11]), pack2(g[12], g[13]), pack2(g[14], g[15]));
+                ok = operand_sync_and(ok);
+                db[l - 1] += warp_column_sums16(g, lane);             // while the next product runs
+            } else {
+                ok = operand_sync_and(ok);
             }
         }
         first = false;
     }
     if (!ok && t == 0) atomicExch(status, 1u);
-    // the warps' bias-gradient sums and losses, added warp by warp (fixed order)
+    // the warps' bias-gradient sums and losses, added in the order of their rows
     for (uint32_t w = 0; w < 4u; ++w) {
-        if (warp == w) {
-            for (int l = 0; l < kLayers - 1; ++l) {
-                dbias[bias_idx(l) + lane] += db[l][0];
-                dbias[bias_idx(l) + 32u + lane] += db[l][1];
-            }
-            if (lane < 3u) dbias[bias_idx(kLayers - 1) + lane] += db_out;
-            if (lane == 0) *loss_acc += loss_sum;
+        if (quad == w) {
+            if (lane < kTrainCols)
+                for (int l = 0; l < kLayers - 1; ++l) dbias[bias_idx(l) + col + lane] += db[l];
+            if (part_id == 0 && lane < 3u) dbias[bias_idx(kLayers - 1) + lane] += db_out;
+            if (part_id == 0 && lane == 0) *loss_acc += loss_sum;
         }
         __syncthreads();
     }
@@ -550,14 +581,15 @@ __global__ void __launch_bounds__(128, 1) k_cache_train(NetDev net, TrainIO io, 
     float *part = io.partial + (size_t)blockIdx.x * kParams;
     for (int l = 0; l < kLayers; ++l) {
         const uint32_t nin = in_of(l), nout = out_of(l);
-        if (warp * 32u < nout) {                      // TMEM lane = output row
-            const uint32_t o = warp * 32u + (t & 31u);
-            for (uint32_t c = 0; c < nin; c += 16) {
+        if (quad * 32u < nout) {                      // TMEM lane = output row
+            for (uint32_t c = col; c < nin; c += kHid) {
                 float v[16];
                 if (ok && !first) tc::tmem_ld16(taddr + lane_base + kDwCol[l] + c, v);
                 else for (int j = 0; j < 16; ++j) v[j] = 0.0f;
-                if (o < nout)
-                    for (int j = 0; j < 16; ++j) part[w_off(l) + o * nin + c + j] = v[j];
+                if (row < nout)
+                    for (int j = 0; j < 16; j += 4)
+                        *reinterpret_cast<float4 *>(part + w_off(l) + row * nin + c + j) =
+                            make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             }
         }
         for (uint32_t o = t; o < nout; o += blockDim.x) part[b_off(l) + o] = dbias[bias_idx(l) + o];
@@ -571,20 +603,18 @@ __global__ void __launch_bounds__(128, 1) k_cache_train(NetDev net, TrainIO io, 
     }
 }
 
-// grad[p] = sum over CTAs of partial[cta][p], in CTA order.
-__global__ void k_cache_reduce(const float *partial, uint32_t n_cta, const float *loss_part, float *grad,
-                               float *loss_out, uint32_t *adam_step) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < (uint32_t)kParams) {
-        float s = 0.0f;
-        for (uint32_t c = 0; c < n_cta; ++c) s += partial[(size_t)c * kParams + p];
-        grad[p] = s;
-    }
-    if (p == 0) {
-        float s = 0.0f;
-        for (uint32_t c = 0; c < n_cta; ++c) s += loss_part[c];
-        *loss_out = s;
-        if (adam_step) *adam_step += 1u;           // the Adam step that follows (kept on the device)
+// Number of samples of weight > 0, added to *count.
+__global__ void __launch_bounds__(256) k_cache_count(const float *samples, uint32_t n, uint32_t *count) {
+    __shared__ uint32_t sums[8];
+    uint32_t v = 0;
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u)
+        v += samples[16 * (size_t)i + 15] > 0.0f ? 1u : 0u;
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31u) == 0u) sums[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) v += sums[k];
+        if (v) atomicAdd(count, v);
     }
 }
 
@@ -599,27 +629,57 @@ __device__ __forceinline__ void param_where(uint32_t p, int *layer, bool *is_bia
     else { *o = r / in_of(l); *i = r - *o * in_of(l); }
 }
 
-// Adam (Kingma & Ba 2015) on the fp32 parameters; refreshes the bf16 weight
-// image and the bias copy the kernels read.
-__global__ void k_cache_adam(float *params, float *m, float *v, const float *grad, float lr, float beta1, float beta2,
-                             float eps, const uint32_t *adam_step, uint8_t *img, float *bias) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+struct AdamIO {
+    float *params, *m, *v;
+    float lr, beta1, beta2, eps;
+    const uint32_t *step;         // null: gradients only
+    uint8_t *img;
+    float *bias;
+};
+
+// grad[p] = sum over CTAs of partial[cta][p], in CTA order; then, when a step
+// is taken, Adam (Kingma & Ba 2015) on the fp32 parameter, and its place in the
+// bf16 weight image or the bias copy the kernels read.  One thread per
+// parameter; kReduceAhead loads are in flight, as a lone warp's sum is bound by
+// their latency (152 CTAs, 13.6 and 8.4 us as two kernels, 15.7 us together).
+constexpr uint32_t kReduceThreads = 64, kReduceAhead = 16;
+__global__ void __launch_bounds__(kReduceThreads) k_cache_reduce(const float *partial, uint32_t n_cta,
+                                                                 const float *loss_part, float *grad,
+                                                                 float *loss_out, AdamIO A) {
+    const uint32_t p = blockIdx.x * kReduceThreads + threadIdx.x;
+    if (p == 0) {
+        float s = 0.0f;
+#pragma unroll 8
+        for (uint32_t c = 0; c < n_cta; ++c) s += loss_part[c];
+        *loss_out = s;
+    }
     if (p >= (uint32_t)kParams) return;
-    const float t = (float)*adam_step;                 // bias corrections of step t
-    const float bc1 = 1.0f - powf(beta1, t), bc2 = 1.0f - powf(beta2, t);
-    const float g = grad[p];
-    const float mi = beta1 * m[p] + (1.0f - beta1) * g;
-    const float vi = beta2 * v[p] + (1.0f - beta2) * (g * g);
-    m[p] = mi;
-    v[p] = vi;
-    const float w = params[p] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-    params[p] = w;
+    float g = 0.0f;
+    for (uint32_t c0 = 0; c0 < n_cta; c0 += kReduceAhead) {
+        float x[kReduceAhead];
+#pragma unroll
+        for (uint32_t k = 0; k < kReduceAhead; ++k)
+            x[k] = partial[(size_t)min(c0 + k, n_cta - 1u) * kParams + p];
+#pragma unroll
+        for (uint32_t k = 0; k < kReduceAhead; ++k)
+            if (c0 + k < n_cta) g += x[k];
+    }
+    grad[p] = g;
+    if (!A.step) return;
+    const float t = (float)*A.step;                    // bias corrections of step t
+    const float bc1 = 1.0f - powf(A.beta1, t), bc2 = 1.0f - powf(A.beta2, t);
+    const float mi = A.beta1 * A.m[p] + (1.0f - A.beta1) * g;
+    const float vi = A.beta2 * A.v[p] + (1.0f - A.beta2) * (g * g);
+    A.m[p] = mi;
+    A.v[p] = vi;
+    const float w = A.params[p] - A.lr * (mi / bc1) / (sqrtf(vi / bc2) + A.eps);
+    A.params[p] = w;
     int l;
     bool is_bias;
     uint32_t o, i;
     param_where(p, &l, &is_bias, &o, &i);
-    if (is_bias) bias[bias_idx(l) + o] = w;
-    else *reinterpret_cast<uint16_t *>(img + img_off(l) + tc::op_offset(o, i, out_of(l))) = (uint16_t)bf16_bits(w);
+    if (is_bias) A.bias[bias_idx(l) + o] = w;
+    else *reinterpret_cast<uint16_t *>(A.img + img_off(l) + tc::op_offset(o, i, out_of(l))) = (uint16_t)bf16_bits(w);
 }
 
 // Weight image and bias copy from the fp32 parameters (after they are set).
@@ -767,7 +827,7 @@ __global__ void k_cache_synth(uint32_t n, NetDev net, float4 *q, float *samples)
 // ---------------------------------------------------------------------------- cache state
 struct CacheState {
     DBuf params, m, v, img, bias, grad, partial, loss_part, loss, samples, queries, status, batch, judge;
-    DBuf adam_step;               // device Adam step counter (advanced by k_cache_reduce)
+    DBuf adam_step;               // device Adam step counter (advanced by k_cache_train)
     uint32_t n_cta_partial = 0;
     uint32_t passes = 0;          // training passes from recorded paths (the batch draws' seed)
     float lo[3] = {0, 0, 0}, inv_ext[3] = {1, 1, 1};
@@ -895,8 +955,9 @@ cudaError_t cache_infer_host(CacheState *c, const float *q12, uint32_t n, float 
 }
 
 // One optimisation step on n device samples (16 floats each): gradients into
-// c->grad (and the loss into c->loss), then Adam when lr > 0.
-cudaError_t cache_step_device(CacheState *c, const float *d_samples, uint32_t n, uint32_t n_valid, float lr,
+// c->grad (and the loss into c->loss), then Adam when lr > 0.  The samples of
+// weight > 0 are n_valid, or counted on the device when count is set.
+cudaError_t cache_step_device(CacheState *c, const float *d_samples, uint32_t n, uint32_t n_valid, bool count, float lr,
                               cudaStream_t st) {
     cudaError_t e;
     if (!g_train_attr) {
@@ -909,20 +970,21 @@ cudaError_t cache_step_device(CacheState *c, const float *d_samples, uint32_t n,
     const uint32_t blocks = std::max(1u, std::min<uint32_t>(tiles, (uint32_t)sm_count()));
     if ((e = c->partial.ensure((size_t)blocks * kParams * 4)) != cudaSuccess) return e;
     if ((e = c->loss_part.ensure((size_t)blocks * 4)) != cudaSuccess) return e;
-    TrainIO io{d_samples, n, 1.0f / (3.0f * (float)std::max(n_valid, 1u)), c->partial.as<float>(),
-               c->loss_part.as<float>()};
-    k_cache_train<<<blocks, 128, kTrainSmem, st>>>(net_of(c), io, c->status.as<uint32_t>());
-    note_launch();
-    uint32_t *adam_step = lr > 0.0f ? c->adam_step.as<uint32_t>() : nullptr;
-    k_cache_reduce<<<(kParams + 255) / 256, 256, 0, st>>>(c->partial.as<float>(), blocks, c->loss_part.as<float>(),
-                                                          c->grad.as<float>(), c->loss.as<float>(), adam_step);
-    note_launch();
-    if (adam_step) {
-        k_cache_adam<<<(kParams + 255) / 256, 256, 0, st>>>(c->params.as<float>(), c->m.as<float>(), c->v.as<float>(),
-                                                            c->grad.as<float>(), lr, 0.9f, 0.99f, 1e-8f, adam_step,
-                                                            c->img.as<uint8_t>(), c->bias.as<float>());
+    uint32_t *d_valid = count ? c->loss.as<uint32_t>() + 1 : nullptr;
+    if (count) {
+        if ((e = cudaMemsetAsync(d_valid, 0, 4, st)) != cudaSuccess) return e;
+        k_cache_count<<<std::min<uint32_t>((n + 255) / 256, 2u * (uint32_t)sm_count()), 256, 0, st>>>(d_samples, n, d_valid);
         note_launch();
     }
+    uint32_t *adam_step = lr > 0.0f ? c->adam_step.as<uint32_t>() : nullptr;
+    TrainIO io{d_samples, n, n_valid, d_valid, adam_step, c->partial.as<float>(), c->loss_part.as<float>()};
+    k_cache_train<<<blocks, kTrainThreads, kTrainSmem, st>>>(net_of(c), io, c->status.as<uint32_t>());
+    note_launch();
+    AdamIO A{c->params.as<float>(), c->m.as<float>(), c->v.as<float>(), lr, 0.9f, 0.99f, 1e-8f, adam_step,
+             c->img.as<uint8_t>(), c->bias.as<float>()};
+    k_cache_reduce<<<(kParams + kReduceThreads - 1) / kReduceThreads, kReduceThreads, 0, st>>>(
+        c->partial.as<float>(), blocks, c->loss_part.as<float>(), c->grad.as<float>(), c->loss.as<float>(), A);
+    note_launch();
     return cudaGetLastError();
 }
 
@@ -994,7 +1056,7 @@ cudaError_t cache_train_records(CacheState *c, const float4 *rec, uint32_t n_tra
         k_cache_gather<<<(b + 255) / 256, 256, 0, st>>>(c->samples.as<float4>(), count, steps, s, b, seed,
                                                         c->batch.as<float4>());
         note_launch();
-        if ((e = cache_step_device(c, c->batch.as<float>(), b, b, lr, st)) != cudaSuccess) return e;
+        if ((e = cache_step_device(c, c->batch.as<float>(), b, b, false, lr, st)) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
@@ -1045,7 +1107,7 @@ cudaError_t cache_bench(CacheState *c, uint32_t n, uint32_t reps, float *ms_infe
     e = timed([&]() { return cache_infer_device(c, c->queries.as<float4>(), nullptr, n, out, nullptr, nullptr, st); },
               ms_infer);
     if (e == cudaSuccess)
-        e = timed([&]() { return cache_step_device(c, c->samples.as<float>(), n, n, 1e-6f, st); }, ms_train);
+        e = timed([&]() { return cache_step_device(c, c->samples.as<float>(), n, n, false, 1e-6f, st); }, ms_train);
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     return e;
@@ -1063,9 +1125,7 @@ cudaError_t cache_train_host(CacheState *c, const float *samples16, uint32_t n, 
     for (uint32_t s = 0; s < std::max(steps, 1u); ++s) {
         const uint32_t first = (uint32_t)(((uint64_t)s * batch) % n);
         const uint32_t cnt = std::min(batch, n - first);
-        uint32_t valid = 0;
-        for (uint32_t i = first; i < first + cnt; ++i) valid += samples16[16 * (size_t)i + 15] > 0.0f ? 1u : 0u;
-        if ((e = cache_step_device(c, c->samples.as<float>() + 16 * (size_t)first, cnt, valid, steps ? lr : 0.0f,
+        if ((e = cache_step_device(c, c->samples.as<float>() + 16 * (size_t)first, cnt, 0u, true, steps ? lr : 0.0f,
                                    st)) != cudaSuccess)
             return e;
         if (out_loss && (e = cudaMemcpyAsync(out_loss + s, c->loss.p, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
