@@ -707,18 +707,28 @@ mcrt_status mcrt_trace_closest(mcrt_ctx *ctx, const mcrt_ray *rays, uint32_t n, 
     if (!ctx) return fail(nullptr, MCRT_ERR_INVALID_ARG, "ctx is NULL");
     if (!ctx->has_scene) return fail(ctx, MCRT_ERR_NO_SCENE, "no scene uploaded");
     if (n && (!rays || !hits)) return fail(ctx, MCRT_ERR_INVALID_ARG, "rays or hits is NULL");
-    for (uint32_t i = 0; i < n; ++i)
-        if (!(rays[i].tmin > 0.0f)) return fail(ctx, MCRT_ERR_INVALID_ARG, "ray.tmin must be > 0");
     if (n == 0) return MCRT_OK;
+    // tmin is checked by the kernel, which reads every ray anyway; for few rays the host's
+    // look is cheaper than the read-back it saves (4,096 rays: 2 us against 10; 250,000: 230 us)
+    const bool host_check = n <= mcrt::kProbeChecked;
+    if (host_check)
+        for (uint32_t i = 0; i < n; ++i)
+            if (!(rays[i].tmin > 0.0f)) return fail(ctx, MCRT_ERR_INVALID_ARG, "ray.tmin must be > 0");
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     cudaStream_t st = ctx->stream;
     CK(ctx->io_a.ensure((size_t)n * 32), "allocate rays");
-    CK(ctx->io_b.ensure((size_t)n * 16), "allocate hits");
+    CK(ctx->io_b.ensure((size_t)n * 16 + mcrt::kProbeCounters * 4), "allocate hits");
     CK(cudaMemcpyAsync(ctx->io_a.p, rays, (size_t)n * 32, cudaMemcpyHostToDevice, st), "upload rays");
     mcrt::DeviceScene S = device_scene(ctx);
-    mcrt::launch_trace_closest(S, ctx->io_a.as<mcrt_ray>(), n, ctx->io_b.as<mcrt_hit>(),
-                               (flags & MCRT_TRACE_REFERENCE_LAYOUT) != 0, st);
-    CK(cudaGetLastError(), "trace launch");
+    uint32_t *counters = reinterpret_cast<uint32_t *>(ctx->io_b.as<mcrt_hit>() + n);
+    CK(mcrt::launch_trace_closest(S, ctx->io_a.as<mcrt_ray>(), n, ctx->io_b.as<mcrt_hit>(),
+                                  (flags & MCRT_TRACE_REFERENCE_LAYOUT) != 0, counters, st), "trace launch");
+    if (!host_check) {
+        uint32_t bad = 0;
+        CK(cudaMemcpyAsync(&bad, counters + mcrt::kBadRay, 4, cudaMemcpyDeviceToHost, st), "read check");
+        CK(cudaStreamSynchronize(st), "trace");
+        if (bad) return fail(ctx, MCRT_ERR_INVALID_ARG, "ray.tmin must be > 0");
+    }
     CK(cudaMemcpyAsync(hits, ctx->io_b.p, (size_t)n * 16, cudaMemcpyDeviceToHost, st), "read hits");
     CK(cudaStreamSynchronize(st), "trace");
     return MCRT_OK;

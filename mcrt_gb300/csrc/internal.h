@@ -132,8 +132,9 @@ void extend_variant_info(int v, int out[6]);
 void prepare_extend_variants();
 
 // Launchers (render.cu)
-void launch_trace_closest(const DeviceScene &S, const mcrt_ray *rays, uint32_t n, mcrt_hit *hits, bool ref_layout,
-                          cudaStream_t st);
+constexpr uint32_t kBadRay = 0u, kProbeCounters = 8u, kProbeChecked = 4096u;
+cudaError_t launch_trace_closest(const DeviceScene &S, const mcrt_ray *rays, uint32_t n, mcrt_hit *hits, bool ref_layout,
+                                 uint32_t *d_counters, cudaStream_t st);
 // keep_radiance: replay of the same paths (the per-path radiance of the primal
 // pass stays in B.L as the radiance still to be accounted for).
 void launch_raygen(const DeviceScene &S, const RenderParams &P, PathBuffers &B, cudaStream_t st,

@@ -434,13 +434,18 @@ __device__ __forceinline__ float light_pdf_of_hit(const DeviceScene &S, float4 h
 
 // ------------------------------------------------------------------ kernels
 
-__global__ void k_trace_closest(DeviceScene S, const mcrt_ray *rays, uint32_t n, mcrt_hit *hits, int ref_layout) {
+// Caller's rays over the reference's node layout in its visit order (the parity probe).
+__global__ void k_trace_reference(DeviceScene S, const mcrt_ray *rays, uint32_t n, mcrt_hit *hits, uint32_t *counters) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     mcrt_ray ry = rays[i];
+    if (!(ry.tmin > 0.0f)) counters[kBadRay] = 1u;
     RayInv r = make_ray(mk3(ry.org[0], ry.org[1], ry.org[2]), mk3(ry.dir[0], ry.dir[1], ry.dir[2]));
     uint32_t nn = 0;
-    Closest c = world_hit(S, r, ry.tmin, ry.tmax, ref_layout != 0, &nn);
+    Closest c{ry.tmax, MCRT_HIT_MISS, 0u, 0.0f, 0.0f};
+    spheres_hit(S, r, ry.tmin, ry.tmax, c, &nn);
+    mesh_hit_ref(S, r, ry.tmin, c, &nn);
+    if (c.prim == MCRT_HIT_MISS) c.t = -1.0f;
     mcrt_hit h;
     h.t = c.t;
     h.prim = c.prim;
@@ -546,8 +551,8 @@ constexpr ExtendVariant kVariantTable[kExtendVariants] = {
 // kTopBit is an entry of the top tree staged in shared memory (s_top).
 template <int STACK, int TOP>
 __device__ __forceinline__ void visit_compact2(const DeviceScene &S, const float4 *s_top, const RayInv &r,
-                                               float tmax, uint32_t *cur, float *cur_t, uint2 *stack, uint32_t *sp,
-                                               bool *overflow) {
+                                               float tmin, float tmax, uint32_t *cur, float *cur_t, uint2 *stack,
+                                               uint32_t *sp, bool *overflow) {
     float4 a, b, c, e4;
     if (TOP > 0 && (*cur & kTopBit)) {
         const float4 *np = s_top + 4u * (*cur & ~kTopBit);
@@ -559,8 +564,8 @@ __device__ __forceinline__ void visit_compact2(const DeviceScene &S, const float
     }
     const uint2 e = make_uint2(__float_as_uint(e4.x), __float_as_uint(e4.y));
     float tl, tr;
-    bool hl = e.x != kNoChild && slab(r, a.x, a.z, c.x, a.y, a.w, c.y, kTMin, tmax, &tl);
-    bool hr = e.y != kNoChild && slab(r, b.x, b.z, c.z, b.y, b.w, c.w, kTMin, tmax, &tr);
+    bool hl = e.x != kNoChild && slab(r, a.x, a.z, c.x, a.y, a.w, c.y, tmin, tmax, &tl);
+    bool hr = e.y != kNoChild && slab(r, b.x, b.z, c.z, b.y, b.w, c.w, tmin, tmax, &tr);
     if (hl && hr) {
         uint32_t near = e.x, far = e.y;
         float tnear = tl, tfar = tr;
@@ -741,8 +746,12 @@ constexpr uint32_t kOvfClosest = 3u, kOvfAny = 7u;
 // The subtrees taken over are the far ones, which a nearer hit often culls,
 // and the code costs registers: with 5 million rays (voxel world) a launch took
 // 1.57 ms with sharing, 1.49 ms without.
+// A lone ray that is done within kProbeSteps never gets there: single caller's
+// rays take 33 us with it, 37 without.
+constexpr uint32_t kProbeSteps = 24;
 constexpr uint32_t kShareLoad = 8;      // SHARE below this many rays per lane of the grid
-template <int WIDTH, int BLOCK, int STACK, int REFILL, int TOP, bool ANY, bool ADJ, bool COUNT, bool SHARE>
+template <int WIDTH, int BLOCK, int STACK, int REFILL, int TOP, bool ANY, bool ADJ, bool COUNT, bool SHARE,
+          bool PROBE = false>
 __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuffers &B, const AdjointParams &A,
                                             float *gacc, const float4 *s_top, uint32_t n, const float4 *qo,
                                             const float4 *qd) {
@@ -754,9 +763,11 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
     // fewer rays than the grid has lanes: every warp takes its share at once
     const bool spread = SHARE && n < n_warps * 32u;
     const uint32_t share = (n + n_warps - 1u) / n_warps;
+    uint32_t share_after = PROBE ? kProbeSteps : kShareSteps;   // steps to the next look for idle lanes
     uint32_t ray = kNoRay;            // queue index of the lane's ray, or none
     bool exhausted = false;           // the queue has been handed out (warp-uniform)
     RayInv r;
+    float tmin = kTMin;               // PROBE: the ray's own
     Closest best;
     uint2 stack[STACK];
     uint32_t sp = 0, sb = 0;          // entries [sb, sp)
@@ -809,11 +820,19 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             const uint32_t mine = base + __popc(idle_mask & below);
             if (ray == kNoRay && mine < end) {
                 ray = mine;
-                float4 o4 = __ldcs(qo + mine), d4 = __ldcs(qd + mine);   // streamed: evict first
+                float4 o4, d4;
+                if (PROBE) {
+                    ld_pair(qo + 2ull * mine, &o4, &d4);
+                    tmin = o4.w;
+                    if (!(tmin > 0.0f)) B.counters[kBadRay] = 1u;
+                } else {
+                    o4 = __ldcs(qo + mine);                              // streamed: evict first
+                    d4 = __ldcs(qd + mine);
+                }
                 r = make_ray(xyz(o4), xyz(d4));
-                const float tmax = ANY ? d4.w : kTMax;
+                const float tmax = ANY || PROBE ? d4.w : kTMax;
                 best = Closest{tmax, MCRT_HIT_MISS, 0u, 0.0f, 0.0f};
-                spheres_hit(S, r, kTMin, tmax, best, &nn);       // path_trace.wgsl:472-474
+                spheres_hit(S, r, tmin, tmax, best, &nn);       // path_trace.wgsl:472-474
                 drop();
                 if (ANY) {
                     slot = __float_as_uint(o4.w);
@@ -824,7 +843,7 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
                     const float4 *np = reinterpret_cast<const float4 *>(S.mesh_nodes);
                     float4 mn = __ldg(np), mx = __ldg(np + 1);
                     float te;
-                    if (slab(r, mn.x, mn.y, mn.z, mx.x, mx.y, mx.z, kTMin, best.t, &te)) {
+                    if (slab(r, mn.x, mn.y, mn.z, mx.x, mx.y, mx.z, tmin, best.t, &te)) {
                         if (S.n_cnodes == 0) {
                             uint4 meta = __ldg(reinterpret_cast<const uint4 *>(np + 2));
                             cur = leaf_code(meta.x, meta.y);
@@ -839,6 +858,7 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             // ---- no ray is left: idle lanes take over the oldest stack entries (the largest subtrees) of busy ones
             const unsigned offers = __ballot_sync(0xffffffffu, sp > sb);
             const uint32_t pairs = min(__popc(idle_mask), __popc(offers));
+            if (PROBE) share_after = kShareSteps;
             if (pairs) {
                 const bool takes = ray == kNoRay && __popc(idle_mask & below) < pairs;
                 const bool gives = sp > sb && __popc(offers & below) < pairs;
@@ -853,6 +873,7 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
                 auto passu = [&](uint32_t &v) { v = __shfl_sync(0xffffffffu, v, from); };
                 passu(best.prim); passu(best.slot); passu(ray); passu(e.x); passu(e.y);
                 if (ANY) passu(slot);
+                if (PROBE) pass(tmin);
                 if (takes) {
                     drop();
                     occl = false;
@@ -868,12 +889,12 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             const unsigned going = __ballot_sync(0xffffffffu, go);
             if (going == 0) break;
             if (__popc(going) < kKeepWalking && __any_sync(0xffffffffu, leaf != kNoChild)) break;
-            if (SHARE && exhausted && idle_mask && step >= kShareSteps) break;
+            if (SHARE && exhausted && idle_mask && step >= share_after) break;
             if (go) {
                 ++nn;
                 bool full = false;
                 if (WIDTH == 4) visit_wide4<STACK>(S, r, best.t, &cur, &cur_t, stack, &sp, &full);
-                else visit_compact2<STACK, TOP>(S, s_top, r, best.t, &cur, &cur_t, stack, &sp, &full);
+                else visit_compact2<STACK, TOP>(S, s_top, r, tmin, best.t, &cur, &cur_t, stack, &sp, &full);
                 if (full) {                                      // to the overflow list
                     ray |= kOvfBit;
                     drop();
@@ -893,7 +914,7 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             } else {
                 const uint32_t cnt = leaf_count(S, leaf);
                 if (COUNT) ntri += cnt;
-                leaf_tris(S, r, (leaf & ~kLeafBit) >> 4, cnt, kTMin, best);
+                leaf_tris(S, r, (leaf & ~kLeafBit) >> 4, cnt, tmin, best);
             }
             leaf = kNoChild;
             if (cur != kNoChild && (cur & kLeafBit) && cur_t <= cull_t(best.t)) {
@@ -942,7 +963,13 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
                 }
             }
         }
-        if (done) {
+        if (done && PROBE) {
+            // too deep for the stack: the stackless walk, from the closest hit so far
+            if (ray & kOvfBit) mesh_walk_stackless<false>(S, r, tmin, best, &nn);
+            if (best.prim == MCRT_HIT_MISS) best.t = -1.0f;
+            __stcs(B.hits + (ray & ~kOvfBit), make_float4(best.t, __uint_as_float(best.prim), best.u, best.v));
+            ray = kNoRay;
+        } else if (done) {
             if (ray & kOvfBit) {
                 B.ovf[atomicAdd(B.counters + (ANY ? kOvfAny : kOvfClosest), 1u)] = ray & ~kOvfBit;
             } else {
@@ -952,7 +979,7 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             ray = kNoRay;
         }
     }
-    if (traced) atomicAdd(B.stats + (ANY ? 1 : 0), (unsigned long long)traced);
+    if (!PROBE && traced) atomicAdd(B.stats + (ANY ? 1 : 0), (unsigned long long)traced);
     if (COUNT) {
         atomicAdd(B.stats + 3, (unsigned long long)nn);
         atomicAdd(B.stats + 4, (unsigned long long)ntri);
@@ -1003,6 +1030,30 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_extend(DeviceScene S, PathBuffe
             if (v != 0.0f) atomicAdd(A.grad + k, (double)v);
         }
     }
+}
+
+// Closest hits of the caller's rays (32 bytes each: origin, tmin, direction,
+// tmax) by the queue walk of the render.  hits in ray order.  counters: the
+// queue's next entry and kBadRay, both zero before the launch.
+// Bound by the L2 round trips of a ray's steps and, at the end, of the longest
+// rays: a thread per ray with a stack of 64 entries, as it was, kept a warp until
+// its longest ray was done.  Calls of 1,000 / 250,000 / 1,000,000 rays into an
+// 80,000-triangle mesh: 294 / 1161 / 3963 us then, 70 / 346 / 1072 us now.
+// Blocks of 64 threads, 12 to an SM with 24 stack entries: 346 us; 18 with 32:
+// 357; 8 of 128 with 64: 357.
+constexpr int kProbeBlock = 64, kProbeBlocks = 12, kProbeStack = 24, kProbeRefill = 8;
+__global__ void __launch_bounds__(kProbeBlock, kProbeBlocks) k_trace_rays(DeviceScene S, const float4 *rays, uint32_t n,
+                                                                          float4 *hits, uint32_t *counters) {
+    PathBuffers B{};
+    B.counters = counters;
+    B.hits = hits;
+    const AdjointParams A{};
+    if (n < kShareLoad * (gridDim.x * kProbeBlock))
+        trace_queue<2, kProbeBlock, kProbeStack, kProbeRefill, 0, false, false, false, true, true>(
+            S, B, A, nullptr, nullptr, n, rays, nullptr);
+    else
+        trace_queue<2, kProbeBlock, kProbeStack, kProbeRefill, 0, false, false, false, false, true>(
+            S, B, A, nullptr, nullptr, n, rays, nullptr);
 }
 
 // The overflow list of the preceding closest-hit (ANY = false) or any-hit
@@ -2059,10 +2110,37 @@ int sm_count() {
     return n;
 }
 
-void launch_trace_closest(const DeviceScene &S, const mcrt_ray *rays, uint32_t n, mcrt_hit *hits, bool ref_layout,
-                          cudaStream_t st) {
-    if (n == 0) return;
-    k_trace_closest<<<(n + 127) / 128, 128, 0, st>>>(S, rays, n, hits, ref_layout ? 1 : 0); ::mcrt::note_launch();
+// d_counters: kProbeCounters words; above kProbeChecked rays, word kBadRay tells
+// afterwards whether some ray's tmin is not positive.  Chunks of 2^30 rays keep the queue's entries
+// below kOvfBit.
+cudaError_t launch_trace_closest(const DeviceScene &S, const mcrt_ray *rays, uint32_t n, mcrt_hit *hits, bool ref_layout,
+                                 uint32_t *d_counters, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    static const int per_sm = [] {
+        int v = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_trace_rays, kProbeBlock, 0);
+        return v > 0 ? v : 1;
+    }();
+    const uint32_t grid = (uint32_t)(per_sm * sm_count());
+    // few rays: the caller has checked them, and a queue that is spread over the warps needs no counter
+    // (a clear costs 2.5 of a single ray's 33 us)
+    const bool clear = n > kProbeChecked || n >= grid * kProbeBlock;
+    cudaError_t e;
+    if (clear && (e = cudaMemsetAsync(d_counters, 0, kProbeCounters * 4, st)) != cudaSuccess) return e;
+    if (ref_layout) {
+        k_trace_reference<<<(n + 127) / 128, 128, 0, st>>>(S, rays, n, hits, d_counters); ::mcrt::note_launch();
+        return cudaGetLastError();
+    }
+    for (uint64_t first = 0; first < n; first += 1u << 30) {
+        const uint32_t m = (uint32_t)std::min<uint64_t>(n - first, 1u << 30);
+        if (first && (e = cudaMemsetAsync(d_counters + 4, 0, 4, st)) != cudaSuccess) return e;
+        // a warp per ray at most
+        const uint32_t blocks = std::min(grid, (m + kProbeBlock / 32 - 1) / (kProbeBlock / 32));
+        k_trace_rays<<<blocks, kProbeBlock, 0, st>>>(S, reinterpret_cast<const float4 *>(rays + first), m,
+                                                     reinterpret_cast<float4 *>(hits + first), d_counters);
+        ::mcrt::note_launch();
+    }
+    return cudaGetLastError();
 }
 
 void launch_raygen(const DeviceScene &S, const RenderParams &P, PathBuffers &B, cudaStream_t st, bool keep_radiance) {

@@ -235,10 +235,8 @@ __device__ __forceinline__ void mesh_hit_ref(const DeviceScene &S, const RayInv 
     }
 }
 
-// Any hit in (tmin, tmax) with the same visibility rules (backface-culled
-// triangles are invisible from behind); used by shadow rays.
-// Any triangle of a leaf that mesh_hit_fast would accept as a hit before its
-// first one: tri_test passes, t < tmax, not culled by the backface flag.
+// Any triangle of a leaf that leaf_tris would accept as a ray's first hit
+// (shadow rays; the same visibility rules): tri_test passes, t < tmax, not culled by the backface flag.
 __device__ __forceinline__ bool leaf_any(const DeviceScene &S, const RayInv &r, uint32_t first, uint32_t count,
                                          float tmin, float tmax) {
     for (uint32_t j = 0; j < count; ++j) {
@@ -346,158 +344,6 @@ __device__ __noinline__ bool mesh_walk_stackless(const DeviceScene &S, const Ray
         from = node;
         node = up;
     }
-}
-
-// Compact layout: node k = {Lx, Ly | Rx, Ry | Lz, Rz | codeL, codeR, parent, 0}.
-// A ray that would overflow the stack is finished by the stackless walk from
-// its current closest hit (which only tightens the cull).
-__device__ __forceinline__ void mesh_hit_fast(const DeviceScene &S, const RayInv &r, float tmin, Closest &best,
-                                              uint32_t *n_nodes) {
-    if (S.n_mesh_nodes == 0) return;
-    if (S.n_cnodes == 0) {                       // the whole tree is one leaf
-        const float4 *np = reinterpret_cast<const float4 *>(S.mesh_nodes);
-        float4 mn = __ldg(np), mx = __ldg(np + 1);
-        uint4 meta = __ldg(reinterpret_cast<const uint4 *>(np + 2));
-        float te;
-        if (slab(r, mn.x, mn.y, mn.z, mx.x, mx.y, mx.z, tmin, best.t, &te)) leaf_tris(S, r, meta.x, meta.y, tmin, best);
-        return;
-    }
-    // the root box itself (reference node 0) is tested first, as the reference does
-    {
-        const float4 *np = reinterpret_cast<const float4 *>(S.mesh_nodes);
-        float4 mn = __ldg(np), mx = __ldg(np + 1);
-        float te;
-        if (!slab(r, mn.x, mn.y, mn.z, mx.x, mx.y, mx.z, tmin, best.t, &te)) return;
-    }
-    uint2 stack[kStackSize];
-    uint32_t sp = 0;
-    uint32_t node = 0;
-    for (;;) {
-        const float4 *np = S.cnodes + 4ull * node;
-        float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-        uint4 e = __ldg(reinterpret_cast<const uint4 *>(np + 3));
-        ++*n_nodes;
-        float tl, tr;
-        bool hl = e.x != kNoChild && slab(r, a.x, a.z, c.x, a.y, a.w, c.y, tmin, best.t, &tl);
-        bool hr = e.y != kNoChild && slab(r, b.x, b.z, c.z, b.y, b.w, c.w, tmin, best.t, &tr);
-        uint32_t next = kNoChild;
-        if (hl && hr) {
-            uint32_t near = e.x, far = e.y;
-            float tfar = tr;
-            if (tr < tl) { near = e.y; far = e.x; tfar = tl; }
-            if (sp == kStackSize) {
-                mesh_walk_stackless<false>(S, r, tmin, best, n_nodes);
-                return;
-            }
-            stack[sp++] = make_uint2(far, __float_as_uint(tfar));
-            next = near;
-        } else if (hl) {
-            next = e.x;
-        } else if (hr) {
-            next = e.y;
-        }
-        // descend through leaves and popped entries until an internal node is found
-        for (;;) {
-            if (next == kNoChild) {
-                // pop, skipping entries that start beyond the current closest hit
-                next = kNoChild;
-                while (sp > 0) {
-                    uint2 s = stack[--sp];
-                    if (__uint_as_float(s.y) <= cull_t(best.t)) { next = s.x; break; }
-                }
-                if (next == kNoChild) return;
-            }
-            if (next & kLeafBit) {
-                uint32_t first = (next & ~kLeafBit) >> 4;
-                leaf_tris(S, r, first, leaf_count(S, next), tmin, best);
-                next = kNoChild;
-                continue;
-            }
-            break;
-        }
-        node = next;
-    }
-}
-
-// world_hit, path_trace.wgsl:471-479: spheres first, then the mesh with t_max =
-// the sphere distance; the mesh wins only when strictly closer.
-__device__ __forceinline__ Closest world_hit(const DeviceScene &S, const RayInv &r, float tmin, float tmax,
-                                             bool ref_layout, uint32_t *n_nodes) {
-    Closest best{tmax, MCRT_HIT_MISS, 0u, 0.0f, 0.0f};
-    spheres_hit(S, r, tmin, tmax, best, n_nodes);
-    if (ref_layout) mesh_hit_ref(S, r, tmin, best, n_nodes);
-    else mesh_hit_fast(S, r, tmin, best, n_nodes);
-    if (best.prim == MCRT_HIT_MISS) best.t = -1.0f;
-    return best;
-}
-
-// Is there a mesh hit in [tmin, tmax)?  mesh_hit_fast's traversal (same
-// order, same cull against tmax) up to its first accepted hit, which alone
-// decides whether it finds one, so the answer is the same; it stops there.
-__device__ __forceinline__ bool mesh_any_hit(const DeviceScene &S, const RayInv &r, float tmin, float tmax) {
-    if (S.n_mesh_nodes == 0) return false;
-    const float4 *root = reinterpret_cast<const float4 *>(S.mesh_nodes);
-    {
-        float4 mn = __ldg(root), mx = __ldg(root + 1);
-        float te;
-        if (!slab(r, mn.x, mn.y, mn.z, mx.x, mx.y, mx.z, tmin, tmax, &te)) return false;
-    }
-    if (S.n_cnodes == 0) {                       // the whole tree is one leaf
-        uint4 meta = __ldg(reinterpret_cast<const uint4 *>(root + 2));
-        return leaf_any(S, r, meta.x, meta.y, tmin, tmax);
-    }
-    uint2 stack[kStackSize];
-    uint32_t sp = 0;
-    uint32_t node = 0;
-    for (;;) {
-        const float4 *np = S.cnodes + 4ull * node;
-        float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-        uint4 e = __ldg(reinterpret_cast<const uint4 *>(np + 3));
-        float tl, tr;
-        bool hl = e.x != kNoChild && slab(r, a.x, a.z, c.x, a.y, a.w, c.y, tmin, tmax, &tl);
-        bool hr = e.y != kNoChild && slab(r, b.x, b.z, c.z, b.y, b.w, c.w, tmin, tmax, &tr);
-        uint32_t next = kNoChild;
-        if (hl && hr) {
-            uint32_t near = e.x, far = e.y;
-            float tfar = tr;
-            if (tr < tl) { near = e.y; far = e.x; tfar = tl; }
-            if (sp == kStackSize) {                // too deep for the stack: walk without one
-                uint32_t nn = 0;
-                Closest b{tmax, MCRT_HIT_MISS, 0u, 0.0f, 0.0f};
-                return mesh_walk_stackless<true>(S, r, tmin, b, &nn);
-            }
-            stack[sp++] = make_uint2(far, __float_as_uint(tfar));
-            next = near;
-        } else if (hl) {
-            next = e.x;
-        } else if (hr) {
-            next = e.y;
-        }
-        for (;;) {
-            if (next == kNoChild) {
-                while (sp > 0) {
-                    uint2 s = stack[--sp];
-                    if (__uint_as_float(s.y) <= cull_t(tmax)) { next = s.x; break; }
-                }
-                if (next == kNoChild) return false;
-            }
-            if (next & kLeafBit) {
-                if (leaf_any(S, r, (next & ~kLeafBit) >> 4, leaf_count(S, next), tmin, tmax)) return true;
-                next = kNoChild;
-                continue;
-            }
-            break;
-        }
-        node = next;
-    }
-}
-
-__device__ __forceinline__ bool occluded(const DeviceScene &S, const RayInv &r, float tmin, float tmax) {
-    uint32_t nn = 0;
-    Closest best{tmax, MCRT_HIT_MISS, 0u, 0.0f, 0.0f};
-    spheres_hit(S, r, tmin, tmax, best, &nn);
-    if (best.prim != MCRT_HIT_MISS) return true;
-    return mesh_any_hit(S, r, tmin, tmax);
 }
 
 }  // namespace mcrt

@@ -1,0 +1,57 @@
+"""Closest hits of the caller's rays: sizes around the limits of the queue walk, own tmin and tmax per ray."""
+import numpy as np
+import pytest
+
+import mcrt_gb300 as M
+from test_gpu_parity import bits, random_scene_rays
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def scene(oracle):
+    rng = np.random.default_rng(11)
+    spheres = np.zeros(60, M.SPHERE)
+    spheres["center_r"][:, :3] = rng.uniform(-3, 3, (60, 3))
+    spheres["center_r"][:, 3] = rng.uniform(0.05, 0.4, 60)
+    n = 3000
+    v = np.zeros(3 * n, M.VERTEX)
+    v["position"][:, :3] = (rng.uniform(-3, 3, (n, 1, 3)) + rng.uniform(-0.2, 0.2, (n, 3, 3))).reshape(-1, 3)
+    v["position"][:, 3] = 1
+    v["normal"][:, 1] = 1
+    t = np.zeros(n, M.TRIANGLE)
+    t["v"] = np.arange(3 * n).reshape(n, 3)
+    md = M.materials([(0, (0.5, 0.5, 0.5), 0, 1)])
+    ctx = M.Context(0)
+    ctx.upload_scene(spheres=spheres, vertices=v, triangles=t, materials=md)
+    yield ctx, oracle.OracleScene(materials=md, spheres=spheres, vertices=v, triangles=t)
+    ctx.close()
+
+
+# a ray per warp, the host's and the kernel's check of tmin (4,096), a queue that fills the grid
+# and one of more than eight rays per lane (152 SMs x 12 blocks x 64 lanes)
+@pytest.mark.parametrize("n", [1, 2, 33, 4096, 4097, 150001, 8 * 152 * 12 * 64 + 5])
+def test_trace_sizes_and_ranges(scene, n):
+    ctx, osc = scene
+    rng = np.random.default_rng(n)
+    rays = random_scene_rays(rng, max(n, 64))[:n]
+    rays["tmin"] = rng.choice([1e-3, 0.5, 2.0], n)
+    rays["tmax"] = rng.choice([0.7, 3.0, 1e9, np.inf], n)
+    got, want = ctx.trace_closest(rays), osc.trace(rays)
+    assert np.array_equal(got["prim"], want["prim"])
+    assert np.array_equal(bits(got["t"]), bits(want["t"]))
+    tri = got["prim"] < 3000
+    for f in ("u", "v"):
+        assert np.array_equal(bits(got[f][tri]), bits(want[f][tri]))
+
+
+@pytest.mark.parametrize("n", [5, 4096, 4097, 20000])
+@pytest.mark.parametrize("bad", [0.0, -1.0, np.nan])
+def test_trace_refuses_a_ray_without_positive_tmin(scene, n, bad):
+    ctx, osc = scene
+    rays = random_scene_rays(np.random.default_rng(n), max(n, 64))[:n]
+    rays["tmin"][n - 2] = bad
+    with pytest.raises(M.MCRTError):
+        ctx.trace_closest(rays)
+    rays["tmin"][n - 2] = 1e-3
+    assert np.array_equal(ctx.trace_closest(rays)["prim"], osc.trace(rays)["prim"])
