@@ -1,12 +1,16 @@
 // api.cu — the extern "C" entry points of libmcrt_cuda.so (include/mcrt_cuda.h):
 // context, scene upload (with host-side validation of every index the kernels
 // will dereference), closest-hit probe, render driver, denoiser.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "common.cuh"
@@ -33,6 +37,69 @@ cudaError_t gpu_build_sphere_bvh(const mcrt_gpu_sphere *d_spheres, uint32_t n, m
 }  // namespace mcrt
 
 namespace {
+
+// Pages for a read-back mesh before the copies into it.  A buffer that nothing
+// has written yet has none, and the copy takes a fault per page, one after the
+// other: 16 MB took 700 us, with its pages there 100.  The kernel fills a whole
+// range in one call (MADV_POPULATE_WRITE: the contents stay as they are; where
+// it is missing or the memory is of another kind, the call fails and the copy
+// faults as before), at 33 GB/s a thread, so a few threads share it.  A buffer
+// whose first, middle and last page are there is left alone, and so are meshes
+// below 8 MB, which mostly come from memory that the caller's allocator has had
+// before (images and ray hits do too: no gain there).  The 29 MB mesh of a
+// 128^3 terrain region is meshed and read in 2.2 ms, 3.5 without.
+struct OutBuf { void *p; size_t bytes; };
+void ready_pages(std::initializer_list<OutBuf> list) noexcept {
+#ifdef __linux__
+    constexpr int kPopulateWrite = 23;                       // MADV_POPULATE_WRITE, Linux 5.14
+    constexpr size_t kPiece = 2u << 20, kSmall = 8u << 20;
+    constexpr int kMaxBufs = 4, kMaxThreads = 4;
+    struct Span { uintptr_t first, end; } spans[kMaxBufs];
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    int n_spans = 0;
+    size_t pieces = 0, total = 0;
+    for (const OutBuf &b : list) total += b.p ? b.bytes : 0;
+    if (total < kSmall) return;
+    for (const OutBuf &b : list) {
+        if (!b.p || b.bytes == 0 || n_spans == kMaxBufs) continue;
+        const uintptr_t a = reinterpret_cast<uintptr_t>(b.p);
+        const Span sp{a & ~(page - 1), (a + b.bytes + page - 1) & ~(page - 1)};
+        bool there = true;
+        for (uintptr_t at : {sp.first, (sp.first + (sp.end - sp.first) / 2) & ~(page - 1), sp.end - page}) {
+            unsigned char in = 1;
+            if (mincore(reinterpret_cast<void *>(at), page, &in) == 0 && !(in & 1)) there = false;
+        }
+        if (there) continue;
+        spans[n_spans++] = sp;
+        pieces += (sp.end - sp.first + kPiece - 1) / kPiece;
+    }
+    if (pieces == 0) return;
+    std::atomic<size_t> next{0};
+    auto fill = [&]() {
+        for (size_t k; (k = next.fetch_add(1)) < pieces;) {
+            int i = 0;
+            size_t of = k;
+            while (of >= (spans[i].end - spans[i].first + kPiece - 1) / kPiece)
+                of -= (spans[i].end - spans[i].first + kPiece - 1) / kPiece, ++i;
+            const uintptr_t at = spans[i].first + of * kPiece;
+            madvise(reinterpret_cast<void *>(at), std::min<size_t>(kPiece, spans[i].end - at), kPopulateWrite);
+        }
+    };
+    std::thread more[kMaxThreads - 1];
+    for (size_t k = 0; k < kMaxThreads - 1 && 2 * (k + 1) < pieces; ++k) {
+        try {
+            more[k] = std::thread(fill);
+        } catch (...) {                                      // no thread to be had: the caller's fills it all
+            break;
+        }
+    }
+    fill();
+    for (std::thread &t : more)
+        if (t.joinable()) t.join();
+#else
+    (void)list;
+#endif
+}
 
 thread_local std::string g_error;   // errors of calls without a context
 
@@ -1302,6 +1369,7 @@ mcrt_status mcrt_world_read_mesh(mcrt_ctx *ctx, mcrt_gpu_vertex *vertices, uint3
     if ((vertices && vertex_capacity < nv) || (triangles && triangle_capacity < nt))
         return fail(ctx, MCRT_ERR_INVALID_ARG, "capacity too small");
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
+    ready_pages({{vertices, (size_t)nv * sizeof(mcrt_gpu_vertex)}, {triangles, (size_t)nt * sizeof(mcrt_gpu_triangle)}});
     if (vertices && nv)
         CK(cudaMemcpy(vertices, ctx->wmesh.vertices.p, (size_t)nv * sizeof(mcrt_gpu_vertex), cudaMemcpyDeviceToHost),
            "read vertices");
@@ -1432,6 +1500,7 @@ mcrt_status mcrt_mesh_read(mcrt_ctx *ctx, mcrt_gpu_vertex *vertices, uint32_t ve
     if ((vertices && vertex_capacity < nv) || (triangles && triangle_capacity < nt))
         return fail(ctx, MCRT_ERR_INVALID_ARG, "capacity too small");
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
+    ready_pages({{vertices, (size_t)nv * 48}, {triangles, (size_t)nt * 16}});
     if (vertices && nv)
         CK(cudaMemcpy(vertices, ctx->dmesh.vertices.p, (size_t)nv * 48, cudaMemcpyDeviceToHost), "read vertices");
     if (triangles && nt)
