@@ -749,7 +749,14 @@ constexpr uint32_t kOvfClosest = 3u, kOvfAny = 7u;
 // A lone ray that is done within kProbeSteps never gets there: single caller's
 // rays take 33 us with it, 37 without.
 constexpr uint32_t kProbeSteps = 24;
-constexpr uint32_t kShareLoad = 8;      // SHARE below this many rays per lane of the grid
+// SHARE below this many rays per lane of the grid: one for the render's queues,
+// more for the caller's rays (250,000 into an 80,000-triangle mesh: 350 us with
+// the limit at eight, 393 at one).  With eight in the render a frame of 1.3M
+// small triangles gains (24.4 instead of 25.5 ms), but voxel worlds, whose rays
+// are soon done, lose: 309,000 paths 1.30 ms instead of 1.23, eight views 7.80
+// instead of 7.73.  (Part of it is register allocation: with the limit hidden from
+// the compiler the frame takes 24.7 and the 309,000 paths 1.27 ms.)
+constexpr uint32_t kShareLoad = 1, kProbeShareLoad = 8;
 template <int WIDTH, int BLOCK, int STACK, int REFILL, int TOP, bool ANY, bool ADJ, bool COUNT, bool SHARE,
           bool PROBE = false>
 __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuffers &B, const AdjointParams &A,
@@ -1048,7 +1055,7 @@ __global__ void __launch_bounds__(kProbeBlock, kProbeBlocks) k_trace_rays(Device
     B.counters = counters;
     B.hits = hits;
     const AdjointParams A{};
-    if (n < kShareLoad * (gridDim.x * kProbeBlock))
+    if (n < kProbeShareLoad * (gridDim.x * kProbeBlock))
         trace_queue<2, kProbeBlock, kProbeStack, kProbeRefill, 0, false, false, false, true, true>(
             S, B, A, nullptr, nullptr, n, rays, nullptr);
     else
@@ -1263,8 +1270,9 @@ __device__ __forceinline__ void record_end(const RenderParams &P, uint32_t slot,
 struct ShadedVertex {
     bool cont = false, shadow = false, queried = false;   // the path goes on; a shadow ray; a cache query
     bool scattered = false, vertex = false;               // the throughput changed; a non-emissive surface was hit
-    f3 no, nd;                                            // continuing ray
-    f3 so, sd, sc;                                        // shadow ray and its contribution
+    f3 p;                                                 // the vertex: origin of both rays
+    f3 nd;                                                // direction of the continuing ray
+    f3 sd, sc;                                            // shadow ray's direction and contribution
     float smax;
     uint32_t rng = 0;                                     // random state: in, of the arriving ray; out, of the next
     float4 cq[4];                                         // radiance-cache query
@@ -1283,7 +1291,7 @@ __device__ __forceinline__ float4 pending_gradient(f3 delta, float4 L, float4 pe
 
 // One vertex of path `slot`: the hit h of its ray (o, d).  get_L / set_L hold
 // the path's radiance; thr4 is its throughput and the last BSDF pdf.
-template <bool ADJ, class GetL, class SetL, class GAdd>
+template <bool ADJ, bool CACHE, class GetL, class SetL, class GAdd>
 __device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderParams &P, f3 o, f3 d, float4 h,
                                              uint32_t slot, uint32_t pixel, uint32_t bounce, bool nee, float4 *gbuf,
                                              f3 delta, float4 &thr4, ShadedVertex &v, GetL get_L, SetL set_L,
@@ -1295,7 +1303,7 @@ __device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderP
         if (write_g) gbuf[pixel] = make_float4(0.0f, 0.0f, 0.0f, kTMax);
         if (!ADJ) {
             f3 e = thr * sample_env(S, d);
-            if (P.cache_query_vertex && slot % P.train_stride == 0u)   // training path ends here
+            if (CACHE && slot % P.train_stride == 0u)               // training path ends here
                 record_end(P, slot, bounce, get_L());
             float4 L = get_L();
             if (nee) set_L(make_float4(L.x + e.x, L.y + e.y, L.z + e.z, 0.0f));
@@ -1322,7 +1330,7 @@ __device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderP
                 f3 g = (wmis * m.ior_pad[0]) * (delta * thr);
                 gadd(mi, make_float4(g.x, g.y, g.z, 0.0f));
             } else {
-                if (P.cache_query_vertex && slot % P.train_stride == 0u)   // training path ends here
+                if (CACHE && slot % P.train_stride == 0u)               // training path ends here
                     record_end(P, slot, bounce, get_L());
                 if (nee) {
                     float4 L = get_L();
@@ -1339,7 +1347,7 @@ __device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderP
             float pdf = -1.0f;
             float4 dlw = make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // adjoint: dlog(weight)/d(params)
             bool has_params = false;
-            if (!ADJ && P.cache_query_vertex) {                         // radiance cache
+            if (CACHE) {                                                // radiance cache
                 if (slot % P.train_stride == 0u) {                      // training path: record the vertex
                     float4 *rec = P.train_records +
                                   ((size_t)(slot / P.train_stride) * P.max_depth + bounce) * kTrainRecordFloat4;
@@ -1415,7 +1423,7 @@ __device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderP
                             if (wl.z > 0.0f && (fc.x > 0.0f || fc.y > 0.0f || fc.z > 0.0f)) {
                                 float wmis = ls.delta ? 1.0f : (ls.pdf * ls.pdf) / (ls.pdf * ls.pdf + bp * bp);
                                 v.sc = (wmis / ls.pdf) * (thr * (fc * ls.Le));
-                                v.so = sh.p; v.sd = ls.dir; v.smax = ls.dist * (1.0f - 1e-4f);
+                                v.sd = ls.dir; v.smax = ls.dist * (1.0f - 1e-4f);
                                 v.shadow = true;
                                 if (ADJ) {
                                     const f3 one = mk3(1.0f, 1.0f, 1.0f);
@@ -1440,7 +1448,7 @@ __device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderP
                         float bp = cs / kPi;
                         float wmis = ls.delta ? 1.0f : (ls.pdf * ls.pdf) / (ls.pdf * ls.pdf + bp * bp);
                         v.sc = (wmis * bp / ls.pdf) * (thr * (albedo * ls.Le));
-                        v.so = sh.p; v.sd = ls.dir; v.smax = ls.dist * (1.0f - 1e-4f);
+                        v.sd = ls.dir; v.smax = ls.dist * (1.0f - 1e-4f);
                         v.shadow = true;
                         if (ADJ) {
                             v.sh_dlog = make_float4(safe_ratio(tex.x, albedo.x), safe_ratio(tex.y, albedo.y),
@@ -1465,7 +1473,6 @@ __device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderP
                 thr = thr * atten;
                 if (bounce + 1 < P.max_depth) {
                     v.cont = true;
-                    v.no = sh.p;
                     v.nd = dir;
                     if (ADJ && has_params) {
                         v.pend = dlw;
@@ -1476,12 +1483,17 @@ __device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderP
                 v.scattered = true;
             }
             v.vertex = true;
+            v.p = sh.p;
         }
     }
 }
 
-template <bool ADJ>
-__global__ void __launch_bounds__(256, ADJ ? 2 : 4) k_shade(DeviceScene S, RenderParams P, PathBuffers B, int qi,
+// CACHE: a render with the radiance cache, whose records and queries are code and
+// 16 registers that the others do without.  Bound by its scattered loads; three
+// blocks of 256 to an SM keep it out of local memory: 1.02 ms for the 18.7M hits of a
+// voxel world frame, four 1.13, two 1.18 (four with the cache's code inside: 1.21).
+template <bool ADJ, bool CACHE>
+__global__ void __launch_bounds__(256, ADJ ? 2 : 3) k_shade(DeviceScene S, RenderParams P, PathBuffers B, int qi,
                                                 uint32_t bounce, float4 *gbuf, AdjointParams A) {
     __shared__ float gacc[ADJ ? 256 : 1];
     if (ADJ) {
@@ -1514,7 +1526,7 @@ __global__ void __launch_bounds__(256, ADJ ? 2 : 4) k_shade(DeviceScene S, Rende
                 const uint32_t pm = (B.pend_mat[slot] >> 8) & 0xffu;
                 if (pm) block_gadd(gacc, pm - 1u, pending_gradient(delta, B.L[slot], B.pend[slot]));
             }
-            shade_vertex<ADJ>(S, P, xyz(o4), xyz(d4), h, slot, pixel, bounce, nee, gbuf, delta, thr4, v,
+            shade_vertex<ADJ, CACHE>(S, P, xyz(o4), xyz(d4), h, slot, pixel, bounce, nee, gbuf, delta, thr4, v,
                               [&]() { return B.L[slot]; }, [&](float4 L) { B.L[slot] = L; },
                               [&](uint32_t mat, float4 g) { block_gadd(gacc, mat, g); });
             if (v.scattered) B.thr[slot] = thr4;
@@ -1532,7 +1544,7 @@ __global__ void __launch_bounds__(256, ADJ ? 2 : 4) k_shade(DeviceScene S, Rende
             basepos = __shfl_sync(0xffffffffu, basepos, leader);
             if (v.cont) {
                 uint32_t pos = basepos + __popc(mask & ((1u << lane) - 1u));
-                __stcs(B.q_o[qi ^ 1] + pos, make_float4(v.no.x, v.no.y, v.no.z, __uint_as_float(slot)));
+                __stcs(B.q_o[qi ^ 1] + pos, make_float4(v.p.x, v.p.y, v.p.z, __uint_as_float(slot)));
                 __stcs(B.q_d[qi ^ 1] + pos, make_float4(v.nd.x, v.nd.y, v.nd.z, __uint_as_float(v.rng)));
             }
         }
@@ -1544,13 +1556,13 @@ __global__ void __launch_bounds__(256, ADJ ? 2 : 4) k_shade(DeviceScene S, Rende
             basepos = __shfl_sync(0xffffffffu, basepos, leader);
             if (v.shadow) {
                 uint32_t pos = basepos + __popc(smask & ((1u << lane) - 1u));
-                B.sh_o[pos] = make_float4(v.so.x, v.so.y, v.so.z, __uint_as_float(slot));
+                B.sh_o[pos] = make_float4(v.p.x, v.p.y, v.p.z, __uint_as_float(slot));
                 B.sh_d[pos] = make_float4(v.sd.x, v.sd.y, v.sd.z, v.smax);
                 B.sh_c[pos] = make_float4(v.sc.x, v.sc.y, v.sc.z, __uint_as_float(v.sh_bits));
                 if (ADJ) B.sh_g[pos] = v.sh_dlog;
             }
         }
-        if (!ADJ && P.cache_query_vertex) {
+        if (CACHE) {
             unsigned qmask = __ballot_sync(0xffffffffu, v.queried);
             if (qmask) {
                 int leader = __ffs(qmask) - 1;
@@ -1826,7 +1838,7 @@ __device__ __forceinline__ bool small_hit(const DeviceScene &S, const float4 *s_
 // threads: 160x120, 1 spp: 0.11 ms a call against 0.16 (queue kernels 0.37).
 constexpr int kPathsBlock = 896, kPathsSmallBlock = 128;
 constexpr uint32_t kFlush = 16;
-template <bool ADJ>
+template <bool ADJ, bool CACHE>
 __global__ void __launch_bounds__(kPathsBlock, 1)
     k_paths(DeviceScene S, RenderParams P, PathBuffers B, const SmallScene *T, uint32_t chunk, float4 *gbuf,
             AdjointParams A) {
@@ -1951,7 +1963,7 @@ __global__ void __launch_bounds__(kPathsBlock, 1)
                     g0 = pending_gradient(delta, L, pend);
                 }
             }
-            shade_vertex<ADJ>(S, P, o, d, h, slot, pixel, bounce, nee, gbuf, delta, thr4, v, [&]() { return L; },
+            shade_vertex<ADJ, CACHE>(S, P, o, d, h, slot, pixel, bounce, nee, gbuf, delta, thr4, v, [&]() { return L; },
                               [&](float4 x) { L = x; }, [&](uint32_t mat, float4 g) { m1 = mat; g1 = g; });
             rng = v.rng;
             if (ADJ) {
@@ -1970,7 +1982,7 @@ __global__ void __launch_bounds__(kPathsBlock, 1)
                     if (x != 0.0f) atomicAdd(A.grad + k, (double)x);
                 }
         }
-        if (!ADJ && P.cache_query_vertex) {
+        if (CACHE) {
             const unsigned qmask = __ballot_sync(0xffffffffu, v.queried);
             if (qmask) {
                 const int leader = __ffs(qmask) - 1;
@@ -1988,8 +2000,8 @@ __global__ void __launch_bounds__(kPathsBlock, 1)
         const bool was = go || shadow;
         go = v.cont;
         shadow = v.shadow;
-        if (go) { o = v.no; d = v.nd; ++bounce; }
-        if (shadow) { o = v.so; sd = v.sd; sc = v.sc; smax = v.smax; }
+        if (go) { o = v.p; d = v.nd; ++bounce; }
+        if (shadow) { o = v.p; sd = v.sd; sc = v.sc; smax = v.smax; }
         if (!ADJ && was && !go && !shadow) __stcs(B.L + slot, L);
     }
     rays = __reduce_add_sync(0xffffffffu, rays);
@@ -2194,10 +2206,10 @@ void prepare_extend_variants() {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_extend_packet<false>, kPacketBlock, 0);
         g_packet_per_sm = n > 0 ? n : 1;
         n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_paths<false>, kPathsSmallBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_paths<false, false>, kPathsSmallBlock, 0);
         g_paths_per_sm = n > 0 ? n : 1;
         n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_paths<true>, kPathsSmallBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_paths<true, false>, kPathsSmallBlock, 0);
         g_paths_adj_per_sm = n > 0 ? n : 1;
     }
     for (int v = 0; v < kExtendVariants; ++v) {
@@ -2270,8 +2282,9 @@ void launch_shade(const DeviceScene &S, const RenderParams &P, PathBuffers &B, i
                   float4 *gbuf, cudaStream_t st, const AdjointParams *adj) {
     uint32_t nmax = P.npix * P.spp_pass;
     int blocks = min(grid_blocks_for(nmax, 256), sm_count() * 8);
-    if (adj) k_shade<true><<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, *adj);
-    else k_shade<false><<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, AdjointParams{});
+    if (adj) k_shade<true, false><<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, *adj);
+    else if (P.cache_query_vertex) k_shade<false, true><<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, AdjointParams{});
+    else k_shade<false, false><<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, AdjointParams{});
     ::mcrt::note_launch();
 }
 
@@ -2308,8 +2321,9 @@ cudaError_t launch_paths(const DeviceScene &S, const RenderParams &P, PathBuffer
     const uint32_t chunk = max(32u, min(256u, n / (8u * warps) / 32u * 32u));
     cudaError_t e = cudaMemsetAsync(B.counters, 0, 8 * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    if (adj) k_paths<true><<<blocks, block, 0, st>>>(S, P, B, T, chunk, gbuf, *adj);
-    else k_paths<false><<<blocks, block, 0, st>>>(S, P, B, T, chunk, gbuf, AdjointParams{});
+    if (adj) k_paths<true, false><<<blocks, block, 0, st>>>(S, P, B, T, chunk, gbuf, *adj);
+    else if (P.cache_query_vertex) k_paths<false, true><<<blocks, block, 0, st>>>(S, P, B, T, chunk, gbuf, AdjointParams{});
+    else k_paths<false, false><<<blocks, block, 0, st>>>(S, P, B, T, chunk, gbuf, AdjointParams{});
     ::mcrt::note_launch();
     return cudaGetLastError();
 }
