@@ -782,23 +782,36 @@ __global__ void k_cache_judge_queries(const float4 *s, const uint32_t *count, fl
 // differences, not of ratios: their quotient is the cache's relative bias on
 // the radiance it stands for, and the per-sample noise of the targets averages
 // out of the numerator.
-__global__ void k_cache_judge(const float4 *s, const float *y, const uint32_t *count, double *acc) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n = *count;
-    float v[7] = {0, 0, 0, 0, 0, 0, 0};
-    if (i < n) {
-        const float4 t = s[4 * (size_t)i + 3];
-        if (t.w > 0.0f) {
-            v[0] = fmaxf(y[3 * (size_t)i], 0.0f) - t.x;
-            v[1] = fmaxf(y[3 * (size_t)i + 1], 0.0f) - t.y;
-            v[2] = fmaxf(y[3 * (size_t)i + 2], 0.0f) - t.z;
-            v[3] = t.x; v[4] = t.y; v[5] = t.z; v[6] = 1.0f;
+// Bound by the double atomics on seven words (73.8 us for up to 524,288 samples with
+// seven per warp of 32 samples, 13.4 now): a warp adds its sums of 32 samples up in
+// doubles, a block its warps', and kJudgeBlocks blocks per SM add seven each.
+constexpr uint32_t kJudgeBlocks = 4;
+__global__ void __launch_bounds__(256) k_cache_judge(const float4 *s, const float *y, const uint32_t *count, double *acc) {
+    __shared__ double part[8][7];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n = *count;
+    double a[7] = {0, 0, 0, 0, 0, 0, 0};
+    for (uint64_t base = blockIdx.x * 256u + (threadIdx.x & ~31u); base < n; base += (uint64_t)gridDim.x * 256u) {
+        const uint64_t i = base + lane;
+        float v[7] = {0, 0, 0, 0, 0, 0, 0};
+        if (i < n) {
+            const float4 t = s[4 * i + 3];
+            if (t.w > 0.0f) {
+                v[0] = fmaxf(y[3 * i], 0.0f) - t.x;
+                v[1] = fmaxf(y[3 * i + 1], 0.0f) - t.y;
+                v[2] = fmaxf(y[3 * i + 2], 0.0f) - t.z;
+                v[3] = t.x; v[4] = t.y; v[5] = t.z; v[6] = 1.0f;
+            }
         }
-    }
 #pragma unroll
-    for (int k = 0; k < 7; ++k) {
-        const float w = warp_sum(v[k]);
-        if ((threadIdx.x & 31u) == 0u && w != 0.0f) atomicAdd(acc + k, (double)w);
+        for (int k = 0; k < 7; ++k) a[k] += (double)warp_sum(v[k]);
+    }
+    if (lane == 0)
+        for (int k = 0; k < 7; ++k) part[warp][k] = a[k];
+    __syncthreads();
+    if (threadIdx.x < 7u) {
+        double sum = 0.0;
+        for (int w = 0; w < 8; ++w) sum += part[w][threadIdx.x];
+        if (sum != 0.0) atomicAdd(acc + threadIdx.x, sum);
     }
 }
 
@@ -1046,7 +1059,7 @@ cudaError_t cache_train_records(CacheState *c, const float4 *rec, uint32_t n_tra
         k_cache_judge_queries<<<grid, 256, 0, st>>>(c->samples.as<float4>(), count, q);
         note_launch();
         if ((e = cache_infer_device(c, q, count, (uint32_t)cap, y, nullptr, nullptr, st)) != cudaSuccess) return e;
-        k_cache_judge<<<grid, 256, 0, st>>>(c->samples.as<float4>(), y, count, c->judge.as<double>());
+        k_cache_judge<<<std::min(grid, kJudgeBlocks * (uint32_t)sm_count()), 256, 0, st>>>(c->samples.as<float4>(), y, count, c->judge.as<double>());
         note_launch();
     }
     if (steps == 0) return cudaSuccess;

@@ -160,3 +160,22 @@ def test_world_invalid_inputs(ctx):
     ctx.world_upload(np.zeros((16, 8, 16), np.uint8))
     with pytest.raises(M.MCRTError):
         ctx.upload_scene(materials=scenes.voxel_world()["materials"], world_mesh=True)   # not meshed yet
+
+
+@pytest.mark.parametrize("shape", [(16, 48, 16), (128, 96, 128)])
+def test_world_mesh_read_into_unwritten_and_used_memory(ctx, shape):
+    """Meshes below and above 8 MB, into pages that are not there yet, off a page's start."""
+    import mmap
+    from mcrt_gb300 import _native as N
+    w = scenes.voxel_world(seed=9, nx=shape[0], ny=shape[1], nz=shape[2])
+    ctx.world_generate(w["params"])
+    nv, nt = ctx.world_mesh(w["block_material"], greedy=False)
+    v, t = ctx.world_read_mesh()
+    assert (nv * 48 + nt * 16 >= 8 << 20) == (shape[0] == 128)
+    m = mmap.mmap(-1, nv * 48 + nt * 16 + 64)                     # anonymous, untouched
+    mem = np.frombuffer(m, np.uint8)
+    for _ in range(2):
+        a, b = mem[16:16 + nv * 48], mem[16 + nv * 48:16 + nv * 48 + nt * 16]
+        assert N.lib().mcrt_world_read_mesh(ctx._h, a.ctypes.data, nv, b.ctypes.data, nt) == 0
+        assert a.tobytes() == v.tobytes() and b.tobytes() == t.tobytes()
+        assert not mem[:16].any() and not mem[16 + nv * 48 + nt * 16:].any()
