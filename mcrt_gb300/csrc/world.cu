@@ -150,7 +150,8 @@ __global__ void __launch_bounds__(32 * kGenWarps) k_world_generate(mcrt_world_pa
                 (lattice_hash(gx, yi, gz, P.seed ^ 0x27d4eb2fu) & 7u) == 0u)
                 b = kCaveGlow;
         } else if (yi == surface + 1) {
-            // shrubs on some grass tops (nothing decorates the surface block itself)
+            // shrubs on some grass tops (nothing decorates the surface block itself); at two layers the
+            // surface is the top one, and surface + 1 no layer of the grid
             if (b == kAir && s_col[(uint32_t)surface * 32u + lane] == kGrass &&
                 (lattice_hash(gx, 0, gz, P.seed ^ 0x165667b1u) & 15u) == 0u)
                 b = kShrub;

@@ -222,7 +222,7 @@ void orc_world_generate(const orc_world_params *P, uint8_t *vox) {
         for (uint32_t y = 1; y + 1 < ny && (int32_t)y < surface; ++y)
             if (at(y) != AIR && at(y + 1) == AIR && (lhash(gx, (int32_t)y, gz, P->seed ^ 0x27d4eb2fu) & 7u) == 0u)
                 at(y) = CAVE_GLOW;
-        if (at((uint32_t)surface) == GRASS && at((uint32_t)surface + 1) == AIR &&
+        if ((uint32_t)surface + 1 < ny && at((uint32_t)surface) == GRASS && at((uint32_t)surface + 1) == AIR &&
             (lhash(gx, 0, gz, P->seed ^ 0x165667b1u) & 15u) == 0u)
             at((uint32_t)surface + 1) = SHRUB;
     }

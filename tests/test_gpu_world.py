@@ -90,6 +90,15 @@ def test_world_generate_ragged_columns(ctx, oracle, shape):
     assert np.array_equal(ctx.world_generate(p, read_back=True), oracle.world_generate(p))
 
 
+@pytest.mark.parametrize("shape", [(16, 2, 16), (48, 2, 32)])
+def test_world_generate_two_layers(ctx, oracle, shape):
+    """The smallest height: grass on top, where a shrub would be outside of the grid."""
+    p = dict(scenes.world_params(7, *shape), sand_line=-1.0, sea_level=-1.0)
+    vox = ctx.world_generate(p, read_back=True)
+    assert np.array_equal(vox, oracle.world_generate(p))
+    assert np.all(vox[:, 1, :] == 3) and not (vox == 8).any()
+
+
 def _world_scene(ctx, seed=3, n=48):
     w = scenes.voxel_world(seed=seed, nx=n, ny=n, nz=n)
     ctx.world_generate(w["params"])

@@ -114,3 +114,16 @@ def test_voxel_world_workload_size(oracle):
     vox = oracle.world_generate(w["params"])
     _, t = oracle.world_mesh(vox, w["block_material"], greedy=False)
     assert 4_000_000 <= len(t) <= 6_000_000
+
+
+def test_generator_at_two_layers_stays_in_its_columns(oracle):
+    """The smallest height accepted: the surface is the top layer, so a shrub has no place in the grid."""
+    import ctypes
+    p = dict(scenes.world_params(7, 32, 2, 48), sand_line=-1.0, sea_level=-1.0)
+    oracle.world_generate(dict(p, ny=8))                          # binds the entry point
+    params = oracle._WorldParams(**p)
+    buf = np.zeros(32 * 2 * 48 + 4096, np.uint8)                  # air behind the grid
+    oracle.lib().orc_world_generate(ctypes.byref(params), buf.ctypes.data_as(ctypes.c_void_p))
+    vox = buf[:32 * 2 * 48].reshape(32, 2, 48)
+    assert not buf[32 * 2 * 48:].any()
+    assert np.all(vox[:, 0, :] == 2) and np.all(vox[:, 1, :] == 3)   # red soil under grass
