@@ -196,6 +196,7 @@ struct BvhScratch {
     void *mem = nullptr;
     BuildState s{};
     uint32_t *scan_tmp = nullptr;
+    bool configured = false;   // k_subtrees' 70 KB of dynamic shared memory, set on the context's device
 };
 
 void free_bvh_scratch(BvhScratch *s) {
@@ -1604,14 +1605,11 @@ static cudaError_t gpu_build(const mcrt_gpu_vertex *d_verts, const mcrt_gpu_tria
         n_sub = 1;
     }
     if (n_sub) {
-        static bool configured[64] = {};                 // per device: 70 KB of dynamic shared memory
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev >= 64 || !configured[dev]) {
+        if (!sc->configured) {
             cudaError_t e = cudaFuncSetAttribute(k_subtrees, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)sizeof(SubShared));
             if (e != cudaSuccess) { if (err) *err = "BVH subtree kernel"; return e; }
-            if (dev < 64) configured[dev] = true;
+            sc->configured = true;
         }
         k_subtrees<<<n_sub, kSubThreads, sizeof(SubShared), st>>>(S, cur); ::mcrt::note_launch();
     }

@@ -8,6 +8,8 @@
 // reference's two texture loads.  The per-tap arithmetic is the reference's
 // (same order of operations, denoise.wgsl:81-108).  Radii whose tile does not
 // fit the shared-memory budget read the taps from global memory.
+#include <atomic>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -117,7 +119,7 @@ void launch_denoise(const float4 *in, const float4 *gbuf, uint32_t w, uint32_t h
         size_t bytes = 2 * (size_t)span * span * sizeof(float4) + wbytes;
         k_denoise<true><<<grid, block, bytes, st>>>(in, gbuf, (int)w, (int)h, q, out); ::mcrt::note_launch();
     } else {
-        static bool configured = false;
+        static std::atomic<bool> configured{false};
         if (!configured) {
             cudaFuncSetAttribute(k_denoise<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
             configured = true;

@@ -4,6 +4,7 @@
 // This file starts with the probe of one tensor-core product, which pins the
 // operand layouts and descriptors of tc.cuh against a CPU product.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -923,7 +924,7 @@ static cudaError_t check_status(CacheState *c, cudaStream_t st, bool *timed_out)
 // the tracer's L / thr.
 // Shared-memory attributes of the two tensor-core kernels, set once (before
 // any capture: cache_prepare sets them too).
-static bool g_infer_attr = false, g_train_attr = false;
+static std::atomic<bool> g_infer_attr{false}, g_train_attr{false};
 
 cudaError_t cache_infer_device(CacheState *c, const float4 *q, const uint32_t *d_count, uint32_t max_n, float *out,
                                float4 *L, const float4 *thr, cudaStream_t st) {

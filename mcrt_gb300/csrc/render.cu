@@ -2115,13 +2115,12 @@ void launch_light_cdf(const DeviceScene &S, float *d_cdf, float *d_total, cudaSt
 // ------------------------------------------------------------------ launchers
 
 int sm_count() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
+    static const int n = [] {
+        int dev = 0, v = 0;
         cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v > 0 ? v : 1;
+    }();
     return n;
 }
 
@@ -2189,11 +2188,33 @@ const ExtendKernel kCountKernels[kExtendVariants] = {
 #undef MCRT_COUNT_KERNEL
 #undef MCRT_EXTEND_TABLE
 #undef MCRT_EXTEND_KERNEL
-int g_extend_per_sm[kExtendVariants] = {0, 0, 0, 0, 0, 0, 0, 0};
-int g_shadow_per_sm[kExtendVariants] = {0, 0, 0, 0, 0, 0, 0, 0};
-int g_shadow_adj_per_sm[kExtendVariants] = {0, 0, 0, 0, 0, 0, 0, 0};
-int g_packet_per_sm = 0, g_paths_per_sm = 0, g_paths_adj_per_sm = 0;
-int g_count_per_sm[kExtendVariants] = {0, 0, 0, 0, 0, 0, 0, 0};
+// Resident blocks per SM of the persistent kernels.
+struct Resident {
+    int extend[kExtendVariants], shadow[kExtendVariants], shadow_adj[kExtendVariants], count[kExtendVariants];
+    int packet, paths, paths_adj;
+};
+template <class Kernel> int resident_blocks(Kernel k, int block) {
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, block, 0);
+    return n > 0 ? n : 1;
+}
+// Queried once per process, by the first caller.
+const Resident &resident() {
+    static const Resident r = [] {
+        Resident q{};
+        q.packet = resident_blocks(k_extend_packet<false>, kPacketBlock);
+        q.paths = resident_blocks(k_paths<false, false>, kPathsSmallBlock);
+        q.paths_adj = resident_blocks(k_paths<true, false>, kPathsSmallBlock);
+        for (int v = 0; v < kExtendVariants; ++v) {
+            q.extend[v] = resident_blocks(kExtendKernels[v], kVariantTable[v].block);
+            q.shadow[v] = resident_blocks(kShadowKernels[v], kVariantTable[v].block);
+            q.shadow_adj[v] = resident_blocks(kShadowAdjKernels[v], kVariantTable[v].block);
+            q.count[v] = resident_blocks(kCountKernels[v], kVariantTable[v].block);
+        }
+        return q;
+    }();
+    return r;
+}
 }  // namespace
 
 void extend_variant_info(int v, int out[6]) {
@@ -2201,43 +2222,8 @@ void extend_variant_info(int v, int out[6]) {
     out[0] = e.width; out[1] = e.block; out[2] = e.min_blocks; out[3] = e.stack; out[4] = e.refill; out[5] = e.top;
 }
 
-// Resident blocks per SM of every variant and of the packet kernel (occupancy
-// queries, made before any stream capture of a render).
-void prepare_extend_variants() {
-    if (g_packet_per_sm == 0) {
-        int n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_extend_packet<false>, kPacketBlock, 0);
-        g_packet_per_sm = n > 0 ? n : 1;
-        n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_paths<false, false>, kPathsSmallBlock, 0);
-        g_paths_per_sm = n > 0 ? n : 1;
-        n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_paths<true, false>, kPathsSmallBlock, 0);
-        g_paths_adj_per_sm = n > 0 ? n : 1;
-    }
-    for (int v = 0; v < kExtendVariants; ++v) {
-        if (g_extend_per_sm[v] == 0) {
-            int n = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kExtendKernels[v], kVariantTable[v].block, 0);
-            g_extend_per_sm[v] = n > 0 ? n : 1;
-        }
-        if (g_shadow_per_sm[v] == 0) {
-            int n = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kShadowKernels[v], kVariantTable[v].block, 0);
-            g_shadow_per_sm[v] = n > 0 ? n : 1;
-        }
-        if (g_shadow_adj_per_sm[v] == 0) {
-            int n = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kShadowAdjKernels[v], kVariantTable[v].block, 0);
-            g_shadow_adj_per_sm[v] = n > 0 ? n : 1;
-        }
-        if (g_count_per_sm[v] == 0) {
-            int n = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kCountKernels[v], kVariantTable[v].block, 0);
-            g_count_per_sm[v] = n > 0 ? n : 1;
-        }
-    }
-}
+// The occupancy queries of the launches below, before any stream capture of a render.
+void prepare_extend_variants() { (void)resident(); }
 
 // The rays of the overflow list (a stack too short for the tree), after each extend launch.
 static void launch_retry(const DeviceScene &S, PathBuffers &B, int qi, bool any, const AdjointParams *adj,
@@ -2252,7 +2238,6 @@ static void launch_retry(const DeviceScene &S, PathBuffers &B, int qi, bool any,
 void launch_extend(const DeviceScene &S, const RenderParams &P, PathBuffers &B, int qi, cudaStream_t st,
                    bool primary) {
     const int v = (P.extend_variant >= 0 && P.extend_variant < kExtendVariants) ? P.extend_variant : 0;
-    prepare_extend_variants();
     const uint32_t nmax = P.npix * P.spp_pass;
     const bool count = (P.flags & MCRT_RENDER_COUNT) != 0;
     // The camera rays as warp packets (every warp resident at once) or one per
@@ -2266,14 +2251,14 @@ void launch_extend(const DeviceScene &S, const RenderParams &P, PathBuffers &B, 
     // of them out of sight, 1280x720, 8 spp (1.5) 893 / 1124.  The line, 4/3
     // paths per triangle, leaves the last with packets.
     if (primary && 3ull * nmax >= 4ull * S.n_triangles) {
-        const int blocks = min(grid_blocks_for(nmax, kPacketBlock), sm_count() * g_packet_per_sm);
+        const int blocks = min(grid_blocks_for(nmax, kPacketBlock), sm_count() * resident().packet);
         if (count) k_extend_packet<true><<<blocks, kPacketBlock, 0, st>>>(S, B, qi);
         else k_extend_packet<false><<<blocks, kPacketBlock, 0, st>>>(S, B, qi);
         ::mcrt::note_launch();
     } else {
         // persistent: as many resident blocks as fit, never more warps than rays
         const int block = kVariantTable[v].block;
-        const int per_sm = count ? g_count_per_sm[v] : g_extend_per_sm[v];
+        const int per_sm = count ? resident().count[v] : resident().extend[v];
         const int blocks = min(grid_blocks_for(nmax, block / 32), sm_count() * per_sm);
         (count ? kCountKernels[v] : kExtendKernels[v])<<<blocks, block, 0, st>>>(S, B, qi, AdjointParams{});
         ::mcrt::note_launch();
@@ -2297,9 +2282,8 @@ void launch_shadow(const DeviceScene &S, const RenderParams &P, PathBuffers &B, 
     // replay's instantiation also adds the gradients of unoccluded rays
     uint32_t nmax = P.npix * P.spp_pass;
     const int v = (P.extend_variant >= 0 && P.extend_variant < kExtendVariants) ? P.extend_variant : 0;
-    prepare_extend_variants();
     const int block = kVariantTable[v].block;
-    const int per_sm = adj ? g_shadow_adj_per_sm[v] : g_shadow_per_sm[v];
+    const int per_sm = adj ? resident().shadow_adj[v] : resident().shadow[v];
     const int blocks = min(grid_blocks_for(nmax, block / 32), sm_count() * per_sm);
     if (adj) kShadowAdjKernels[v]<<<blocks, block, 0, st>>>(S, B, 0, *adj);
     else kShadowKernels[v]<<<blocks, block, 0, st>>>(S, B, 0, AdjointParams{});
@@ -2313,11 +2297,10 @@ void launch_small_scene(const DeviceScene &S, SmallScene *out, cudaStream_t st) 
 
 cudaError_t launch_paths(const DeviceScene &S, const RenderParams &P, PathBuffers &B, const SmallScene *T,
                          float4 *gbuf, cudaStream_t st, const AdjointParams *adj) {
-    prepare_extend_variants();
     const uint32_t n = P.npix * P.spp_pass;
     const bool large = n > kSmallPass;
     const int block = large ? kPathsBlock : kPathsSmallBlock;
-    const int per_sm = large ? 1 : adj ? g_paths_adj_per_sm : g_paths_per_sm;
+    const int per_sm = large ? 1 : adj ? resident().paths_adj : resident().paths;
     const int blocks = min(grid_blocks_for(n, block), sm_count() * per_sm);
     // slots per fetch: about eight fetches per warp, at most 256 slots
     const uint32_t warps = (uint32_t)blocks * (uint32_t)(block / 32);
