@@ -109,3 +109,30 @@ def test_adjoint_equals_the_queue_kernels(ctx, n_tri, n_sph, w, h):
     assert np.array_equal(bits(img), bits(want_img))
     assert np.array_equal(got != 0, want != 0)
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+def queue_adjoint(ctx, cam, w, h, spp, d, **kw):
+    """The adjoint with a named closest-hit variant: the queue kernels."""
+    import ctypes
+    o = M._native.RenderOpts(max_depth=kw["max_depth"], flags=M._native.RENDER_NEE if kw["nee"] else 0, variant=1)
+    grad, img = np.zeros(256, np.float64), np.zeros((h, w, 4), np.float32)
+    M.check(M.lib().mcrt_adjoint(ctx._h, M.ptr(cam), w, h, spp, 0, ctypes.byref(o), M.ptr(d), M.ptr(grad), M.ptr(img)), ctx._h)
+    return grad.reshape(64, 4), img
+
+
+# passes of 272,384 paths (two rounds of 896 per SM) and fewer take the small blocks and more scenes
+@pytest.mark.parametrize("n_tri,n_sph,w,h,spp,nee", [(64, 0, 100, 75, 16, True), (20, 16, 100, 75, 16, False),
+                                                    (40, 0, 256, 256, 8, True), (1, 0, 256, 200, 8, False)])
+def test_adjoint_of_both_path_kernel_forms(ctx, n_tri, n_sph, w, h, spp, nee):
+    """Sums of at most 2^13 float terms per block and parameter, of either sign, in another order (the queue kernels'
+    blocks): a random walk of 2^-24 of the partial sums, 2^6.5 x 2^-24 = 5e-6 of the result; doubles above them."""
+    ctx.upload_scene(env=M.gradient_env_map(), **soup(n_tri, n_sph, 11))
+    d = np.random.default_rng(1).standard_normal((h, w, 4)).astype(np.float32)
+    cam = camera(w, h)
+    got, img = ctx.adjoint(cam, w, h, spp, d, max_depth=6, nee=nee, with_image=True)
+    assert ctx.timings()["render_launches"] == 3               # paths, resolve, replay
+    want, want_img = queue_adjoint(ctx, cam, w, h, spp, d, max_depth=6, nee=nee)
+    assert ctx.timings()["render_launches"] > 12
+    assert np.array_equal(bits(img), bits(want_img))
+    assert np.array_equal(got != 0, want != 0)
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
