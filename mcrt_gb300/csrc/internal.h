@@ -55,7 +55,7 @@ struct PathBuffers {
     float4 *sh_c = nullptr;      // contribution rgb | unused
     // [0],[1] ray queue sizes, [2] shadow queue size, [3] closest-hit overflow list size,
     // [4],[5] work counters of the closest-hit and any-hit launches, [6] cache queries,
-    // [7] any-hit overflow list size
+    // [7] any-hit overflow list size, [8] what sharing a ray's subtrees was worth so far in the pass (trace_queue)
     uint32_t *counters = nullptr;
     unsigned long long *stats = nullptr;  // [0] rays traced, [1] shadow rays, [2] rays traced stackless
     uint32_t *ovf = nullptr;     // overflow list: queue entries whose traversal stack would overflow

@@ -490,7 +490,7 @@ __global__ void k_raygen(DeviceScene S, RenderParams P, PathBuffers B, int keep_
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {
         B.counters[0] = n; B.counters[1] = 0; B.counters[2] = 0; B.counters[3] = 0; B.counters[4] = 0;
-        B.counters[5] = 0; B.counters[6] = 0; B.counters[7] = 0;
+        B.counters[5] = 0; B.counters[6] = 0; B.counters[7] = 0; B.counters[8] = 0;
     }
     if (i >= n) return;
     f3 o, d;
@@ -743,19 +743,29 @@ constexpr uint32_t kOvfClosest = 3u, kOvfAny = 7u;
 // Taking over the oldest stack entry of a busy lane (its largest pending
 // subtree) cuts that tail: bounces of 20 to 200 thousand rays into an 80,000
 // triangle mesh took 112 to 131 us without sharing, 75 to 105 us with it.
-// The subtrees taken over are the far ones, which a nearer hit often culls,
-// and the code costs registers: with 5 million rays (voxel world) a launch took
-// 1.57 ms with sharing, 1.49 ms without.
+//
+// For closest hits the subtree taken over is a far one, and a hit in the nearer
+// ones makes it useless.  Rays that leave the scene (an open mesh) need all their
+// subtrees, rays into a voxel world hardly any of the far ones, so what sharing
+// is worth shows in its results: when a lane's result joins its ray's closest
+// hit, the subtree counts as useful unless it begins beyond that hit, and the sum
+// over the pass's launches (counters[kShareScore]) sets how many nodes a ray must
+// have visited before it gives: kGiveEarly, kGiveLate, or kGiveUnknown while
+// nothing is known.  It only shapes scheduling.  Closest hits per frame, in us,
+// giving at once / by the score / rays alone: voxel world of 4.9M faces, 200x150,
+// 4 spp 860 / 577 / 539, 480x270, 1 spp 894 / 614 / 552; 1.3M-triangle mesh,
+// 320x180, 1 spp 858 / 920 / 1515; 80,000 triangles 638 / 670 / 986.
+constexpr uint32_t kShareScore = 8u;
+constexpr uint32_t kGiveEarly = 4u, kGiveUnknown = 32u, kGiveLate = 128u;
 // A lone ray that is done within kProbeSteps never gets there: single caller's
 // rays take 33 us with it, 37 without.
 constexpr uint32_t kProbeSteps = 24;
 // SHARE below this many rays per lane of the grid: one for the render's queues,
 // more for the caller's rays (250,000 into an 80,000-triangle mesh: 350 us with
-// the limit at eight, 393 at one).  With eight in the render a frame of 1.3M
-// small triangles gains (24.4 instead of 25.5 ms), but voxel worlds, whose rays
-// are soon done, lose: 309,000 paths 1.30 ms instead of 1.23, eight views 7.80
-// instead of 7.73.  (Part of it is register allocation: with the limit hidden from
-// the compiler the frame takes 24.7 and the 309,000 paths 1.27 ms.)
+// the limit at eight, 393 at one).  With eight in the render, and subtrees given
+// at once, a frame of 1.3M small triangles gained (24.4 instead of 25.5 ms), but
+// voxel worlds lost: 309,000 paths 1.30 ms instead of 1.23, eight views 7.80
+// instead of 7.73.
 constexpr uint32_t kShareLoad = 1, kProbeShareLoad = 8;
 template <int WIDTH, int BLOCK, int STACK, int REFILL, int TOP, bool ANY, bool ADJ, bool COUNT, bool SHARE,
           bool PROBE = false>
@@ -786,6 +796,19 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
     uint32_t ntri = 0;                // COUNT: triangles tested
     uint32_t slot = 0;                // ANY: the shadow ray's path
     bool occl = false;                // ANY: an accepted hit was found
+    // SHARE, closest hit (see above): visits before the ray gives, visits so far, entry distance of the subtree
+    // that the lane took over (-1: the ray's first lane), useful less useless subtrees
+    uint32_t give_after = 0, visits = 0;
+    float taken_t = -1.0f;
+    int score = 0;
+    if (SHARE && !ANY && !PROBE) {
+        const int known = __ldcg(reinterpret_cast<const int *>(B.counters) + kShareScore);
+        give_after = known > 0 ? kGiveEarly : (known < 0 ? kGiveLate : kGiveUnknown);
+    }
+    // a queue spread over the warps walks on until no lane has an internal node left: with few rays to a warp,
+    // testing leaves early only repeats the rounds around the walk (4.9M faces, 480x270, 1 spp: 1060 us with
+    // kKeepWalking, 900 without; 80,000 triangles, 320x180: 672 and 644)
+    const int keep_walking = spread ? 1 : kKeepWalking;
     // drops everything the lane has left to do for its ray
     auto drop = [&]() {
         cur = kNoChild;
@@ -827,6 +850,8 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             const uint32_t mine = base + __popc(idle_mask & below);
             if (ray == kNoRay && mine < end) {
                 ray = mine;
+                visits = 0;
+                taken_t = -1.0f;
                 float4 o4, d4;
                 if (PROBE) {
                     ld_pair(qo + 2ull * mine, &o4, &d4);
@@ -863,12 +888,17 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             }
         } else if (SHARE && exhausted && idle_mask) {
             // ---- no ray is left: idle lanes take over the oldest stack entries (the largest subtrees) of busy ones
-            const unsigned offers = __ballot_sync(0xffffffffu, sp > sb);
+            if (!ANY) {                                         // entries that a hit has culled since are not worth giving
+                while (sb < sp && __uint_as_float(stack[sb].y) > cull_t(best.t)) ++sb;
+                if (sb == sp) sp = sb = 0;
+            }
+            const bool offer = sp > sb && (ANY || visits >= give_after);
+            const unsigned offers = __ballot_sync(0xffffffffu, offer);
             const uint32_t pairs = min(__popc(idle_mask), __popc(offers));
             if (PROBE) share_after = kShareSteps;
             if (pairs) {
                 const bool takes = ray == kNoRay && __popc(idle_mask & below) < pairs;
-                const bool gives = sp > sb && __popc(offers & below) < pairs;
+                const bool gives = offer && __popc(offers & below) < pairs;
                 uint2 e = make_uint2(kNoChild, 0u);
                 if (gives) e = stack[sb++];
                 const int from = takes ? (int)nth_bit(offers, __popc(idle_mask & below)) : (int)lane;
@@ -886,6 +916,8 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
                     occl = false;
                     cur = e.x;
                     cur_t = __uint_as_float(e.y);
+                    visits = 0;
+                    taken_t = cur_t;
                 }
             }
         }
@@ -895,10 +927,11 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             const bool go = cur < kLeafBit;                      // an internal node (leaves and kNoChild have bit 31)
             const unsigned going = __ballot_sync(0xffffffffu, go);
             if (going == 0) break;
-            if (__popc(going) < kKeepWalking && __any_sync(0xffffffffu, leaf != kNoChild)) break;
+            if (__popc(going) < keep_walking && __any_sync(0xffffffffu, leaf != kNoChild)) break;
             if (SHARE && exhausted && idle_mask && step >= share_after) break;
             if (go) {
                 ++nn;
+                ++visits;
                 bool full = false;
                 if (WIDTH == 4) visit_wide4<STACK>(S, r, best.t, &cur, &cur_t, stack, &sp, &full);
                 else visit_compact2<STACK, TOP>(S, s_top, r, tmin, best.t, &cur, &cur_t, stack, &sp, &full);
@@ -963,6 +996,11 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
                             drop();
                         }
                     }
+                    if (!PROBE) {
+                        const float begins = __shfl_sync(0xffffffffu, taken_t, f);
+                        const float hit_t = __shfl_sync(0xffffffffu, best.t, __ffs(others) - 1);
+                        if (begins >= 0.0f) score += begins > cull_t(hit_t) ? -1 : 1;
+                    }
                 }
                 if ((int)lane == f) {
                     ray = kNoRay;
@@ -986,6 +1024,7 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             ray = kNoRay;
         }
     }
+    if (SHARE && !ANY && !PROBE && score && lane == 0) atomicAdd(reinterpret_cast<int *>(B.counters) + kShareScore, score);
     if (!PROBE && traced) atomicAdd(B.stats + (ANY ? 1 : 0), (unsigned long long)traced);
     if (COUNT) {
         atomicAdd(B.stats + 3, (unsigned long long)nn);

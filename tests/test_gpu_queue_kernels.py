@@ -99,3 +99,21 @@ def test_adjoint_matches_bruteforce_gradient(ctx, oracle, name, nee):
     assert scale > 0
     assert np.all(np.abs(g - want) <= 2e-4 * scale + 2e-3 * np.abs(want)), np.abs(g - want).max() / scale
     assert np.array_equal(g != 0, want != 0)
+
+
+def test_sharing_does_little_useless_work(ctx):
+    """Idle lanes take over subtrees of busy rays.  In a voxel world most of those lie behind the ray's hit: a frame of
+    few paths, whose queues are shared, may visit at most a quarter more nodes per ray than a frame of many."""
+    sc = scenes.voxel_world(3, 256, 128, 256)
+    ctx.world_generate(sc["params"])
+    ctx.world_mesh(sc["block_material"], sc["voxel_size"], greedy=False)
+    ctx.upload_scene(materials=sc["materials"], env=M.gradient_env_map(), sun_dir=sc["sun_dir"],
+                     sun_irradiance=sc["sun_irradiance"], world_mesh=True)
+    cam = camera(sc, 320, 180)
+
+    def nodes_per_ray(spp):
+        ctx.render(cam, 320, 180, spp, max_depth=6, nee=True, outputs=(), count=True)
+        t = ctx.timings()
+        return t["node_fetches"] / t["rays"]
+
+    assert nodes_per_ray(2) <= 1.25 * nodes_per_ray(64)
