@@ -511,10 +511,8 @@ __global__ void k_raygen(DeviceScene S, RenderParams P, PathBuffers B, int keep_
 //    idle, so lanes do not sit out the longest ray of a fixed assignment.
 //  * Traversal phase: a lane walks internal nodes and postpones the first leaf
 //    it reaches, going on until it reaches a second; once fewer than
-//    kKeepWalking lanes still walk while others hold a leaf, the warp tests
-//    its leaves together.  (Going on until the last lane reached a leaf cost
-//    22.2 ms of closest-hit time per 1.3M-triangle frame, leaving at 8, 12, 16
-//    and 20 lanes 18.9, 18.55, 18.65 and 19.1.)  The vote only shapes
+//    kKeepWalking lanes still walk, or all that do hold a leaf, the warp tests
+//    its leaves together.  This only shapes
 //    scheduling: every order enters every box that can hold a hit at or before
 //    the closest t (the cull's slack, kCullSlack), so the hit is the reference
 //    order's.
@@ -533,8 +531,15 @@ __global__ void k_raygen(DeviceScene S, RenderParams P, PathBuffers B, int keep_
 // below are read through L1 as in the other variants).
 struct ExtendVariant { int width, block, min_blocks, stack, refill, top; };
 // Lanes that must still be walking nodes for a warp to go on with them while
-// others hold a postponed leaf.
-constexpr int kKeepWalking = 12;
+// others hold a postponed leaf: kKeepWalking in a long queue's walk, whose lanes
+// leave the loop one by one, kKeepWalkingShared in the sharing walk's vote.
+// Closest hits, in us: 1.3M-triangle frame, voxel world frame, closed rooms of 252
+// and 972 triangles, 16 spp: lanes leaving one by one, going on at 0 / 8 / 12 / 16
+// lanes: 17670 / 16403 / 16170 / 16382, 4959 / 4927 / 4924 / 4892, 4621 / 4559 /
+// 4593 / 4675 and 8184 / 7895 / 7858 / 8057; by a vote of all lanes at 12:
+// 16593, 4958, 4704 and 8175.  Shadow rays in the rooms are best at 8 (3040 and
+// 3458 against 3061 and 3530 at 12).
+constexpr int kKeepWalking = 8, kKeepWalkingShared = 12;
 // Node visits between two rounds of sharing, once a warp has idle lanes and no ray is left.
 constexpr uint32_t kShareSteps = 4;
 constexpr uint32_t kNoRay = 0xffffffffu;
@@ -807,8 +812,8 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
     }
     // a queue spread over the warps walks on until no lane has an internal node left: with few rays to a warp,
     // testing leaves early only repeats the rounds around the walk (4.9M faces, 480x270, 1 spp: 1060 us with
-    // kKeepWalking, 900 without; 80,000 triangles, 320x180: 672 and 644)
-    const int keep_walking = spread ? 1 : kKeepWalking;
+    // kKeepWalkingShared, 900 without; 80,000 triangles, 320x180: 672 and 644)
+    const int keep_walking = spread ? 1 : kKeepWalkingShared;
     // drops everything the lane has left to do for its ray
     auto drop = [&]() {
         cur = kNoChild;
@@ -922,25 +927,40 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
             }
         }
         // ---- traversal phase
-        if (ray != kNoRay) settle();
-        for (uint32_t step = 0;; ++step) {
+        auto visit = [&]() {                                     // the internal node cur
+            ++nn;
+            ++visits;
+            bool full = false;
+            if (WIDTH == 4) visit_wide4<STACK>(S, r, best.t, &cur, &cur_t, stack, &sp, &full);
+            else visit_compact2<STACK, TOP>(S, s_top, r, tmin, best.t, &cur, &cur_t, stack, &sp, &full);
+            if (full) {                                          // to the overflow list
+                ray |= kOvfBit;
+                drop();
+            }
+        };
+        if (!SHARE && ray != kNoRay) {
+            for (;;) {
+                settle();
+                if (cur >= kLeafBit) break;                      // a second leaf, or none left
+                visit();
+                const unsigned walking = __activemask();
+                if (__popc(walking) < kKeepWalking || __all_sync(walking, leaf != kNoChild)) {
+                    settle();
+                    break;
+                }
+            }
+        }
+        __syncwarp();
+        if (SHARE && ray != kNoRay) settle();
+        for (uint32_t step = 0; SHARE; ++step) {
             const bool go = cur < kLeafBit;                      // an internal node (leaves and kNoChild have bit 31)
             const unsigned going = __ballot_sync(0xffffffffu, go);
             if (going == 0) break;
             if (__popc(going) < keep_walking && __any_sync(0xffffffffu, leaf != kNoChild)) break;
-            if (SHARE && exhausted && idle_mask && step >= share_after) break;
+            if (exhausted && idle_mask && step >= share_after) break;
             if (go) {
-                ++nn;
-                ++visits;
-                bool full = false;
-                if (WIDTH == 4) visit_wide4<STACK>(S, r, best.t, &cur, &cur_t, stack, &sp, &full);
-                else visit_compact2<STACK, TOP>(S, s_top, r, tmin, best.t, &cur, &cur_t, stack, &sp, &full);
-                if (full) {                                      // to the overflow list
-                    ray |= kOvfBit;
-                    drop();
-                } else {
-                    settle();
-                }
+                visit();
+                settle();
             }
         }
         // ---- leaf phase
