@@ -239,6 +239,7 @@ mcrt::DeviceScene device_scene(const mcrt_ctx *c) {
     S.has_sun = c->has_sun ? 1 : 0;
     S.sun_dir = make_float4(c->sun_dir[0], c->sun_dir[1], c->sun_dir[2], 0.0f);
     S.sun_E = make_float4(c->sun_E[0], c->sun_E[1], c->sun_E[2], 0.0f);
+    for (const mcrt_gpu_material &m : c->host_materials.materials) S.has_ggx |= m.type_pad[0] == MCRT_MAT_GGX ? 1 : 0;
     return S;
 }
 

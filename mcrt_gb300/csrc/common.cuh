@@ -130,6 +130,7 @@ struct DeviceScene {
     // directional light: unit direction towards it, irradiance at normal incidence
     int has_sun;
     float4 sun_dir, sun_E;
+    int has_ggx;                                     // a material of the table is a GGX conductor
 };
 
 }  // namespace mcrt

@@ -1313,9 +1313,6 @@ __global__ void __launch_bounds__(kPacketBlock) k_extend_packet(DeviceScene S, P
 // kernel: it is stored (B.pend, material in B.pend_mat bits 8..15) and applied at
 // the path's next vertex.  Gradients collect in shared memory per block, then
 // one double atomic per parameter and block.
-// Four resident blocks per SM (a 64-register budget) for the forward kernel:
-// it is bound by the latency of its scattered loads, and at the natural 88
-// registers only two blocks fit.  The replay variant keeps its registers.
 // Radiance-cache training path: the path ends at this bounce (a miss or an
 // emitter); record the radiance gathered before this event (which includes the
 // previous vertex's light sample) in place of a vertex.
@@ -1548,11 +1545,17 @@ __device__ __forceinline__ void shade_vertex(const DeviceScene &S, const RenderP
 }
 
 // CACHE: a render with the radiance cache, whose records and queries are code and
-// 16 registers that the others do without.  Bound by its scattered loads; three
-// blocks of 256 to an SM keep it out of local memory: 1.02 ms for the 18.7M hits of a
-// voxel world frame, four 1.13, two 1.18 (four with the cache's code inside: 1.21).
-template <bool ADJ, bool CACHE>
-__global__ void __launch_bounds__(256, ADJ ? 2 : 3) k_shade(DeviceScene S, RenderParams P, PathBuffers B, int qi,
+// 16 registers that the others do without.  Bound by its scattered loads.
+// BLOCKS: resident blocks of 256 per SM, four (64 registers, 44 bytes spilt) or three
+// (80, none).  Shading per frame, four / three, in us: 1.3M-triangle mesh 3151 /
+// 3455; closed rooms with area lights, 60 triangles 2124 / 2623, 972 2756 / 3871; a
+// voxel world without next-event estimation 660 / 747, with area lights 1396 /
+// 1640; the sun as the only light and GGX materials, 80,000 triangles 850 / 936; but
+// the sun and no GGX material, whose threads use the fewest of the registers, voxel
+// worlds 990 / 910 and 1050 / 970, 80,000 triangles 724 / 686: launch_shade's
+// rule.  Seven blocks of 128 (72 registers, none spilt) are like three of 256.
+template <bool ADJ, bool CACHE, int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS) k_shade(DeviceScene S, RenderParams P, PathBuffers B, int qi,
                                                 uint32_t bounce, float4 *gbuf, AdjointParams A) {
     __shared__ float gacc[ADJ ? 256 : 1];
     if (ADJ) {
@@ -2329,9 +2332,14 @@ void launch_shade(const DeviceScene &S, const RenderParams &P, PathBuffers &B, i
                   float4 *gbuf, cudaStream_t st, const AdjointParams *adj) {
     uint32_t nmax = P.npix * P.spp_pass;
     int blocks = min(grid_blocks_for(nmax, 256), sm_count() * 8);
-    if (adj) k_shade<true, false><<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, *adj);
-    else if (P.cache_query_vertex) k_shade<false, true><<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, AdjointParams{});
-    else k_shade<false, false><<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, AdjointParams{});
+    const AdjointParams none{};
+    // three blocks per SM where a vertex needs little code (see k_shade)
+    const bool lean = (P.flags & MCRT_RENDER_NEE) != 0 && S.has_sun && S.n_lights == 0 && !S.has_ggx;
+    if (adj) k_shade<true, false, 2><<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, *adj);
+    else if (P.cache_query_vertex)
+        (lean ? k_shade<false, true, 3> : k_shade<false, true, 4>)<<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, none);
+    else
+        (lean ? k_shade<false, false, 3> : k_shade<false, false, 4>)<<<blocks, 256, 0, st>>>(S, P, B, qi, bounce, gbuf, none);
     ::mcrt::note_launch();
 }
 
