@@ -376,12 +376,14 @@ mcrt_status render_variant(mcrt_ctx *ctx, const mcrt_render_opts &o, int *varian
 }
 
 // Whether a render with passes of n_slots paths takes the path kernel of small
-// scenes: few triangles and spheres for its passes (kSmallPass), and neither a
-// closest-hit variant nor the counting kernels asked for.
-bool small_scene(const mcrt_ctx *ctx, const mcrt_render_opts &o, uint32_t n_slots) {
+// scenes: few triangles and spheres for its passes, in large ones paths long
+// enough (kSmallPass), and neither a closest-hit variant nor the counting
+// kernels asked for.
+bool small_scene(const mcrt_ctx *ctx, const mcrt_render_opts &o, uint32_t n_slots, uint32_t depth, bool nee) {
     if (!ctx->small_ok || o.variant != 0 || (o.flags & MCRT_RENDER_COUNT)) return false;
-    return n_slots <= mcrt::kSmallPass ? ctx->n_spheres <= mcrt::kSmallSpheres
-                                       : ctx->n_spheres == 0 && ctx->n_triangles <= mcrt::kFewTris;
+    return n_slots <= mcrt::kSmallPass
+               ? ctx->n_spheres <= mcrt::kSmallSpheres
+               : ctx->n_spheres == 0 && ctx->n_triangles <= mcrt::kFewTris && depth > (nee ? 2u : 1u);
 }
 
 // Light CDF over the light list (device), total weight read back.
@@ -949,7 +951,7 @@ static mcrt_status render_core(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, ui
     };
     mcrt_status pass_status = MCRT_OK;
     // one pass: raygen, the bounces, resolve (into the accumulation)
-    const bool small = small_scene(ctx, o, n_slots);
+    const bool small = small_scene(ctx, o, n_slots, depth, nee);
     auto enqueue_pass = [&](const mcrt::RenderParams &P, bool keep_pass, bool timed) {
         if (small) {                                  // whole paths in one kernel, counted as closest-hit time
             size_t a0 = 0;
@@ -1222,7 +1224,7 @@ mcrt_status mcrt_adjoint(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, uint32_t
     A.inv_spp = 1.0f / (float)spp;
     A.grad = ctx->grad.as<double>();
     const bool nee = (o.flags & MCRT_RENDER_NEE) != 0 && (ctx->n_lights > 0 || ctx->has_sun);
-    const bool small = small_scene(ctx, o, npix * spp_pass);
+    const bool small = small_scene(ctx, o, npix * spp_pass, depth, nee);
     const unsigned long long launches0 = mcrt::launch_count();
     cudaEvent_t e_begin = ev(ctx, 2), e_end = ev(ctx, 3);
     cudaEventRecord(e_begin, st);

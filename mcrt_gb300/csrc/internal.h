@@ -80,6 +80,11 @@ constexpr uint32_t kSmallSpheres = 16;   // the path kernel's limit for a scene'
 // 2.24, of 64 3.80 / 3.26; 64 triangles and 16 spheres, NEE 14.3 / 9.5; 16
 // spheres, NEE 2.4 / 1.9.  160x120, 1 spp, where the queue kernels' launches
 // count: 64 triangles 0.10 / 0.36 ms, with 16 spheres and NEE 0.23 / 0.67.
+// Nor do they take it for paths of one segment (two with NEE): the warp packets of
+// the camera rays and of their pixel's shadow rays leave it little to gain.  Depth
+// 1 and 2, 16 spp: Cornell box NEE 0.99 / 0.91 and 1.82 / 2.05 ms, with GGX 1.20
+// / 0.97 and 1.90 / 2.02, a closed room of 36 triangles NEE 1.15 / 0.89 and 2.54 /
+// 2.18, without NEE 0.40 / 0.44 and 0.87 / 1.09, 36 triangles in the open 0.37 / 0.33.
 constexpr uint32_t kSmallPass = 2u * 896u * 152u, kFewTris = 40;
 struct SmallScene {
     float4 pair[8 * (kSmallTris / 2)];

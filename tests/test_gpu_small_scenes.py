@@ -136,3 +136,19 @@ def test_adjoint_of_both_path_kernel_forms(ctx, n_tri, n_sph, w, h, spp, nee):
     assert np.array_equal(bits(img), bits(want_img))
     assert np.array_equal(got != 0, want != 0)
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("depth,nee,path", [(1, False, False), (1, True, False), (2, False, True), (2, True, False), (3, True, True)])
+def test_large_passes_of_short_paths(ctx, depth, nee, path):
+    """Paths of one segment (two with next-event estimation) go through the queue kernels when there are many."""
+    from mcrt_gb300 import scenes
+    sc = scenes.cornell_box(3)
+    c = sc["camera"]
+    ctx.upload_scene(vertices=sc["vertices"], triangles=sc["triangles"], materials=sc["materials"], env=M.gradient_env_map())
+    for spp in (1, 16):
+        cam = M.compute_camera(160, 120, c["look_from"], c["look_at"], c["vfov"], 0.0)
+        got = ctx.render(cam, 160, 120, spp, max_depth=depth, nee=nee)
+        assert (ctx.timings()["shade_ms"] == 0.0) == (path or spp == 1)
+        want = ctx.render(cam, 160, 120, spp, max_depth=depth, nee=nee, variant=0)
+        for k in ("rgba", "sum", "gbuf"):
+            assert np.array_equal(bits(got[k]), bits(want[k])), k
