@@ -124,8 +124,8 @@ struct mcrt_ctx {
     DBuf wnodes;
     uint32_t n_wnodes = 0;
     bool wide_valid = false;    // wnodes matches the current mesh BVH
-    DBuf small;                 // SmallScene of the current mesh, usable when small_ok
-    bool small_ok = false;
+    DBuf small;                 // SmallScene of the current mesh (at most kSmallTris triangles)
+    uint32_t *small_ok = nullptr;   // host memory that the device writes: whether it may be used
     DBuf spheres, sphere_ids, sphere_nodes, vertices, triangles, mesh_nodes, tri_order, trirecs, cnodes, materials,
         env, lights, light_cdf, tmp, staging, albedo, shade_recs, top;
     uint32_t albedo_layers = 0, albedo_size = 0;
@@ -311,7 +311,6 @@ cudaEvent_t ev(mcrt_ctx *ctx, size_t i) {
 mcrt_status finish_mesh(mcrt_ctx *ctx) {
     cudaStream_t st = ctx->stream;
     uint32_t nt = ctx->n_triangles, nn = ctx->n_mesh_nodes;
-    ctx->small_ok = false;
     CK(ctx->trirecs.ensure((size_t)std::max(nt, 1u) * sizeof(mcrt::TriRec)), "allocate triangle records");
     CK(ctx->shade_recs.ensure((size_t)std::max(nt, 1u) * 48), "allocate shading records");
     mcrt::launch_shade_recs(ctx->vertices.as<mcrt_gpu_vertex>(), ctx->triangles.as<mcrt_gpu_triangle>(), nt,
@@ -328,15 +327,14 @@ mcrt_status finish_mesh(mcrt_ctx *ctx) {
     ctx->n_cnodes = ncn;
     if (ncn >= mcrt::kTopBit) return fail(ctx, MCRT_ERR_INVALID_ARG, "mesh too large for the compact BVH codes");
     CK(ctx->top.ensure((size_t)mcrt::kTopNodes * 64), "allocate top tree");
-    CK(mcrt::gpu_make_top(cn, ncn, ctx->top.as<float4>(), st), "top tree");
+    if (ncn) CK(mcrt::gpu_make_top(cn, ncn, ctx->top.as<float4>(), st), "top tree");   // else no walk enters it
     if (nt <= mcrt::kSmallTris) {
+        // the verdict goes straight to host memory and is there when the caller has waited for the stream, as
+        // every caller does (a read-back of its own: 76 us for a rebuild of one triangle, 58 this way)
         CK(ctx->small.ensure(sizeof(mcrt::SmallScene)), "allocate small scene");
-        mcrt::launch_small_scene(device_scene(ctx), ctx->small.as<mcrt::SmallScene>(), st);
-        uint32_t ok = 0;
-        CK(cudaMemcpyAsync(&ok, &ctx->small.as<mcrt::SmallScene>()->ok, 4, cudaMemcpyDeviceToHost, st),
-           "read small scene");
-        CK(cudaStreamSynchronize(st), "small scene");
-        ctx->small_ok = ok != 0;
+        if (!ctx->small_ok) CK(cudaHostAlloc((void **)&ctx->small_ok, 4, cudaHostAllocMapped), "allocate small scene");
+        *ctx->small_ok = 0;
+        mcrt::launch_small_scene(device_scene(ctx), ctx->small.as<mcrt::SmallScene>(), ctx->small_ok, st);
     }
     ctx->wide_valid = false;                  // the 4-wide layout is built when a render first needs it
     ctx->n_wnodes = 0;
@@ -380,7 +378,8 @@ mcrt_status render_variant(mcrt_ctx *ctx, const mcrt_render_opts &o, int *varian
 // enough (kSmallPass), and neither a closest-hit variant nor the counting
 // kernels asked for.
 bool small_scene(const mcrt_ctx *ctx, const mcrt_render_opts &o, uint32_t n_slots, uint32_t depth, bool nee) {
-    if (!ctx->small_ok || o.variant != 0 || (o.flags & MCRT_RENDER_COUNT)) return false;
+    if (o.variant != 0 || (o.flags & MCRT_RENDER_COUNT) || ctx->n_triangles > mcrt::kSmallTris) return false;
+    if (ctx->n_triangles && !*ctx->small_ok) return false;
     return n_slots <= mcrt::kSmallPass
                ? ctx->n_spheres <= mcrt::kSmallSpheres
                : ctx->n_spheres == 0 && ctx->n_triangles <= mcrt::kFewTris && depth > (nee ? 2u : 1u);
@@ -510,6 +509,7 @@ void mcrt_destroy(mcrt_ctx *ctx) {
     mcrt::cache_destroy(ctx->cache);
     mcrt::free_bvh_scratch(ctx->bvh_scratch);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
+    if (ctx->small_ok) cudaFreeHost(ctx->small_ok);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -641,9 +641,6 @@ mcrt_status mcrt_upload_scene(mcrt_ctx *ctx, const mcrt_scene_desc *d) {
         }
     } else {
         ctx->n_cnodes = 0;
-        CK(ctx->small.ensure(sizeof(mcrt::SmallScene)), "allocate small scene");
-        CK(cudaMemsetAsync(ctx->small.p, 0, sizeof(mcrt::SmallScene), st), "clear small scene");
-        ctx->small_ok = true;                  // no triangle: the spheres, or nothing
     }
     // ---- albedo texture array (binding 10)
     {
@@ -1043,8 +1040,8 @@ static mcrt_status render_core(mcrt_ctx *ctx, const mcrt_camera_uniform *cam, ui
             std::memcpy(k, extra, sizeof(extra)); k += sizeof(extra);
             std::memcpy(k, cbufs, sizeof(cbufs)); k += sizeof(cbufs);
             std::memcpy(k, &ccfg, sizeof(ccfg)); k += sizeof(ccfg);
-            const void *small_scene_ptr = small ? ctx->small.p : nullptr;
-            std::memcpy(k, &small_scene_ptr, sizeof(void *));
+            const uintptr_t path_kernel = small ? 1u + reinterpret_cast<uintptr_t>(ctx->small.p) : 0u;
+            std::memcpy(k, &path_kernel, sizeof(path_kernel));
         }
         if (!ctx->graph_exec || ctx->graph_key != key) {
             if (ctx->graph_exec) { cudaGraphExecDestroy(ctx->graph_exec); ctx->graph_exec = nullptr; }

@@ -88,9 +88,7 @@ constexpr uint32_t kSmallSpheres = 16;   // the path kernel's limit for a scene'
 constexpr uint32_t kSmallPass = 2u * 896u * 152u, kFewTris = 40;
 struct SmallScene {
     float4 pair[8 * (kSmallTris / 2)];
-    uint32_t n;
     float emax, vmax;
-    uint32_t ok;                         // 0: not for the path kernel
 };
 
 // Adjoint (path-replay backpropagation) inputs of the replay kernels.
@@ -152,9 +150,10 @@ void launch_shade(const DeviceScene &S, const RenderParams &P, PathBuffers &B, i
                   float4 *gbuf, cudaStream_t st, const AdjointParams *adj = nullptr);
 void launch_shadow(const DeviceScene &S, const RenderParams &P, PathBuffers &B, cudaStream_t st,
                    const AdjointParams *adj = nullptr);
-// Small scenes: the table of the current mesh (ok = 0: not for the path kernel), into device memory.
-void launch_small_scene(const DeviceScene &S, SmallScene *out, cudaStream_t st);
+// Small scenes: the table of the current mesh, into device memory (*ok = 0: not for the path kernel).
+void launch_small_scene(const DeviceScene &S, SmallScene *out, uint32_t *ok, cudaStream_t st);
 // Whole paths of a pass in one kernel (in place of raygen, extend, shade and shadow); adj: the replay.
+// T: the mesh's table, not read where there is no triangle.
 cudaError_t launch_paths(const DeviceScene &S, const RenderParams &P, PathBuffers &B, const SmallScene *T,
                          float4 *gbuf, cudaStream_t st, const AdjointParams *adj = nullptr);
 void launch_resolve(const RenderParams &P, const PathBuffers &B, float4 *mean, double *sum, bool keep,

@@ -1662,13 +1662,13 @@ __global__ void __launch_bounds__(256, BLOCKS) k_shade(DeviceScene S, RenderPara
 // its parent's (then a triangle is reached exactly when its leaf's box is
 // entered), and finite coordinates of moderate size.  One block of 2 kSmallTris
 // threads, a node and a triangle each.
-__global__ void __launch_bounds__(2 * kSmallTris) k_small_scene(DeviceScene S, SmallScene *out) {
+__global__ void __launch_bounds__(2 * kSmallTris) k_small_scene(DeviceScene S, SmallScene *out, uint32_t *ok) {
     __shared__ uint32_t covered[kSmallTris], parents[2 * kSmallTris];
-    __shared__ uint32_t bad;
-    __shared__ float red[2][kSmallTris];
+    __shared__ uint32_t bad, emax, vmax;                          // the bounds as bits: non-negative floats order so
     const uint32_t t = threadIdx.x;
-    if (t < kSmallTris) { covered[t] = 0; red[0][t] = red[1][t] = 0.0f; }
+    if (t < kSmallTris) covered[t] = 0;
     parents[t] = 0;
+    if (t == 0) emax = vmax = 0u;
     if (t == 0) bad = (S.n_triangles > kSmallTris || S.n_mesh_nodes >= 2 * kSmallTris) ? 1u : 0u;
     __syncthreads();
     const float limit = 1e9f;
@@ -1710,8 +1710,8 @@ __global__ void __launch_bounds__(2 * kSmallTris) k_small_scene(DeviceScene S, S
             ve += fabsf((float)v[a]); le1 += fabsf((float)e1[a]); le2 += fabsf((float)e2[a]);
         }
         q[3] = (float)k;
-        red[0][t] = fmaxf(le1, le2);
-        red[1][t] = ve;
+        atomicMax(&emax, __float_as_uint(fmaxf(le1, le2)));
+        atomicMax(&vmax, __float_as_uint(ve));
     }
     __syncthreads();
     if (t < S.n_triangles && t < kSmallTris && covered[t] != 1u) bad = 1u;
@@ -1722,12 +1722,9 @@ __global__ void __launch_bounds__(2 * kSmallTris) k_small_scene(DeviceScene S, S
         for (int k = 0; k < 16; ++k) pair[2 * k] = q[k];
     }
     if (t == 0) {
-        float emax = 0.0f, vmax = 0.0f;
-        for (uint32_t k = 0; k < kSmallTris; ++k) { emax = fmaxf(emax, red[0][k]); vmax = fmaxf(vmax, red[1][k]); }
-        out->n = min(S.n_triangles, kSmallTris);
-        out->emax = emax;
-        out->vmax = vmax + emax;
-        out->ok = bad ? 0u : 1u;
+        out->emax = __uint_as_float(emax);
+        out->vmax = __uint_as_float(vmax) + __uint_as_float(emax);
+        *ok = bad ? 0u : 1u;
     }
 }
 
@@ -1909,8 +1906,8 @@ __global__ void __launch_bounds__(kPathsBlock, 1)
             AdjointParams A) {
     __shared__ float gacc[ADJ ? 256 : 1];
     __shared__ float4 s_pair[4 * kSmallTris], s_tri[3 * kSmallTris], s_box[2 * kSmallTris];
-    const uint32_t nt = T->n;
-    const float emax = T->emax, vmax = T->vmax;
+    const uint32_t nt = S.n_triangles;
+    const float emax = nt ? T->emax : 0.0f, vmax = nt ? T->vmax : 0.0f;
     if (ADJ)
         for (uint32_t k = threadIdx.x; k < 256u; k += blockDim.x) gacc[k] = 0.0f;
     for (uint32_t k = threadIdx.x; k < 8u * ((nt + 1u) / 2u); k += blockDim.x) s_pair[k] = __ldg(T->pair + k);
@@ -2358,8 +2355,8 @@ void launch_shadow(const DeviceScene &S, const RenderParams &P, PathBuffers &B, 
     launch_retry(S, B, 0, true, adj, st);
 }
 
-void launch_small_scene(const DeviceScene &S, SmallScene *out, cudaStream_t st) {
-    k_small_scene<<<1, 2 * kSmallTris, 0, st>>>(S, out); ::mcrt::note_launch();
+void launch_small_scene(const DeviceScene &S, SmallScene *out, uint32_t *ok, cudaStream_t st) {
+    k_small_scene<<<1, 2 * kSmallTris, 0, st>>>(S, out, ok); ::mcrt::note_launch();
 }
 
 cudaError_t launch_paths(const DeviceScene &S, const RenderParams &P, PathBuffers &B, const SmallScene *T,

@@ -152,3 +152,21 @@ def test_large_passes_of_short_paths(ctx, depth, nee, path):
         want = ctx.render(cam, 160, 120, spp, max_depth=depth, nee=nee, variant=0)
         for k in ("rgba", "sum", "gbuf"):
             assert np.array_equal(bits(got[k]), bits(want[k])), k
+
+
+def test_table_follows_the_geometry(ctx):
+    """The path kernel's table after new vertices: refused beyond coordinates of 1e9, taken again after them; a scene
+    without triangles, from one graph to the other."""
+    s = soup(20, 0, 9)
+    ctx.upload_scene(env=M.gradient_env_map(), **s)
+    far = s["vertices"].copy()
+    far["position"][:3, :3] *= np.float32(4e9)
+    for v, path in ((None, True), (far, False), (s["vertices"], True)):
+        if v is not None:
+            ctx.update_vertices(v)
+        got = ctx.render(camera(40, 30), 40, 30, 2, nee=True)["rgba"]
+        assert (ctx.timings()["shade_ms"] == 0.0) == path
+        assert np.array_equal(bits(got), bits(ctx.render(camera(40, 30), 40, 30, 2, nee=True, variant=0)["rgba"]))
+    ctx.upload_scene(env=M.gradient_env_map(), **soup(0, 3, 9))
+    imgs = [ctx.render(camera(40, 30), 40, 30, 4, nee=True, spp_per_pass=2, graph=True, variant=v)["rgba"] for v in (None, 0, None)]
+    assert np.array_equal(bits(imgs[0]), bits(imgs[1])) and np.array_equal(bits(imgs[0]), bits(imgs[2]))
