@@ -196,12 +196,16 @@ struct BvhScratch {
     void *mem = nullptr;
     BuildState s{};
     uint32_t *scan_tmp = nullptr;
+    uint32_t *large = nullptr;  // host memory that the device writes: the large tasks that the first split left
+    cudaEvent_t looked = nullptr;
     bool configured = false;   // k_subtrees' 70 KB of dynamic shared memory, set on the context's device
 };
 
 void free_bvh_scratch(BvhScratch *s) {
     if (!s) return;
     if (s->mem) cudaFree(s->mem);
+    if (s->large) cudaFreeHost(s->large);
+    if (s->looked) cudaEventDestroy(s->looked);
     delete s;
 }
 
@@ -414,10 +418,13 @@ __device__ __forceinline__ void level_advance(BuildState &S, uint32_t level) {
 // The start of a level with large tasks, in one launch: level_advance, the
 // status words of the level's partition scan zeroed (n_part), and the large
 // tasks' centroid bounds and bins set to empty.
-// ntasks: at least the number of large tasks.
-__global__ void k_task_reset(BuildState S, uint32_t level, uint32_t ntasks, uint32_t n_part) {
+// ntasks: at least the number of large tasks, which goes to *large when given.
+__global__ void k_task_reset(BuildState S, uint32_t level, uint32_t ntasks, uint32_t n_part, uint32_t *large) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) level_advance(S, level);
+    if (i == 0) {
+        if (large) *large = S.counters[0];
+        level_advance(S, level);
+    }
     if (i < n_part) S.part[i] = 0ull;
     if (i >= ntasks * (6 + kTaskBinWords)) return;
     uint32_t t = i / (6 + kTaskBinWords), k = i % (6 + kTaskBinWords);
@@ -1563,7 +1570,12 @@ static cudaError_t gpu_build(const mcrt_gpu_vertex *d_verts, const mcrt_gpu_tria
     // node count when level r starts, so level r creates the nodes
     // [level_end[r], level_end[r + 1]).  A level at most halves the largest task,
     // so the first log2(nt / kSub) levels run without a look at the count of
-    // large tasks; after those the host reads it once per level.
+    // large tasks; after those the host reads it once per level.  Where the root
+    // itself has no split (all centroids in one place: a leaf of any size), the
+    // levels after it would be run for nothing, so the second level's first kernel
+    // writes the count to host memory, and the host looks at it once the rest of
+    // that level is queued: the device does not wait.  (50,000 triangles in one
+    // place: 306 us without a look, 241 with it, 236 with one at every level.)
     const uint32_t nbp = (nt + per - 1) / per;
     const uint32_t flag_tile = nt < kWideBlocks ? kMinFlagTile : 4u * kMinFlagTile;
     const uint32_t n_flag_tiles = (nt + flag_tile - 1) / flag_tile, n_part = 2 + n_flag_tiles;
@@ -1578,7 +1590,16 @@ static cudaError_t gpu_build(const mcrt_gpu_vertex *d_verts, const mcrt_gpu_tria
             return cudaErrorUnknown;
         }
         const uint32_t nw = std::max(n_large * (6 + kTaskBinWords), n_part);
-        k_task_reset<<<(nw + TB - 1) / TB, TB, 0, st>>>(S, level++, n_large, n_part); ::mcrt::note_launch();
+        const bool look = level == 1 && unseen > 1;
+        if (look) {
+            cudaError_t e = cudaSuccess;
+            if (!sc->large) e = cudaHostAlloc(reinterpret_cast<void **>(&sc->large), 4, cudaHostAllocMapped);
+            if (e == cudaSuccess && !sc->looked) e = cudaEventCreateWithFlags(&sc->looked, cudaEventDisableTiming);
+            if (e != cudaSuccess) { if (err) *err = "BVH level count"; return e; }
+        }
+        k_task_reset<<<(nw + TB - 1) / TB, TB, 0, st>>>(S, level++, n_large, n_part, look ? sc->large : nullptr);
+        ::mcrt::note_launch();
+        if (look) cudaEventRecord(sc->looked, st);
         k_centroid_bounds<<<nbp, 256, 0, st>>>(S, cur, per); ::mcrt::note_launch();
         k_bins<<<nbp, 256, 0, st>>>(S, cur, per); ::mcrt::note_launch();
         k_split<<<(n_large + 3) / 4, 128, 0, st>>>(S, cur); ::mcrt::note_launch();
@@ -1590,7 +1611,8 @@ static cudaError_t gpu_build(const mcrt_gpu_vertex *d_verts, const mcrt_gpu_tria
         if (unseen > 1) {                                // at most twice as many, each above kSub primitives
             --unseen;
             n_large = std::min(2u * n_large, nt / (kSub + 1u));
-            continue;
+            if (look) cudaEventSynchronize(sc->looked);
+            if (!look || *sc->large > 0) continue;
         }
         cudaMemcpyAsync(host_counters, S.counters, sizeof(host_counters), cudaMemcpyDeviceToHost, st);
         cudaError_t e = cudaStreamSynchronize(st);

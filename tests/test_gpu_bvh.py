@@ -68,3 +68,15 @@ def test_bvh_sizes_around_the_subtree_limits(ctx, oracle, n, kind):
     nodes, want = build_both(ctx, oracle, shape(kind, n, np.random.default_rng(n)))
     for f in ("aabb_min", "aabb_max"):
         assert np.array_equal(bits(nodes[f]), bits(want[f]))
+
+
+def test_triangles_in_one_place_take_two_levels(ctx, oracle):
+    """No split of the root: a leaf of any size, found after the second of the levels (six launches each) that a mesh of
+    this size would need."""
+    rng = np.random.default_rng(2)
+    n = 40000
+    build_both(ctx, oracle, np.repeat(rng.uniform(-1, 1, (1, 3, 3)), n, 0).astype(np.float32))
+    same = ctx.timings()["build_launches"]
+    build_both(ctx, oracle, shape("cloud", n, rng))
+    cloud = ctx.timings()["build_launches"]                     # six levels at least, and the subtrees
+    assert same + 4 * 6 <= cloud
