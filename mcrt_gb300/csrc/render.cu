@@ -765,6 +765,13 @@ constexpr uint32_t kGiveEarly = 4u, kGiveUnknown = 32u, kGiveLate = 128u;
 // A lone ray that is done within kProbeSteps never gets there: single caller's
 // rays take 33 us with it, 37 without.
 constexpr uint32_t kProbeSteps = 24;
+// The caller's rays give at once, above kFewRays.  A few rays have the device to
+// themselves, and what they lose to useless subtrees is the call: 1 / 8 rays giving at
+// once and after kGiveUnknown visits, in us: 1.3M-triangle mesh 34 / 43 and 33 / 43, from
+// a voxel world's camera 31 / 80 and 32 / 55, within it 36 / 55 and 34 / 35 (a thread
+// per ray: 31 / 69, 31 / 93 and 30 / 66).  More rays lose by waiting: 100 into 10,000
+// triangles 49 and 57, 1,000 into 80,000 70 and 82.
+constexpr uint32_t kFewRays = 16;
 // SHARE below this many rays per lane of the grid: one for the render's queues,
 // more for the caller's rays (250,000 into an 80,000-triangle mesh: 350 us with
 // the limit at eight, 393 at one).  With eight in the render, and subtrees given
@@ -806,7 +813,9 @@ __device__ __forceinline__ void trace_queue(const DeviceScene &S, const PathBuff
     uint32_t give_after = 0, visits = 0;
     float taken_t = -1.0f;
     int score = 0;
-    if (SHARE && !ANY && !PROBE) {
+    if (PROBE) {
+        give_after = n <= kFewRays ? kGiveUnknown : 0u;
+    } else if (SHARE && !ANY) {
         const int known = __ldcg(reinterpret_cast<const int *>(B.counters) + kShareScore);
         give_after = known > 0 ? kGiveEarly : (known < 0 ? kGiveLate : kGiveUnknown);
     }

@@ -55,3 +55,26 @@ def test_trace_refuses_a_ray_without_positive_tmin(scene, n, bad):
         ctx.trace_closest(rays)
     rays["tmin"][n - 2] = 1e-3
     assert np.array_equal(ctx.trace_closest(rays)["prim"], osc.trace(rays)["prim"])
+
+
+# the host looks at tmin up to 8,192 rays, the kernel above
+@pytest.mark.parametrize("layout", [False, True])
+@pytest.mark.parametrize("n", [8192, 8193])
+def test_trace_checks_tmin_on_both_sides_of_the_limit(scene, n, layout):
+    ctx, osc = scene
+    rays = random_scene_rays(np.random.default_rng(n), n)
+    rays["tmin"][n - 1] = -1e-3
+    with pytest.raises(M.MCRTError):
+        ctx.trace_closest(rays, reference_layout=layout)
+    rays["tmin"][n - 1] = 1e-3
+    got, want = ctx.trace_closest(rays, reference_layout=layout), osc.trace(rays)
+    assert np.array_equal(got["prim"], want["prim"]) and np.array_equal(bits(got["t"]), bits(want["t"]))
+
+
+@pytest.mark.parametrize("n", [8, 16, 17])
+def test_trace_few_rays(scene, n):
+    """A warp to a ray, with late and with early sharing of its subtrees."""
+    ctx, osc = scene
+    rays = random_scene_rays(np.random.default_rng(n), 64)[:n]
+    got, want = ctx.trace_closest(rays), osc.trace(rays)
+    assert np.array_equal(got["prim"], want["prim"]) and np.array_equal(bits(got["t"]), bits(want["t"]))
