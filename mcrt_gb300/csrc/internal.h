@@ -135,7 +135,7 @@ void extend_variant_info(int v, int out[6]);
 void prepare_extend_variants();
 
 // Launchers (render.cu)
-constexpr uint32_t kBadRay = 0u, kProbeCounters = 8u, kProbeChecked = 4096u;
+constexpr uint32_t kBadRay = 0u, kProbeCounters = 8u, kProbeChecked = 8192u;
 cudaError_t launch_trace_closest(const DeviceScene &S, const mcrt_ray *rays, uint32_t n, mcrt_hit *hits, bool ref_layout,
                                  uint32_t *d_counters, cudaStream_t st);
 // keep_radiance: replay of the same paths (the per-path radiance of the primal
