@@ -375,12 +375,12 @@ mcrt_status render_variant(mcrt_ctx *ctx, const mcrt_render_opts &o, int *varian
 
 // Whether a render with passes of n_slots paths takes the path kernel of small
 // scenes: few triangles and spheres for its passes, in large ones paths long
-// enough (kSmallPass), and neither a closest-hit variant nor the counting
+// enough (small_pass_paths), and neither a closest-hit variant nor the counting
 // kernels asked for.
 bool small_scene(const mcrt_ctx *ctx, const mcrt_render_opts &o, uint32_t n_slots, uint32_t depth, bool nee) {
     if (o.variant != 0 || (o.flags & MCRT_RENDER_COUNT) || ctx->n_triangles > mcrt::kSmallTris) return false;
     if (ctx->n_triangles && !*ctx->small_ok) return false;
-    return n_slots <= mcrt::kSmallPass
+    return n_slots <= mcrt::small_pass_paths()
                ? ctx->n_spheres <= mcrt::kSmallSpheres
                : ctx->n_spheres == 0 && ctx->n_triangles <= mcrt::kFewTris && depth > (nee ? 2u : 1u);
 }

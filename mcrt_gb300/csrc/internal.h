@@ -73,7 +73,7 @@ struct PathBuffers {
 // emax and vmax bound the edges' and the vertices' 1-norms.
 constexpr uint32_t kSmallTris = 64;
 constexpr uint32_t kSmallSpheres = 16;   // the path kernel's limit for a scene's spheres
-// Passes of more paths than this take the path kernel only for scenes of at
+// Passes of more than small_pass_paths() paths take the path kernel only for scenes of at
 // most kFewTris triangles and no sphere.  512x512, depth 8, path kernel / queue
 // kernels: Cornell box (36 triangles) NEE, 64 spp 14.2 / 20.0 ms; 32 spp: 16
 // triangles 0.61 / 0.84, NEE 0.63 / 0.96; a closed mesh of 32 triangles 2.25 /
@@ -85,7 +85,8 @@ constexpr uint32_t kSmallSpheres = 16;   // the path kernel's limit for a scene'
 // 1 and 2, 16 spp: Cornell box NEE 0.99 / 0.91 and 1.82 / 2.05 ms, with GGX 1.20
 // / 0.97 and 1.90 / 2.02, a closed room of 36 triangles NEE 1.15 / 0.89 and 2.54 /
 // 2.18, without NEE 0.40 / 0.44 and 0.87 / 1.09, 36 triangles in the open 0.37 / 0.33.
-constexpr uint32_t kSmallPass = 2u * 896u * 152u, kFewTris = 40;
+constexpr uint32_t kFewTris = 40;
+uint32_t small_pass_paths();             // two rounds of the path kernel's large blocks: 272,384 on 152 SMs
 struct SmallScene {
     float4 pair[8 * (kSmallTris / 2)];
     float emax, vmax;

@@ -1905,7 +1905,7 @@ __device__ __forceinline__ bool small_hit(const DeviceScene &S, const float4 *s_
 // keeps them in the same part of it: Cornell box, 512x512, 64 spp, next-event
 // estimation: five blocks of 128 threads 16.8 ms, the same with the barrier
 // 16.4, one of 640 15.0, of 768 14.7, of 896 14.2 (72 registers), of 1024 14.3;
-// the queue kernels 20.0.  Passes of at most kSmallPass paths use 128
+// the queue kernels 20.0.  Passes of at most small_pass_paths() paths use 128
 // threads: 160x120, 1 spp: 0.11 ms a call against 0.16 (queue kernels 0.37).
 constexpr int kPathsBlock = 896, kPathsSmallBlock = 128;
 constexpr uint32_t kFlush = 2;
@@ -2364,6 +2364,8 @@ void launch_shadow(const DeviceScene &S, const RenderParams &P, PathBuffers &B, 
     launch_retry(S, B, 0, true, adj, st);
 }
 
+uint32_t small_pass_paths() { return 2u * (uint32_t)kPathsBlock * (uint32_t)sm_count(); }
+
 void launch_small_scene(const DeviceScene &S, SmallScene *out, uint32_t *ok, cudaStream_t st) {
     k_small_scene<<<1, 2 * kSmallTris, 0, st>>>(S, out, ok); ::mcrt::note_launch();
 }
@@ -2371,7 +2373,7 @@ void launch_small_scene(const DeviceScene &S, SmallScene *out, uint32_t *ok, cud
 cudaError_t launch_paths(const DeviceScene &S, const RenderParams &P, PathBuffers &B, const SmallScene *T,
                          float4 *gbuf, cudaStream_t st, const AdjointParams *adj) {
     const uint32_t n = P.npix * P.spp_pass;
-    const bool large = n > kSmallPass;
+    const bool large = n > small_pass_paths();
     const int block = large ? kPathsBlock : kPathsSmallBlock;
     const int per_sm = large ? 1 : adj ? resident().paths_adj : resident().paths;
     const int blocks = min(grid_blocks_for(n, block), sm_count() * per_sm);
