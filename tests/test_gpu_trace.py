@@ -78,3 +78,22 @@ def test_trace_few_rays(scene, n):
     rays = random_scene_rays(np.random.default_rng(n), 64)[:n]
     got, want = ctx.trace_closest(rays), osc.trace(rays)
     assert np.array_equal(got["prim"], want["prim"]) and np.array_equal(bits(got["t"]), bits(want["t"]))
+
+
+# the kernel without a queue, around its blocks and the limit of the host's check
+@pytest.mark.parametrize("n_tri,n_sph", [(1, 0), (4, 4), (0, 3)])
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 8192, 8193])
+def test_trace_scenes_of_single_leaves(ctx, oracle, n_tri, n_sph, n):
+    rng = np.random.default_rng(n + n_tri)
+    v, t, s = np.zeros(3 * n_tri, M.VERTEX), np.zeros(n_tri, M.TRIANGLE), np.zeros(n_sph, M.SPHERE)
+    v["position"][:, :3], v["position"][:, 3], v["normal"][:, 1] = rng.uniform(-3, 3, (3 * n_tri, 3)), 1, 1
+    t["v"] = np.arange(3 * n_tri).reshape(n_tri, 3)
+    s["center_r"][:, :3], s["center_r"][:, 3] = rng.uniform(-2, 2, (n_sph, 3)), 0.8
+    scene = dict(materials=M.materials([(0, (0.5, 0.5, 0.5), 0, 1)]), vertices=v if n_tri else None,
+                 triangles=t if n_tri else None, spheres=s if n_sph else None)
+    ctx.upload_scene(**scene)
+    rays = random_scene_rays(rng, max(n, 64))[:n]
+    for _ in range(2):                              # a second call: nothing left over from the first
+        rays["org"] += np.float32(0.01)
+        got, want = ctx.trace_closest(rays), oracle.OracleScene(**scene).trace(rays)
+        assert np.array_equal(got["prim"], want["prim"]) and np.array_equal(bits(got["t"]), bits(want["t"]))
