@@ -221,7 +221,8 @@ typedef struct {
  * mcrt_variant_info — keeps the fastest for this context and
  * reports it.  Every variant gives the same images: a ray whose stack would
  * overflow is traced again without a stack, which costs its variant time on
- * a deep tree but never a hit.  out_ms (optional) receives the extend time of
+ * a deep tree but never a hit.  The choice is not used where a small scene is
+ * traced whole by one kernel (mcrt_last_timings) instead of the variants.  out_ms (optional) receives the extend time of
  * every variant; its capacity is 8 floats. */
 /* out6: BVH width, block size, minimum resident blocks per SM, stack depth,
  * idle lanes at which a warp fetches new rays, records of the compact tree's
@@ -528,8 +529,13 @@ mcrt_status mcrt_read_image_rgba8(mcrt_ctx *ctx, uint32_t mode, uint8_t *out);
  * tree (included in [0] and [1]), [6] / [7] with MCRT_RENDER_COUNT: compact
  * BVH node records (64 B) and triangle records (48 B) the closest-hit kernels
  * fetched (the bounce-0 warp packets fetch one record per warp).
- * Small scenes (at most 64 triangles and 16 spheres) are traced by one kernel
- * per pass unless a variant is named: its time is [1], [2] and [3] are 0.
+ * Small scenes may be traced whole by one kernel per pass: its time is [1], and
+ * [2] and [3] are 0.  Those are passes of up to two paths per thread of the device's
+ * blocks of 896 (272,384 paths on 152 SMs) into at most 64 triangles and 16
+ * spheres, and larger passes of more than one segment per path (two with
+ * MCRT_RENDER_NEE) into at most 40 triangles and no sphere; never with a named
+ * variant or MCRT_RENDER_COUNT, nor where a given tree's child boxes leave their
+ * parents'.
  * out_ms: 6 floats, out_counts: 8 uint64. */
 mcrt_status mcrt_last_timings(mcrt_ctx *ctx, float *out_ms, uint64_t *out_counts);
 

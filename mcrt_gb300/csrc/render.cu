@@ -1900,9 +1900,11 @@ __device__ __forceinline__ bool small_hit(const DeviceScene &S, const float4 *s_
 // and 1.7 to 3.3e-7 by the queue kernels' sums (8.5 ms).
 // counters[4] hands out chunks of slots, counters[6] collects cache queries.
 //
-// Bound by instruction fetch and issue: a step is some 5,000 instructions of
-// straight-line code.  One block per SM whose warps meet at a barrier each step
-// keeps them in the same part of it: Cornell box, 512x512, 64 spp, next-event
+// Bound by issue: 0.69 of the issue slots at 22 of 32 lanes (replay 0.60 at 23),
+// the warps waiting for the math pipes, fixed latencies and one another.  A step is
+// some 5,000 instructions of straight-line code, and one block per SM whose warps
+// meet at a barrier each step keeps them in the same part of it (then they hardly
+// wait for instructions): Cornell box, 512x512, 64 spp, next-event
 // estimation: five blocks of 128 threads 16.8 ms, the same with the barrier
 // 16.4, one of 640 15.0, of 768 14.7, of 896 14.2 (72 registers), of 1024 14.3;
 // the queue kernels 20.0.  Passes of at most small_pass_paths() paths use 128
